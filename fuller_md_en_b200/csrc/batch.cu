@@ -33,6 +33,7 @@ using namespace fmd;
 namespace {
 
 constexpr int kAtomThreads = 256;   // per-particle kernels (kicks, rescale)
+constexpr int kClusAtomsPerBlock = 144;   // cluster gather: 36 clusters, three per warp
 constexpr int kSideStreams = 8;     // parallel branches of a rebuild
 
 struct Tune {
@@ -102,6 +103,7 @@ struct fmd_batch {
             q.in_list = const_cast<int*>(s->arr.in_list);
             q.err = ctx->d_err;
             q.prune_words = s->prune.ok ? s->prune.words : nullptr;
+            q.lazy_edge = bd.lj_clus ? s->lazy_edge() : 0.0;
             const int M = s->mol.M;
             const int share = (int)std::max(1LL, (kRowBlocks * (long long)s->arr.n + ntot / 2) / ntot);
             off[r + 1] = off[r] + (M * 32 + 255) / 256;
@@ -201,7 +203,7 @@ struct fmd_batch {
             const StepArrays& a = sys[r]->arr;
             const long long terms = (long long)a.topo.nb + a.topo.nang + a.topo.ndih + a.topo.nimp;
             off[r + 1] = off[r] + blocks_for(a.n, kAtomThreads);
-            off[(R + 1) + r + 1] = off[(R + 1) + r] + blocks_for(a.n, t.lj_apb);
+            off[(R + 1) + r + 1] = off[(R + 1) + r] + blocks_for(a.n, bd.lj_clus ? kClusAtomsPerBlock : t.lj_apb);
             off[2 * (R + 1) + r + 1] = off[2 * (R + 1) + r] + blocks_for(std::max(terms, 1LL), t.f1_tpb);
         }
         if (cudaMemcpyAsync(dOff, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice, ctx->stream) !=
@@ -269,11 +271,18 @@ struct fmd_batch {
         // staged rows need one row stride (16-byte multiple) across replicas
         bool can_stage = sys[0]->arr.in_cap % 4 == 0;
         for (System* s : sys) can_stage = can_stage && s->arr.in_cap == sys[0]->arr.in_cap;
+        // cluster rows have one launch shape
+        if (bd.lj_clus) {
+            best.lj_threads = 256; best.lj_unroll = kClusG; best.lj_apb = kClusAtomsPerBlock; best.lj_staged = 0;
+            int rc = set_offsets(best);
+            if (rc) return rc;
+            best.lj_ms = time_ms(3, [&]() { return batch_lj_clus_launch(dA, bd.off_lj, R, bd.nblk_lj, bd.precision, st); });
+        }
         for (int staged : {0, 1})
             for (int nt : {128, 256})
                 for (int u : {2, 4})
                     for (int apb : {8, 16, 32, 64}) {
-                        if (staged && !can_stage) continue;
+                        if (bd.lj_clus || (staged && !can_stage)) continue;
                         Tune t = best;
                         t.lj_threads = nt; t.lj_unroll = u; t.lj_apb = apb; t.lj_staged = staged;
                         int rc = set_offsets(t);
@@ -317,7 +326,7 @@ struct fmd_batch {
             for (int k = 0; k < kSideStreams; k++)
                 if ((e = cudaStreamWaitEvent(side[k], ev_fork, 0)) != cudaSuccess) return e;
             for (int r = 0; r < R; r++)
-                if ((e = sys[r]->enqueue_rebuild(side[r % kSideStreams])) != cudaSuccess) return e;
+                if ((e = sys[r]->enqueue_rebuild(side[r % kSideStreams], bd.lj_clus)) != cudaSuccess) return e;
             for (int k = 0; k < kSideStreams; k++) {
                 if ((e = cudaEventRecord(ev_join[k], side[k])) != cudaSuccess) return e;
                 if ((e = cudaStreamWaitEvent(st, ev_join[k], 0)) != cudaSuccess) return e;
@@ -416,6 +425,16 @@ struct fmd_batch {
         return ctx->sync_check("batch graph capture");
     }
 
+    // The full rows of every replica for the row gather (a system's own
+    // rebuilds may have left them unbuilt).
+    int full_rows() {
+        if (!bd.lj_clus)
+            for (System* s : sys)
+                if (s->ensure_full_rows(ctx->stream) != cudaSuccess)
+                    return ctx->fail(FMD_ERR_CUDA, "batch: full rows failed");
+        return FMD_OK;
+    }
+
     int enqueue(int first, int last) {
         if (last < first) return FMD_OK;
         cudaStream_t st = ctx->stream;
@@ -423,9 +442,12 @@ struct fmd_batch {
         for (System* s : sys)
             if (cudaMemcpyAsync(&s->arr.S->gstep, &g0, sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess)
                 return ctx->fail(FMD_ERR_CUDA, "batch: step counter upload failed");
+        if (int rc = full_rows()) return rc;
         const fmd_run_params& p = sys[0]->p;
         for (int g = first; g <= last; g++) {
             const int r = (g % p.nlup) == 0, ph = g <= p.coldstart + p.warmup;
+            if (r)
+                for (System* s : sys) s->full_rows_stale = bd.lj_clus;
             int rc = capture(r != 0, ph != 0);
             if (rc != FMD_OK) return rc;
             if (cudaGraphLaunch(graphs[r][ph], st) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "batch: graph launch failed");
@@ -474,7 +496,14 @@ extern "C" int fmd_batch_create(fmd_ctx* ctx, int R, fmd_system* const* systems,
         }
     std::vector<StepArrays> A(R);
     std::vector<StepParams> P(R);
-    for (int r = 0; r < R; r++) { A[r] = b->sys[r]->arr; P[r] = b->sys[r]->sp; }
+    // the batch's gather walks cluster rows where every replica's does, else full rows
+    b->bd.lj_clus = 1;
+    for (System* s : b->sys) b->bd.lj_clus &= s->arr.clus.on;
+    for (int r = 0; r < R; r++) {
+        A[r] = b->sys[r]->arr;
+        A[r].prune_walk = b->bd.lj_clus;
+        P[r] = b->sys[r]->sp;
+    }
     cudaStream_t st = ctx->stream;
     if (cudaMalloc(&b->dA, sizeof(StepArrays) * R) != cudaSuccess ||
         cudaMalloc(&b->dP, sizeof(StepParams) * R) != cudaSuccess ||
@@ -500,6 +529,7 @@ extern "C" int fmd_batch_create(fmd_ctx* ctx, int R, fmd_system* const* systems,
     b->bd.ff = FMD_FF_MM;
     b->bd.precision = b->sys[0]->arr.precision;
     int rc = b->pending("before the batch set-up");
+    if (!rc) rc = b->full_rows();
     if (!rc) rc = autotune ? b->autotune() : b->set_offsets(b->tune);
     if (!rc) rc = b->pending("after the launch-shape set-up");
     if (!rc) rc = b->setup_mol_batch();

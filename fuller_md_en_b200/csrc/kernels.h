@@ -191,6 +191,36 @@ struct LJPruneOut {
     double delta = 0.0, rc = 0.0;
 };
 int lj_gather_blocks(int ff, int precision, const LJShape& shape, int in_cap);
+
+// Cluster rows of the atomistic LJ gather (ljclus.cu): kClusG atoms of one
+// molecule share one pruned row, each entry naming a partner atom, the
+// cluster's atoms that list it and the partner's image.
+constexpr int kClusG = 4;                  // atoms per cluster
+constexpr int kClusMaxAtoms = 1 << 22;     // partner index bits of an entry
+struct LJClus {
+    int on = 0;                 // 1: the step's gather walks cluster rows
+    int S = 0, cpm = 0;         // atoms and clusters per molecule
+    int nclus = 0, pmax = 0;    // clusters of the system, partner table width
+    const int* perm = nullptr;  // [cpm * kClusG] atoms of each cluster within its molecule, -1: none
+    // the molecule builder's tables and candidate bitmaps (molnlist.h)
+    const int* npart = nullptr; const int* part = nullptr; const int* rev = nullptr;
+    const unsigned* bm = nullptr;
+    const int* flag = nullptr;  // [0]: the last build was the molecule builder's
+    int4* cnt = nullptr;        // [nclus] {entries that count energy, all entries, images of its atoms}
+    int* rows = nullptr;        // [nclus * stride]
+    int stride = 0;
+    int in_lim = 0;             // entries from lower molecules an atom's full row holds
+    double* upos = nullptr;     // [3 n] positions followed without wrapping since the last prune
+    DevErr* err = nullptr;
+};
+// The step's LJ term over cluster rows: each evaluation builds them when a
+// prune is due (lj_prune_needed) and walks them, or the full rows when they
+// cannot be built (LJClus).  F, Facc, part as lj_gather_launch.  mode < 0:
+// decide (lj_clus_mode); 2: walk the rows of the last prune as they are.
+int lj_clus_blocks(int ff, int precision);
+cudaError_t lj_clus_launch(int ff, const LJClus& c, const double* pos, const double* hh, const int* in_cnt,
+                           const int* in_list, int in_cap, int na, double* F, double* Facc, double* part,
+                           cudaStream_t st, int precision, const LJPruneOut& po, int nrec, int mode = -1);
 cudaError_t lj_gather_launch(int ff, const double* pos, const double* hh, const int* cnt,
                              const int* list, int cap, const int* in_cnt, const int* in_list,
                              int in_cap, int na, double* F, double* Facc, double* part,

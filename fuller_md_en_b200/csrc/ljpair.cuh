@@ -64,6 +64,15 @@ struct LJF {
     float sig2, sig2_lo, c4, c24;
 };
 
+// 1/x of a normal x: the approximation and one Newton step in FMAs (within an
+// ulp, nearly always the rounded quotient), without the division's branch for
+// subnormal operands.
+__device__ __forceinline__ float rcp_f32(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return fmaf(fmaf(-x, y, 1.0f), y, y);
+}
+
 // One listed pair seen from atom i: d = r_j - r_i after the minimum image.
 // The cutoff test is the reference's FP64 one in both precisions, so both
 // modes interact through exactly the reference's pair set.  FP64: the
@@ -83,7 +92,7 @@ __device__ __forceinline__ void lj_pair(double dx, double dy, double dz, const L
     if (r2 < 0.25) r2 = 0.25;
     double fm, e = 0.0;
     if (F32) {
-        const float ri2 = __frcp_rn((float)r2);
+        const float ri2 = rcp_f32((float)r2);
         const float s2 = fmaf(pf.sig2, ri2, pf.sig2_lo * ri2), s6 = s2 * s2 * s2, s12 = s6 * s6;
         fm = (double)(pf.c24 * (2.f * s12 - s6) * ri2);
         if (COUNT) e = (double)(pf.c4 * (s12 - s6)) - p.vshift;

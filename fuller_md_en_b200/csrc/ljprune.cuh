@@ -1,18 +1,32 @@
 // ljprune.cuh -- the device-side decision of the pruned LJ rows (ljprune.cu).
 #pragma once
+#include <cuda_runtime.h>
+
 #include <cmath>
 
 namespace fmd {
 
-// 1 when the pruned rows may miss a pair now within the cutoff: the cell is
+// What the pruned rows' memory holds (words[1]): rows of single atoms or of
+// clusters, and the buffer they were built with.  A gather that finds other
+// rows there than its own (a replica batch and its system may use different
+// ones) builds its own first.
+constexpr unsigned long long kRowsAtoms = 1ull, kRowsClusters = 2ull;
+__host__ __device__ inline unsigned long long lj_rows_tag(unsigned long long kind, double delta) {
+    union { double d; unsigned long long u; } b;
+    b.d = delta;
+    return (b.u & ~3ull) | kind;
+}
+
+// 1 when the memory does not hold rows of this kind, or the pruned rows may miss a pair now within the cutoff: the cell is
 // not diagonal (now or at the prune), or k (rc + delta) + 2u >= delta less a
 // rounding margin, u the largest displacement since the last prune (bits in
-// *words, raised by the drift; a list build stores a huge value) and k the
+// words[0], raised by the drift; a list build stores a huge value) and k the
 // largest relative change of a cell edge since then.  Every block of the
 // gather and the step's reduction evaluate it on the same, unchanged inputs.
 __device__ __forceinline__ bool lj_prune_needed(const unsigned long long* words, const double* hh, const double* hb,
-                                                double delta, double rc) {
-    const double u = __longlong_as_double((long long)*words);
+                                                double delta, double rc, unsigned long long kind) {
+    if (words[1] != lj_rows_tag(kind, delta)) return true;
+    const double u = __longlong_as_double((long long)words[0]);
     double k = 0.0;
     for (int a = 0; a < 3; a++) k = fmax(k, fabs(hh[4 * a] - hb[4 * a]) / fabs(hb[4 * a]));
     const bool diag = hh[1] == 0.0 && hh[2] == 0.0 && hh[3] == 0.0 && hh[5] == 0.0 && hh[6] == 0.0 &&

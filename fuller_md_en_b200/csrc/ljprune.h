@@ -20,7 +20,7 @@ struct LJPrune {
     int* list = nullptr;          // [n * stride] pruned rows
     double* sb = nullptr;         // [3 n] fractional positions at the last prune
     double* hb = nullptr;         // [9] cell at the last prune
-    unsigned long long* words = nullptr;  // [1] bits of the largest displacement since the last prune
+    unsigned long long* words = nullptr;  // [2] bits of the largest displacement since the last prune, kind of rows
     unsigned long long* stats = nullptr;  // [2] {force evaluations, prune evaluations}
 };
 

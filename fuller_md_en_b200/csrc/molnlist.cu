@@ -433,6 +433,9 @@ __global__ void k_mol_rev(int M, const int* __restrict__ npart, const int* __res
 // i < j whose kept row lists j, ascending, then j's own row -- the rows the
 // transpose (nlist_transpose) builds, without atomics or a sort.  The own rows
 // are copied with 8 loads in flight per lane.
+__device__ __forceinline__ bool rows_deferred(const double* hh, double lazy_edge) {
+    return lazy_edge > 0.0 && fmin(hh[0], fmin(hh[4], hh[8])) > lazy_edge;
+}
 constexpr int kInChunk = 32;
 constexpr int kInWarps = 8;
 constexpr int kInAtoms = 32 / kInWarps;               // atoms per warp
@@ -543,7 +546,9 @@ __global__ void __launch_bounds__(32 * kInWarps)
 k_mol_incoming(int M, int S, const int* __restrict__ npart, const int* __restrict__ part, int pmax,
                const int* __restrict__ rev, int W, const unsigned* __restrict__ bm, int cap,
                const int* __restrict__ cnt, const int* __restrict__ list, int* __restrict__ in_cnt,
-               int* __restrict__ in_list, int in_cap, DevErr* err, const int* __restrict__ flag) {
+               int* __restrict__ in_list, int in_cap, DevErr* err, const int* __restrict__ flag,
+               const double* __restrict__ hh, double lazy_edge) {
+    if (rows_deferred(hh, lazy_edge)) return;
     mol_incoming_body(M, S, npart, part, pmax, rev, W, bm, cap, cnt, list, in_cnt, in_list, in_cap, err, flag,
                       blockIdx.x, gridDim.x);
 }
@@ -618,6 +623,7 @@ __global__ void __launch_bounds__(32 * kInWarps)
 k_b_mol_incoming(const MolRep* __restrict__ reps, const int* __restrict__ off, int R) {
     const int r = rep_of(off, R, blockIdx.x);
     const MolRep& q = reps[r];
+    if (rows_deferred(q.hh, q.lazy_edge)) return;
     mol_incoming_body(q.m.M, q.m.usize, q.m.npart, q.m.part, q.m.pmax, q.m.rev, q.m.words, q.m.bm, q.cap, q.cnt,
                       q.list, q.in_cnt, q.in_list, q.in_cap, q.err, q.m.flag, blockIdx.x - off[r],
                       off[r + 1] - off[r]);
@@ -761,11 +767,13 @@ cudaError_t mol_rows_half(const MolLists& m, const double* pos, const double* hh
 }
 
 cudaError_t mol_rows_incoming(const MolLists& m, int cap, const int* cnt, const int* list, int* in_cnt,
-                              int* in_list, int in_cap, DevErr* err, cudaStream_t st) {
+                              int* in_list, int in_cap, DevErr* err, cudaStream_t st, const double* hh,
+                              double lazy_edge) {
     if (!m.masks) return cudaErrorInvalidValue;
     const int blocks = 2 * m.M < kRowBlocksMol ? 2 * m.M : kRowBlocksMol;
     k_mol_incoming<<<blocks, 32 * kInWarps, 0, st>>>(m.M, m.usize, m.npart, m.part, m.pmax, m.rev, m.words, m.bm,
-                                                     cap, cnt, list, in_cnt, in_list, in_cap, err, m.flag);
+                                                     cap, cnt, list, in_cnt, in_list, in_cap, err, m.flag, hh,
+                                                     hh ? lazy_edge : 0.0);
     return cudaGetLastError();
 }
 

@@ -48,8 +48,12 @@ cudaError_t mol_rows_half(const MolLists& m, const double* pos, const double* hh
 // The LJ gather's full rows (incoming entries ascending, then the row) from
 // the candidate bitmaps of the last mol_rows_half (m.masks only); no-op
 // unless flag[0] is set.
+// hh, lazy_edge > 0: nothing is built while every edge of the (diagonal) cell
+// exceeds lazy_edge -- the system's gather walks cluster rows and the full
+// rows are built when somebody asks for them (System::ensure_full_rows).
 cudaError_t mol_rows_incoming(const MolLists& m, int cap, const int* cnt, const int* list, int* in_cnt,
-                              int* in_list, int in_cap, DevErr* err, cudaStream_t st);
+                              int* in_list, int in_cap, DevErr* err, cudaStream_t st, const double* hh = nullptr,
+                              double lazy_edge = 0.0);
 
 // One replica of a batched molecule-path rebuild (replica batches of MM
 // systems, batch.cu): its molecule tables and the lists it builds.
@@ -64,6 +68,7 @@ struct MolRep {
     int* dropped = nullptr;
     int* in_cnt = nullptr;
     int* in_list = nullptr;
+    double lazy_edge = 0.0;               // as mol_rows_incoming
     DevErr* err = nullptr;
     unsigned long long* prune_words = nullptr;   // the replica's pruned-row bound (marked stale), or null
 };

@@ -27,6 +27,7 @@
 #include "step.h"
 #include "ljprune.h"
 #include "ljprune.cuh"
+#include "ljclus.cuh"
 #include "geom.cuh"
 #include "sg_host.h"
 #include "pdl.cuh"
@@ -151,7 +152,15 @@ __device__ void kick_body(const StepArrays& a, double dt, int blk, int nblk, con
         if (a.prune_sb) {
             // nearest-image fractional displacement, measured in the new cell
             double ex = sx - a.prune_sb[3 * i], ey = sy - a.prune_sb[3 * i + 1], ez = sz - a.prune_sb[3 * i + 2];
-            ex -= rint(ex); ey -= rint(ey); ez -= rint(ez);
+            const double kx = rint(ex), ky = rint(ey), kz = rint(ez);
+            ex -= kx; ey -= ky; ez -= kz;
+            if (a.clus.on) {
+                // the position followed from the last prune without wrapping
+                const double wx = sx - kx, wy = sy - ky, wz = sz - kz;
+                a.clus.upos[3 * i] = h[0] * wx + h[1] * wy + h[2] * wz;
+                a.clus.upos[3 * i + 1] = h[3] * wx + h[4] * wy + h[5] * wz;
+                a.clus.upos[3 * i + 2] = h[6] * wx + h[7] * wy + h[8] * wz;
+            }
             const double ux = h[0] * ex + h[1] * ey + h[2] * ez, uy = h[3] * ex + h[4] * ey + h[5] * ez,
                          uz = h[6] * ex + h[7] * ey + h[8] * ez;
             u2 = fmax(u2, ux * ux + uy * uy + uz * uz);
@@ -397,8 +406,17 @@ __device__ void record(SysScal* S, int kind, const StepParams& p) {
 // and prunes.
 __device__ void lj_prune_commit(const StepArrays& a, const double* hh) {
     if (!a.prune_hb || !(a.prune_delta > 0.0)) return;
-    if (lj_prune_needed(a.prune_umax, hh, a.prune_hb, a.prune_delta, a.prune_rc)) {
-        *a.prune_umax = 0ull;
+    if (!a.prune_walk) {
+        a.prune_stats[0] += 1ull;
+        return;
+    }
+    const bool pruned = a.clus.on ? lj_clus_mode(a.clus, a.prune_umax, hh, a.prune_hb, a.prune_delta, a.prune_rc) ==
+                                        CLUS_PRUNE
+                                  : lj_prune_needed(a.prune_umax, hh, a.prune_hb, a.prune_delta, a.prune_rc,
+                                                    kRowsAtoms);
+    if (pruned) {
+        a.prune_umax[0] = 0ull;
+        a.prune_umax[1] = lj_rows_tag(a.clus.on ? kRowsClusters : kRowsAtoms, a.prune_delta);
         for (int q = 0; q < 9; q++) a.prune_hb[q] = hh[q];
         a.prune_stats[1] += 1ull;
     }
@@ -567,6 +585,9 @@ cudaError_t enqueue_lj(const StepArrays& a, int ff, cudaStream_t st) {
     if (!a.prune || a.prune->delta <= 0.0)
         return lj_gather_launch(ff, a.pos, hh, a.cnt_a, a.list_a, a.cap_a, a.in_cnt, a.in_list, a.in_cap, a.n, a.F,
                                 a.Facc, a.part_f2, st, a.precision, a.lj_shape, a.err, LJPruneOut{}, a.lj_blocks);
+    if (a.clus.on)
+        return lj_clus_launch(ff, a.clus, a.pos, hh, a.in_cnt, a.in_list, a.in_cap, a.n, a.F, a.Facc, a.part_f2, st,
+                              a.precision, lj_prune_out(*a.prune), a.lj_blocks);
     // one launch: each block decides whether this evaluation prunes (full
     // rows, pruned rows written) or walks the pruned rows; the step's
     // reduction then restarts the displacement bound (lj_prune_commit)
@@ -641,7 +662,9 @@ cudaError_t enqueue_batch_step(const BatchDev& b, bool rescale_phase, cudaStream
     k_b_kick<<<b.nblk_atom, kPB, 0, st>>>(b);
     if (b.kind == FMD_SYS_MM)
         if ((e = batch_mm_bonded_launch(b.A, b.off_f1, b.R, b.nblk_f1, b.f1_threads, st)) != cudaSuccess) return e;
-    if ((e = batch_lj_launch(b.A, b.off_lj, b.R, b.nblk_lj, b.ff, b.precision, b.lj_threads, b.lj_unroll, st,
+    if (b.lj_clus) {
+        if ((e = batch_lj_clus_launch(b.A, b.off_lj, b.R, b.nblk_lj, b.precision, st)) != cudaSuccess) return e;
+    } else if ((e = batch_lj_launch(b.A, b.off_lj, b.R, b.nblk_lj, b.ff, b.precision, b.lj_threads, b.lj_unroll, st,
                              b.lj_staged_in_cap)) != cudaSuccess)
         return e;
     k_b_kick2<<<b.nblk_atom, kPB, 0, st>>>(b);

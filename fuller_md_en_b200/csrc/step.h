@@ -77,11 +77,14 @@ struct StepArrays {
     // step), and the fractional positions of the last prune and the
     // displacement word the drift raises.
     const LJPrune* prune = nullptr;
+    int prune_walk = 1;                         // 0: the gather walks the full rows and builds none (row-gather batch)
+    int* prune_cnt = nullptr;
     const double* prune_sb = nullptr;
     unsigned long long* prune_umax = nullptr;
     double* prune_hb = nullptr;                 // cell of the last prune
     unsigned long long* prune_stats = nullptr;  // {evaluations, prunes}
     double prune_delta = 0.0, prune_rc = 0.0;   // buffer (0: off) and LJ cutoff
+    LJClus clus{};                              // cluster rows (clus.on: the LJ term walks them)
 };
 
 struct StepParams {
@@ -133,12 +136,16 @@ struct BatchDev {
     int nblk_atom = 0, nblk_lj = 0, nblk_f1 = 0;   // totals (off[R])
     int lj_threads = 256, lj_unroll = 4, f1_threads = 128;
     int lj_staged_in_cap = 0;        // > 0: LJ rows staged in shared memory
+    int lj_clus = 0;                 // 1: cluster rows (every replica's clus.on)
     int kind = FMD_SYS_MM, ff = FMD_FF_MM, precision = FMD_PREC_FP64;
 };
 // LJ gather / MM bonded terms over all replicas in one launch each.
 // staged_in_cap > 0: rows staged in shared memory (all replicas' row stride).
 cudaError_t batch_lj_launch(const StepArrays* As, const int* off, int R, int nblocks, int ff, int precision,
                             int threads, int unroll, cudaStream_t st, int staged_in_cap = 0);
+// The LJ term over cluster rows of every replica (MM), off by cluster blocks.
+cudaError_t batch_lj_clus_launch(const StepArrays* As, const int* off, int R, int nblocks, int precision,
+                                 cudaStream_t st);
 cudaError_t batch_mm_bonded_launch(const StepArrays* As, const int* off, int R, int nblocks, int threads,
                                    cudaStream_t st);
 // One step of every replica (the single-system step's launches, each once

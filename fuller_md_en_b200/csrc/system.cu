@@ -12,6 +12,8 @@
 #include <map>
 #include <memory>
 #include <tuple>
+#include "ljclus.h"
+#include "ljprune.cuh"
 #include "step.h"
 #include "system.h"
 #include "sg_host.h"
@@ -149,7 +151,7 @@ int System::alloc_prune(double rc_lj) {
     LJPrune q;
     if (alloc(&q.cnt, n, (const int*)nullptr) || alloc(&q.list, (size_t)n * arr.in_cap, (const int*)nullptr) ||
         alloc(&q.sb, 3 * (size_t)n, (const double*)nullptr) || alloc(&q.hb, 9, (const double*)nullptr) ||
-        alloc(&q.words, 1, (const unsigned long long*)nullptr) ||
+        alloc(&q.words, 2, (const unsigned long long*)nullptr) ||
         alloc(&q.stats, 2, (const unsigned long long*)nullptr))
         return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
     q.n = n;
@@ -160,6 +162,7 @@ int System::alloc_prune(double rc_lj) {
     if (lj_prune_clear(q, ctx->stream) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
     prune = q;
     arr.prune = &prune;
+    arr.prune_cnt = prune.cnt;
     arr.prune_sb = prune.sb;
     arr.prune_umax = prune.words;
     arr.prune_hb = prune.hb;
@@ -169,7 +172,71 @@ int System::alloc_prune(double rc_lj) {
     return FMD_OK;
 }
 
-cudaError_t System::enqueue_rebuild(cudaStream_t st) {
+// Tables of the cluster gather (ljclus.cu), for equal contiguous molecules
+// whose list builder keeps candidate bitmaps: the clusters are those of the
+// first molecule's initial geometry (crystals are copies of one molecule; a
+// molecule whose atoms are ordered otherwise only has wider clusters).  The
+// rows share the pruned rows' memory: a cluster's row is at most as long as
+// its atoms' rows together.
+int System::alloc_clus(const double* pos_h) {
+    if (!prune.ok || !mol.ok || !mol.masks || arr.n >= kClusMaxAtoms) return FMD_OK;
+    // no buffer makes a cell with edges below twice the cutoff take cluster rows
+    if (!(std::min(h0[0], std::min(h0[4], h0[8])) > 2.0 * prune.rc)) return FMD_OK;
+    LJClus q;
+    q.S = mol.usize;
+    q.cpm = (q.S + kClusG - 1) / kClusG;
+    q.nclus = mol.M * q.cpm;
+    q.pmax = mol.pmax;
+    std::vector<double> x(3 * (size_t)q.S);
+    for (int a = 0; a < q.S; a++)
+        for (int c = 0; c < 3; c++) {
+            const double L = h0[4 * c], d = pos_h[3 * a + c] - pos_h[c];
+            x[3 * a + c] = L > 0.0 ? d - L * std::rint(d / L) : d;
+        }
+    const std::vector<int> perm = lj_clus_assign(x.data(), q.S);
+    int* dp;
+    if (alloc(&dp, perm.size(), (const int*)nullptr) || alloc(&q.cnt, q.nclus, (const int4*)nullptr) ||
+        alloc(&q.upos, 3 * (size_t)arr.n, (const double*)nullptr))
+        return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
+    if (cudaMemcpyAsync(dp, perm.data(), sizeof(int) * perm.size(), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
+        return ctx->fail(FMD_ERR_CUDA, "cluster table copy failed");
+    q.perm = dp;
+    q.npart = mol.npart; q.part = mol.part; q.rev = mol.rev; q.bm = mol.bm; q.flag = mol.flag;
+    q.err = ctx->d_err;
+    q.in_lim = arr.in_cap - arr.cap_a;
+    q.rows = prune.list;
+    q.stride = (int)std::min<size_t>((size_t)kClusG * arr.in_cap, (size_t)arr.n * arr.in_cap / q.nclus);
+    arr.clus = q;
+    return FMD_OK;
+}
+
+// The step's LJ term walks cluster rows when the tables exist, pruning is on,
+// no launch shape of the row gather is pinned and the initial cell takes them
+// (lj_clus_mode; a cell that stops doing so walks the full rows).
+void System::set_clus(bool allowed) {
+    const bool diag = h0[1] == 0.0 && h0[2] == 0.0 && h0[3] == 0.0 && h0[5] == 0.0 && h0[6] == 0.0 && h0[7] == 0.0;
+    const double edge = std::min(h0[0], std::min(h0[4], h0[8]));
+    arr.clus.on = allowed && arr.clus.perm && prune.delta > 0.0 && diag &&
+                  edge > 1.02 * (2.0 * (prune.rc + prune.delta) + 0.1);
+}
+
+// Cell edges beyond which a rebuild leaves the full rows unbuilt (0: it builds
+// them): those the cluster gather takes, with a margin above what the barostat
+// (edge rates clamped at 0.005 A/fs) can shorten them by before the next one.
+double System::lazy_edge() const {
+    if (!arr.clus.on) return 0.0;
+    return 2.0 * (prune.rc + prune.delta) + 0.2 + 0.01 * std::fabs(sp.dt) * p.nlup;
+}
+
+// The full rows of the last build, when the gather left them unbuilt.
+cudaError_t System::ensure_full_rows(cudaStream_t st) {
+    if (!full_rows_stale) return cudaSuccess;
+    full_rows_stale = false;
+    return mol_rows_incoming(mol, arr.cap_a, arr.cnt_a, arr.list_a, const_cast<int*>(arr.in_cnt),
+                             const_cast<int*>(arr.in_list), arr.in_cap, ctx->d_err, st);
+}
+
+cudaError_t System::enqueue_rebuild(cudaStream_t st, bool lazy) {
     cudaError_t e;
     double* hh = arr.S->h;
     if ((e = inv9_launch(hh, st)) != cudaSuccess) return e;
@@ -215,7 +282,8 @@ cudaError_t System::enqueue_rebuild(cudaStream_t st) {
         if ((e = mol_rows_half(mol, arr.pos, hh, rc2_a, arr.cap_a, cnt_a, list_a, dropped, st)) != cudaSuccess)
             return e;
         if ((e = mol_rows_incoming(mol, arr.cap_a, arr.cnt_a, arr.list_a, const_cast<int*>(arr.in_cnt),
-                                   const_cast<int*>(arr.in_list), arr.in_cap, ctx->d_err, st)) != cudaSuccess)
+                                   const_cast<int*>(arr.in_list), arr.in_cap, ctx->d_err, st, hh, lazy ? lazy_edge() : 0.0)) !=
+            cudaSuccess)
             return e;
         if (prune.ok) return lj_prune_mark(prune, st);
         return cudaSuccess;
@@ -235,7 +303,8 @@ cudaError_t System::enqueue_rebuild(cudaStream_t st) {
                                  const_cast<int*>(arr.in_list), arr.in_cap, ctx->d_err, st, gate)) != cudaSuccess)
             return e;
         if ((e = mol_rows_incoming(mol, arr.cap_a, arr.cnt_a, arr.list_a, const_cast<int*>(arr.in_cnt),
-                                   const_cast<int*>(arr.in_list), arr.in_cap, ctx->d_err, st)) != cudaSuccess)
+                                   const_cast<int*>(arr.in_list), arr.in_cap, ctx->d_err, st, hh, lazy ? lazy_edge() : 0.0)) !=
+            cudaSuccess)
             return e;
     } else if ((e = nlist_transpose(arr.cnt_a, arr.list_a, arr.cap_a, arr.n, const_cast<int*>(arr.in_cnt),
                                     const_cast<int*>(arr.in_list), arr.in_cap, ctx->d_err, st)) != cudaSuccess) {
@@ -371,6 +440,11 @@ LJShape System::pick_lj_shape(bool pruned, int& rc) {
 // smaller one zero-fills the rest).
 void System::set_lj_blocks() {
     const int ff = arr.kind == FMD_SYS_AIREBO ? FMD_FF_AIREBO : FMD_FF_MM;
+    if (arr.clus.on) {
+        arr.lj_shape_p = LJShape{256, 4, 0, 1};       // reported: 256 threads, 4 atoms in flight, contiguous runs
+        arr.lj_blocks = lj_clus_blocks(ff, arr.precision);
+        return;
+    }
     arr.lj_blocks = std::max(lj_gather_blocks(ff, arr.precision, arr.lj_shape, arr.in_cap),
                              lj_gather_blocks(ff, arr.precision, arr.lj_shape_p, arr.in_cap));
 }
@@ -410,6 +484,13 @@ int System::tune_lj() {
         return ctx->fail(FMD_ERR_ARG, "FMD_LJ_SHAPE: expected threads,unroll,feed[;threads,unroll,feed] with "
                                       "threads 128|256, unroll 2|4, feed 0..2 or 4..6");
     }
+    // the cluster gather has one shape; the row gather then only runs when
+    // pruning is switched off, which tunes it
+    if (arr.clus.on) {
+        arr.lj_shape = LJShape{256, 4, 2, 1};
+        set_lj_blocks();
+        return FMD_OK;
+    }
     const auto key = std::make_tuple(ctx->device, arr.kind, arr.n, arr.cap_a, arr.precision);
     auto it = cache.find(key);
     if (it != cache.end()) {
@@ -426,13 +507,33 @@ int System::tune_lj() {
     return FMD_OK;
 }
 
+// After a change of the prune buffer of a running system: cluster rows or the
+// row gather, which is tuned (into F's scratch: F again from the current
+// state) when no shape is pinned or cached.
+int System::retune_lj() {
+    if (lj_pinned) return FMD_OK;
+    const bool was = arr.clus.on;
+    if (ensure_full_rows(ctx->stream) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "full rows failed");
+    set_clus(true);
+    if (arr.clus.on == was) return FMD_OK;
+    if (arr.clus.on) {
+        set_lj_blocks();
+        return FMD_OK;
+    }
+    const int rc = tune_lj();
+    if (rc != FMD_OK) return rc;
+    if (enqueue_forces(arr, ctx->stream) != cudaSuccess || enqueue_force_reduce(arr, ctx->stream) != cudaSuccess)
+        return ctx->fail(FMD_ERR_CUDA, "force launch failed");
+    return ctx->sync_check("LJ launch-shape tuning");
+}
+
 // run_tuner false: only a shape cached by an earlier system of the same size
 // is applied, and *pending tells whether the tuner still has to run (after
 // the first evaluation has written the pruned rows).
 int System::tune_lj_pruned(bool run_tuner, bool* pending) {
     static std::map<std::tuple<int, int, int, int, int>, LJShape> cache;
     if (pending) *pending = false;
-    if (!prune.ok || prune.delta <= 0.0 || std::getenv("FMD_LJ_SHAPE")) return FMD_OK;
+    if (!prune.ok || prune.delta <= 0.0 || arr.clus.on || std::getenv("FMD_LJ_SHAPE")) return FMD_OK;
     const auto key = std::make_tuple(ctx->device, arr.kind, arr.n, arr.cap_a, arr.precision);
     auto it = cache.find(key);
     if (it != cache.end()) {
@@ -500,7 +601,10 @@ int System::init() {
     cudaStream_t st = ctx->stream;
     // Pre-loop order of the reference: lists from the unwrapped positions,
     // then apply_pbc, then the first forces (LJ:813-828, AI:830-853).
+    if (std::getenv("FMD_LJ_SHAPE")) lj_pinned = true;
+    set_clus(!lj_pinned);
     if (enqueue_rebuild(st) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "list build launch failed");
+    full_rows_stale = arr.clus.on;
     if (apply_pbc_launch(arr.pos, arr.n, arr.S->h, st) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "apply_pbc failed");
     if (arr.kind != FMD_SYS_RIGID) {
         const int rc = tune_lj();
@@ -588,7 +692,10 @@ int System::enqueue(int first, int last) {
     cudaStream_t st = ctx->stream;
     const int g0 = first - 1;
     cudaMemcpyAsync(&arr.S->gstep, &g0, sizeof(int), cudaMemcpyHostToDevice, st);
+    // rows a batch left unbuilt, for a gather that needs them
+    if (!arr.clus.on && ensure_full_rows(st) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "full rows failed");
     for (int g = first; g <= last; g++) {
+        if (arr.clus.on && g % p.nlup == 0) full_rows_stale = true;
         if (p.use_graphs) {
             const int r = (g % p.nlup) == 0, ph = g <= p.coldstart + p.warmup, j = judge_step(g);
             int rc = capture(r != 0, ph != 0, j != 0);
@@ -687,7 +794,7 @@ extern "C" int fmd_system_create_airebo(fmd_ctx* ctx, const fmd_run_params* p, i
     const double rebo_rcut = 2.0 + 0.3;         // AI:116
     if ((rc = s->alloc_lists(lj_rcut + 2.0, 400, rebo_rcut, 12, true)) != FMD_OK) return rc;
     if (fmd::mol_lists_alloc(s->mol, na, mol_id, s->owned_alloc()) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "list allocation failed");
-    if ((rc = s->alloc_prune(lj_rcut)) != FMD_OK) return rc;
+    if ((rc = s->alloc_prune(lj_rcut)) != FMD_OK || (rc = s->alloc_clus(pos)) != FMD_OK) return rc;
     out[0] = new fmd_system{std::move(s)};
     return FMD_OK;
 }
@@ -724,7 +831,7 @@ int create_mm(fmd_ctx* ctx, const fmd_run_params* p, int na, const double* pos, 
     const double rcut = 3.0 * 3.431;            // MM:114
     if ((rc = s->alloc_lists(rcut + 2.0, 400, 0.0, 0, true)) != FMD_OK) return rc;
     if (fmd::mol_lists_alloc(s->mol, na, mol_id, s->owned_alloc()) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "list allocation failed");
-    if ((rc = s->alloc_prune(rcut)) != FMD_OK) return rc;
+    if ((rc = s->alloc_prune(rcut)) != FMD_OK || (rc = s->alloc_clus(pos)) != FMD_OK) return rc;
     out[0] = new fmd_system{std::move(s)};
     return FMD_OK;
 }
@@ -916,6 +1023,8 @@ extern "C" int fmd_system_lj_rows(fmd_system* s, int* full_cnt, int* pruned_cnt)
     fmd::System& y = *s->sys;
     cudaStream_t st = y.ctx->stream;
     const size_t n = y.arr.n;
+    if (full_cnt && y.initialized && y.ensure_full_rows(st) != cudaSuccess)
+        return y.ctx->fail(FMD_ERR_CUDA, "full rows failed");
     if (full_cnt && y.arr.in_cnt) cudaMemcpyAsync(full_cnt, y.arr.in_cnt, sizeof(int) * n, cudaMemcpyDeviceToHost, st);
     if (pruned_cnt && y.prune.ok) cudaMemcpyAsync(pruned_cnt, y.prune.cnt, sizeof(int) * n, cudaMemcpyDeviceToHost, st);
     return y.ctx->sync_check("system LJ rows");
@@ -993,6 +1102,8 @@ extern "C" int fmd_system_lj_full_rows(fmd_system* s, int* cnt, int* list, int* 
     if (!y.arr.in_list) return FMD_OK;
     cudaStream_t st = y.ctx->stream;
     const size_t n = y.arr.n;
+    if ((cnt || list) && y.initialized && y.ensure_full_rows(st) != cudaSuccess)
+        return y.ctx->fail(FMD_ERR_CUDA, "full rows failed");
     if (cnt) cudaMemcpyAsync(cnt, y.arr.in_cnt, sizeof(int) * n, cudaMemcpyDeviceToHost, st);
     if (list) cudaMemcpyAsync(list, y.arr.in_list, sizeof(int) * n * y.arr.in_cap, cudaMemcpyDeviceToHost, st);
     return y.ctx->sync_check("system LJ full rows");
@@ -1041,10 +1152,15 @@ extern "C" int fmd_system_kernel_ms(fmd_system* s, int stage, int reps, double* 
                 return rigid_launch(a.precision, a.pos, a.qv, a.body, hh, a.cnt_a, a.list_a, a.cap_a, a.n, a.natom,
                                     a.rmcut2, a.F, a.T, a.part_f1, st, a.rigid_lab, a.rigid_shape);
             case 2:
+                y.full_rows_stale = a.clus.on;
                 return y.enqueue_rebuild(st);
             case 4:
                 // the gather over the pruned rows of the last prune, into the scratch accumulator
                 if (!a.prune) return cudaErrorInvalidValue;
+                if (a.clus.on)
+                    return lj_clus_launch(a.kind == FMD_SYS_AIREBO ? FMD_FF_AIREBO : FMD_FF_MM, a.clus, a.pos, hh,
+                                          a.in_cnt, a.in_list, a.in_cap, a.n, a.Facc, a.Facc, a.part_f2, st,
+                                          a.precision, lj_prune_out(*a.prune), 0, 2);
                 return lj_gather_launch(a.kind == FMD_SYS_AIREBO ? FMD_FF_AIREBO : FMD_FF_MM, a.pos, hh, a.cnt_a,
                                         a.list_a, a.cap_a, a.prune->cnt, a.prune->list, a.in_cap, a.n, a.Facc,
                                         a.Facc, a.part_f2, st, a.precision, a.lj_shape_p, a.err);
@@ -1057,6 +1173,19 @@ extern "C" int fmd_system_kernel_ms(fmd_system* s, int stage, int reps, double* 
                 return enqueue_forces(a, st);
         }
     };
+    // stage 4 walks the rows as they are: of this system's gather
+    if (stage == 4 && a.prune) {
+        unsigned long long kind = 0;
+        if (cudaMemcpyAsync(&kind, a.prune_umax + 1, sizeof(kind), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess)
+            return y.ctx->fail(FMD_ERR_CUDA, "kernel timing: read failed");
+        if (kind != fmd::lj_rows_tag(a.clus.on ? fmd::kRowsClusters : fmd::kRowsAtoms, a.prune_delta)) {
+            enqueue_forces(a, st);
+            enqueue_force_reduce(a, st);
+        }
+    }
+    if (stage == 0 && a.kind != FMD_SYS_RIGID && y.ensure_full_rows(st) != cudaSuccess)
+        return y.ctx->fail(FMD_ERR_CUDA, "full rows failed");
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -1107,6 +1236,12 @@ extern "C" int fmd_system_set_lj_shape(fmd_system* s, int threads, int unroll, i
     if (nb < 1) return y.ctx->fail(FMD_ERR_ARG, "fmd_system_set_lj_shape: shape cannot run with this list");
     if (cudaStreamSynchronize(y.ctx->stream) != cudaSuccess) return y.ctx->fail(FMD_ERR_CUDA, "sync failed");
     y.drop_graphs();                     // captured graphs hold the old launch
+    if (y.initialized && y.ensure_full_rows(y.ctx->stream) != cudaSuccess)
+        return y.ctx->fail(FMD_ERR_CUDA, "full rows failed");
+    y.lj_pinned = true;
+    y.set_clus(false);                   // the pinned row gather; the memory it shares with the cluster rows is stale
+    if (y.prune.ok && lj_prune_mark(y.prune, y.ctx->stream) != cudaSuccess)
+        return y.ctx->fail(FMD_ERR_CUDA, "prune mark failed");
     y.arr.lj_shape = sh;
     y.arr.lj_shape_p = sh;
     y.arr.lj_blocks = nb;
@@ -1134,6 +1269,10 @@ extern "C" int fmd_system_set_lj_prune(fmd_system* s, double delta) {
     y.drop_graphs();                     // captured graphs hold the old launches
     y.prune.delta = delta;
     y.arr.prune_delta = delta;
+    if (y.initialized) {
+        const int rc = y.retune_lj();
+        if (rc != FMD_OK) return rc;
+    }
     if (lj_prune_mark(y.prune, y.ctx->stream) != cudaSuccess) return y.ctx->fail(FMD_ERR_CUDA, "prune mark failed");
     if (y.initialized && y.p.use_graphs) {
         int rc = FMD_OK;

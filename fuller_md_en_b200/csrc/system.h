@@ -27,6 +27,8 @@ struct System {
     cudaStream_t side = nullptr;       // captures the rebuild fallback's conditional body
     cudaEvent_t obs_ev[2] = {};        // fmd_system_enqueue_obs: copies of odd / even last steps
     bool initialized = false;
+    bool full_rows_stale = false;      // the last rebuild left the LJ gather's full rows unbuilt
+    bool lj_pinned = false;            // launch shape of the row gather pinned by the caller
     // one graph per {rebuild, cold/warm phase, judge of the learned REBO term}
     cudaGraphExec_t graphs[2][2][2] = {};
     std::vector<std::pair<void*, size_t>> owned;   // blocks from the context's cache, with their sizes
@@ -39,12 +41,18 @@ struct System {
     int alloc_common(const double* pos, const double* vel, const double* h, const fmd_npt* npt);
     int alloc_lists(double rc_list_a, int cap_a, double rc_list_b, int cap_b, bool transpose);
     int alloc_prune(double rc_lj);
+    int alloc_clus(const double* pos);
+    double lazy_edge() const;
+    cudaError_t ensure_full_rows(cudaStream_t st);
+    void set_clus(bool allowed);
+    int retune_lj();
     int upload_topology(const fmd_mm_topology* t);
     int upload_topology_arrays(const fmd_mm_topology* t);
     // One molecule's topology t (indices within the molecule) replicated on
     // the device over nmol contiguous molecules of natom atoms.
     int replicate_topology(const fmd_mm_topology* t, int nmol, int natom);
-    cudaError_t enqueue_rebuild(cudaStream_t st);
+    // lazy: the full LJ rows may stay unbuilt (lazy_edge)
+    cudaError_t enqueue_rebuild(cudaStream_t st, bool lazy = true);
     // The cell-grid half rows and their transpose, gated off on the device
     // when the molecule path built this rebuild (the fallback part of
     // enqueue_rebuild for systems whose full rows come from the candidate
