@@ -228,9 +228,7 @@ cudaError_t lj_gather_launch(int ff, const double* pos, const double* hh, const 
                              DevErr* err = nullptr, const LJPruneOut& po = LJPruneOut{}, int nrec = 0);
 // Rigid site-site LJ (a5-a6): writes F, T; per-block {E, W9} partials (grid n).
 // lab (may be null): scratch of n * natom * 4 doubles for the lab-frame sites;
-// with it (and natom <= 64) the warp-per-neighbour kernel runs, in launch
-// shape 0 (4 warps per molecule), 1 (4 warps, registers capped for 4 blocks
-// per SM) or 2 (8 warps, capped for 2 blocks per SM).
+// with it (and natom <= 64) the warp-per-neighbour kernel runs.
 constexpr int kRigidLabDoubles = 4;   // per site
 // Site pairs within the cutoff (each molecule pair once) into *total
 // (device), by the FP64 test; rebuilds the lab-frame sites in FP64 into lab.
@@ -240,8 +238,36 @@ cudaError_t rigid_count_pairs(const double* pos, const double* qv, const double*
 cudaError_t rigid_launch(int precision, const double* pos, const double* qv, const double* body,
                          const double* hh, const int* cnt, const int* list, int cap, int n,
                          int natom, double rmcut2, double* F, double* T, double* part,
-                         cudaStream_t st, double* lab = nullptr, int shape = 0);
+                         cudaStream_t st, double* lab = nullptr);
 int rigid_grid(int n);
+
+// The same over a symmetric, ascending list of a device-resident system, each
+// molecule pair once (rigidpair.cu): for up to 64 sites.  Memory of
+// rigid_pair_bytes laid out by rigid_pair_layout; rigid_pair_lists after each
+// list build.  rigid_pair_launch evaluates the pairs; the sums are taken by
+// rigid_pair_reduce or by the step's second kick, either with
+// rigid_pair_records partial {E, W9} records.
+constexpr int kRigidListMax = 128;    // list width
+struct RigidPair {
+    int on = 0;
+    int parts = 0, chunks = 0; // warps per molecule, units per own pair
+    void* lab = nullptr;       // [n * natom] lab-frame sites
+    void* own = nullptr;       // [n * cap] each molecule's own pairs
+    int* nown = nullptr;       // [n]
+    int* back = nullptr;       // [n * cap] position of the molecule in its partners' rows
+    double* rec = nullptr;     // [n * cap * chunks * 6] force and torque on the partner of an own pair
+    double* out = nullptr;     // sums of the molecules' parts
+};
+bool rigid_pair_fits(int natom, int cap);
+size_t rigid_pair_bytes(int n, int natom, int cap);
+RigidPair rigid_pair_layout(void* mem, int n, int natom, int cap);
+int rigid_pair_records(int n);
+cudaError_t rigid_pair_lists(const RigidPair& r, const int* cnt, const int* list, int cap, int n, cudaStream_t st);
+cudaError_t rigid_pair_launch(const RigidPair& r, int precision, const double* pos, const double* qv,
+                              const double* body, const double* hh, const int* cnt, const int* list, int cap, int n,
+                              int natom, double rmcut2, cudaStream_t st);
+cudaError_t rigid_pair_reduce(const RigidPair& r, const int* cnt, const int* list, int cap, int n, double* F,
+                              double* T, double* part, cudaStream_t st);
 
 // MM bonded terms (a10-a13): atomics into Facc; partials {E_b,E_a,E_d,E_i, W00,W11,W22}
 struct MMTopoDev {

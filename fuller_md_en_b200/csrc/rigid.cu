@@ -209,9 +209,10 @@ k_rigid(const double* __restrict__ pos, const double* __restrict__ qv, const dou
 }
 
 // ---------------------------------------------------------------------------
-// Warp-per-neighbour variant.  k_rigid_lab writes every molecule's lab-frame
-// sites once per step (the reference computes the whole lab frame first too,
-// LJ:276-291).  In k_rigid_w one CTA owns molecule i; each warp takes one
+// Warp-per-neighbour variant, for callers' lists, which need not be symmetric
+// (a system's are evaluated pair by pair in rigidpair.cu).  k_rigid_lab writes
+// every molecule's lab-frame sites once per step (the reference computes the
+// whole lab frame first too, LJ:276-291).  In k_rigid_w one CTA owns molecule i; each warp takes one
 // listed neighbour j at a time, copies j's sites from the lab array into its
 // own shared-memory slice with coalesced 16/32-byte loads, and lane l handles
 // sites l and l + 32 of i against all sites of j -- no block-wide barrier in
@@ -237,14 +238,13 @@ k_rigid_lab(const double* __restrict__ qv, const double* __restrict__ body, int 
     }
 }
 
-// W warps per molecule; MINB resident blocks per SM requested from the
-// compiler (a register cap: 0 leaves the register count free).
-template <class P, int W, int MINB>
-__global__ void __launch_bounds__(32 * W, MINB)
+constexpr int kRigidWarps = 4;   // warps per molecule
+
+template <class P>
+__global__ void __launch_bounds__(32 * kRigidWarps)
 k_rigid_w(const double* __restrict__ pos, const Site<P>* __restrict__ lab, const double* __restrict__ hh,
           const int* __restrict__ cnt, const int* __restrict__ list, int cap, int n, int natom, double rmcut2,
           RigidConst rc, double* __restrict__ F, double* __restrict__ T, double* __restrict__ part) {
-    constexpr int kRigidWarps = W;
     __shared__ Site<P> lab_i[2 * 32];
     __shared__ Site<P> lab_j[kRigidWarps][2 * 32];
     __shared__ double sm[32 * 16];
@@ -503,22 +503,20 @@ cudaError_t rigid_count_pairs(const double* pos, const double* qv, const double*
 
 cudaError_t rigid_launch(int precision, const double* pos, const double* qv, const double* body,
                          const double* hh, const int* cnt, const int* list, int cap, int n, int natom,
-                         double rmcut2, double* F, double* T, double* part, cudaStream_t st, double* lab,
-                         int shape) {
+                         double rmcut2, double* F, double* T, double* part, cudaStream_t st, double* lab) {
     if (n <= 0) return cudaSuccess;
     if (natom < 1 || natom > kMaxSites) return cudaErrorInvalidValue;
     const RigidConst rc = rigid_const();
     if (lab != nullptr && natom <= 64 && cap <= kRigidMaxNeigh) {
         const int lb = (int)std::min<long long>(((long long)n * natom + 255) / 256, kSMs * 16);
-#define FMD_RW(P, W, MB) \
-    k_rigid_w<P, W, MB><<<n, 32 * W, 0, st>>>(pos, reinterpret_cast<const Site<P>*>(lab), hh, cnt, list, cap, n, natom, \
-                                              rmcut2, rc, F, T, part)
+#define FMD_RW(P) \
+    k_rigid_lab<P><<<lb, 256, 0, st>>>(qv, body, n, natom, reinterpret_cast<Site<P>*>(lab)); \
+    k_rigid_w<P><<<n, 32 * kRigidWarps, 0, st>>>(pos, reinterpret_cast<const Site<P>*>(lab), hh, cnt, list, cap, n, \
+                                                 natom, rmcut2, rc, F, T, part)
         if (precision == FMD_PREC_FP32_PAIR) {
-            k_rigid_lab<float><<<lb, 256, 0, st>>>(qv, body, n, natom, reinterpret_cast<Site<float>*>(lab));
-            if (shape == 1) FMD_RW(float, 4, 4); else if (shape == 2) FMD_RW(float, 8, 2); else FMD_RW(float, 4, 1);
+            FMD_RW(float);
         } else {
-            k_rigid_lab<double><<<lb, 256, 0, st>>>(qv, body, n, natom, reinterpret_cast<Site<double>*>(lab));
-            if (shape == 1) FMD_RW(double, 4, 4); else if (shape == 2) FMD_RW(double, 8, 2); else FMD_RW(double, 4, 1);
+            FMD_RW(double);
         }
 #undef FMD_RW
         return cudaGetLastError();

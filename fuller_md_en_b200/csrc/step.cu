@@ -31,6 +31,7 @@
 #include "geom.cuh"
 #include "sg_host.h"
 #include "pdl.cuh"
+#include "rigidpair.cuh"
 
 namespace fmd {
 namespace {
@@ -510,6 +511,53 @@ __global__ void __launch_bounds__(kPB) k_kick2_end(StepArrays a, StepParams p, i
     end_body(a, p, nblk_f1, gridDim.x, a.lj_blocks, sm, &sS);   // resets kick2_done
 }
 
+// The same for the rigid pair kernel (rigidpair.cu), a warp per molecule: its
+// force and torque are summed here, kept for the next step's first kick and
+// applied by the warp's first lane.  Each block writes one force and one
+// kinetic record.
+__global__ void __launch_bounds__(kPB) k_rigid_kick2_end(StepArrays a, StepParams p) {
+    FMD_PDL_WAIT();
+    __shared__ double sm[32 * kRedFields];
+    __shared__ SysScal sS;
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31;
+    const double hdt = 0.5 * p.dt, sc_v2 = a.S->sc_v2, sc_nh = a.S->sc_nh, cF = kConv / a.Mmol, cT = kConv / a.I0;
+    double tot[kNV], vv = 0.0, ww = 0.0, acc[kNV + 2];
+#pragma unroll
+    for (int k = 0; k < kNV; k++) tot[k] = 0.0;
+    for (int i = blockIdx.x * (kPB / 32) + (threadIdx.x >> 5); i < a.n; i += gridDim.x * (kPB / 32)) {
+        double v[6];
+        rigid_pair_sum(a.rigid_pair, a.cnt_a, a.list_a, a.cap_a, i, lane, v, tot);
+        if (lane == 0)
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                a.F[3 * i + c] = v[c];
+                a.T[3 * i + c] = v[3 + c];
+                const double x = (a.vel[3 * i + c] + hdt * v[c] * cF) * sc_v2;
+                a.vel[3 * i + c] = x;
+                vv += x * x;
+                const double w = (a.omg[3 * i + c] + hdt * v[3 + c] * cT) * sc_nh;
+                a.omg[3 * i + c] = w;
+                ww += w * w;
+            }
+    }
+#pragma unroll
+    for (int k = 0; k < kNV; k++) acc[k] = tot[k];
+    acc[kNV] = vv;
+    acc[kNV + 1] = ww;
+    __shared__ double rec[kNV + 2];
+    block_sum_store<kNV + 2>(acc, sm, rec);
+    if (threadIdx.x < kNV) a.part_f1[(size_t)blockIdx.x * kNV + threadIdx.x] = rec[threadIdx.x];
+    else if (threadIdx.x < kNV + 2) a.part_ke[2 * blockIdx.x + threadIdx.x - kNV] = rec[threadIdx.x];
+    __threadfence();                      // this block's records before its ticket
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&a.S->kick2_done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    end_body(a, p, gridDim.x, gridDim.x, 0, sm, &sS);   // resets kick2_done
+}
+
 __global__ void __launch_bounds__(kRedThreads) k_rescale_end(StepArrays a, StepParams p, int nblk_ke) {
     FMD_PDL_WAIT();
     __shared__ double sm[32 * kRedFields];
@@ -574,6 +622,7 @@ __global__ void __launch_bounds__(kRedThreads) k_force_final(StepArrays a, int n
 }  // namespace
 
 int force_partial_blocks(const StepArrays& a) {
+    if (a.kind == FMD_SYS_RIGID && a.rigid_pair.on) return rigid_pair_records(a.n);
     return a.kind == FMD_SYS_RIGID ? rigid_grid(a.n) : (a.kind == FMD_SYS_AIREBO ? a.rebo_blocks : kForceBlocks);
 }
 
@@ -596,12 +645,23 @@ cudaError_t enqueue_lj(const StepArrays& a, int ff, cudaStream_t st) {
                             a.lj_blocks);
 }
 
-cudaError_t enqueue_forces(const StepArrays& a, cudaStream_t st, bool judge) {
+cudaError_t enqueue_rigid(const StepArrays& a, cudaStream_t st, bool reduce) {
+    const double* hh = a.S->h;
+    if (a.rigid_pair.on) {
+        const cudaError_t e = rigid_pair_launch(a.rigid_pair, a.precision, a.pos, a.qv, a.body, hh, a.cnt_a, a.list_a,
+                                                a.cap_a, a.n, a.natom, a.rmcut2, st);
+        if (e != cudaSuccess || !reduce) return e;
+        return rigid_pair_reduce(a.rigid_pair, a.cnt_a, a.list_a, a.cap_a, a.n, a.F, a.T, a.part_f1, st);
+    }
+    return rigid_launch(a.precision, a.pos, a.qv, a.body, hh, a.cnt_a, a.list_a, a.cap_a, a.n, a.natom, a.rmcut2, a.F,
+                        a.T, a.part_f1, st, a.rigid_lab);
+}
+
+cudaError_t enqueue_forces(const StepArrays& a, cudaStream_t st, bool judge, bool reduce) {
     cudaError_t e = cudaSuccess;
     const double* hh = a.S->h;
     if (a.kind == FMD_SYS_RIGID) {
-        e = rigid_launch(a.precision, a.pos, a.qv, a.body, hh, a.cnt_a, a.list_a, a.cap_a, a.n, a.natom,
-                         a.rmcut2, a.F, a.T, a.part_f1, st, a.rigid_lab, a.rigid_shape);
+        e = enqueue_rigid(a, st, reduce);
     } else if (a.kind == FMD_SYS_AIREBO) {
         if (a.rebo2_flags & FMD_REBO2_BOND_ORDER)
             e = rebo2_launch(a.rebo2, a.pos, hh, a.cnt_b, a.list_b, a.cap_b, a.n, a.Facc, a.part_f1, a.rebo_blocks,
@@ -645,8 +705,12 @@ cudaError_t enqueue_step(const StepArrays& a, const StepParams& p, bool rescale_
     // per-particle kernels: one thread per particle (grid-stride beyond kForceBlocks)
     const int pblocks = std::max(1, std::min(kForceBlocks, (a.n + kPB - 1) / kPB));
     if ((e = launch_pdl(k_begin_kick, dim3(pblocks), dim3(kPB), 0, st, a, p)) != cudaSuccess) return e;
-    if ((e = enqueue_forces(a, st, judge)) != cudaSuccess) return e;
-    if ((e = launch_pdl(k_kick2_end, dim3(pblocks), dim3(kPB), 0, st, a, p, force_partial_blocks(a))) != cudaSuccess)
+    const bool pairs = a.kind == FMD_SYS_RIGID && a.rigid_pair.on;
+    if ((e = enqueue_forces(a, st, judge, !pairs)) != cudaSuccess) return e;
+    if (pairs) {
+        const int blocks = force_partial_blocks(a);
+        if ((e = launch_pdl(k_rigid_kick2_end, dim3(blocks), dim3(kPB), 0, st, a, p)) != cudaSuccess) return e;
+    } else if ((e = launch_pdl(k_kick2_end, dim3(pblocks), dim3(kPB), 0, st, a, p, force_partial_blocks(a))) != cudaSuccess)
         return e;
     if (rescale_phase && p.schedule) {
         if ((e = launch_pdl(k_rescale, dim3(kForceBlocks), dim3(kPB), 0, st, a)) != cudaSuccess) return e;

@@ -58,7 +58,7 @@ struct StepArrays {
     MMTopoDev topo{};
     double rmcut2 = 0, Mmol = 0, I0 = 0;
     double* rigid_lab = nullptr;   // [n * natom * kRigidLabDoubles] lab-frame sites (rigid)
-    int rigid_shape = 0;           // launch shape of the rigid pair kernel (rigid_launch)
+    RigidPair rigid_pair{};        // on: each molecule pair once (rigidpair.cu)
     int precision = FMD_PREC_FP64;
     int quat_left = 0;              // FMD_PHYS_QUAT: the rotation increment multiplies q on the left
     int rebo_phys = 0;              // FMD_PHYS_REBO: bond-order gradient instead of the reference's three-body forces
@@ -93,10 +93,13 @@ struct StepParams {
     int schedule = 0;        // 1: driver schedule, observables and averages (system runs)
 };
 
+// The rigid model's forces and torques of the current state.  reduce false
+// leaves the pair kernel's sums (rigid_pair.on) to the step's second kick.
+cudaError_t enqueue_rigid(const StepArrays& a, cudaStream_t st, bool reduce = true);
 // Force evaluation of the step's kind; fills partials and F (and T).
 // judge: AIREBO with a learned REBO term also runs the plain REBO kernel and
 // compares the two (sg_step.cu).
-cudaError_t enqueue_forces(const StepArrays& a, cudaStream_t st, bool judge = false);
+cudaError_t enqueue_forces(const StepArrays& a, cudaStream_t st, bool judge = false, bool reduce = true);
 // The LJ term alone (ff: FMD_FF_AIREBO / FMD_FF_MM): F = Facc + LJ, Facc zeroed.
 cudaError_t enqueue_lj(const StepArrays& a, int ff, cudaStream_t st);
 // Reduces the force partials into S->W9 / S->E (one small kernel).

@@ -91,7 +91,7 @@ int System::alloc_common(const double* pos_h, const double* vel_h, const double*
         alloc(&arr.part_f1, (size_t)std::max(kForceBlocks, n) * kNV, (const double*)nullptr) ||
         alloc(&arr.part_f2, (size_t)kLJMaxBlocks * kNV, (const double*)nullptr) ||
         alloc(&arr.part_f3, (size_t)kForceBlocks, (const double*)nullptr) ||
-        alloc(&arr.part_ke, (size_t)kForceBlocks * 2, (const double*)nullptr) ||
+        alloc(&arr.part_ke, (size_t)std::max(kForceBlocks, (n + 7) / 8) * 2, (const double*)nullptr) ||
         alloc(&dropped, 2, (const int*)nullptr) || alloc(&arr.S, 1, (const SysScal*)nullptr))
         return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
     arr.err = ctx->d_err;
@@ -244,8 +244,10 @@ cudaError_t System::enqueue_rebuild(cudaStream_t st, bool lazy) {
     int* list_a = const_cast<int*>(arr.list_a);
     if (arr.kind == FMD_SYS_RIGID) {
         if ((e = cells_build(cells_a, arr.pos, arr.n, hh, rc_a, ctx->d_err, st)) != cudaSuccess) return e;
-        return nlist_build(cells_a, LIST_SYM, arr.pos, nullptr, arr.n, hh, rc2_a, arr.cap_a, cnt_a, list_a,
-                           dropped, ctx->d_err, st);
+        if ((e = nlist_build(cells_a, LIST_SYM, arr.pos, nullptr, arr.n, hh, rc2_a, arr.cap_a, cnt_a, list_a, dropped,
+                             ctx->d_err, st)) != cudaSuccess)
+            return e;
+        return arr.rigid_pair.on ? rigid_pair_lists(arr.rigid_pair, cnt_a, list_a, arr.cap_a, arr.n, st) : cudaSuccess;
     }
     if (arr.kind == FMD_SYS_AIREBO) {
         if (mol.ok) {
@@ -556,47 +558,6 @@ int System::tune_lj_pruned(bool run_tuner, bool* pending) {
     return FMD_OK;
 }
 
-// Launch shape of the rigid pair kernel, timed on this system's own list at
-// set-up (the pair kernel writes F, T and partials only, which the first
-// force evaluation below recomputes); cached per (device, molecules, sites,
-// precision).
-int System::tune_rigid() {
-    static std::map<std::tuple<int, int, int, int>, int> cache;
-    const auto key = std::make_tuple(ctx->device, arr.n, arr.natom, arr.precision);
-    auto it = cache.find(key);
-    if (it != cache.end()) {
-        arr.rigid_shape = it->second;
-        return FMD_OK;
-    }
-    cudaStream_t st = ctx->stream;
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    float best = 1e30f;
-    int pick = 0;
-    for (int shape : {0, 1, 2}) {
-        auto go = [&]() {
-            return rigid_launch(arr.precision, arr.pos, arr.qv, arr.body, arr.S->h, arr.cnt_a, arr.list_a, arr.cap_a,
-                                arr.n, arr.natom, arr.rmcut2, arr.F, arr.T, arr.part_f1, st, arr.rigid_lab, shape);
-        };
-        go();
-        cudaEventRecord(e0, st);
-        for (int r = 0; r < 3; r++) go();
-        cudaEventRecord(e1, st);
-        cudaEventSynchronize(e1);
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best) { best = ms; pick = shape; }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    const int rc = ctx->sync_check("rigid launch-shape tuning");
-    if (rc != FMD_OK) return rc;
-    cache[key] = pick;
-    arr.rigid_shape = pick;
-    return FMD_OK;
-}
-
 int System::init() {
     cudaStream_t st = ctx->stream;
     // Pre-loop order of the reference: lists from the unwrapped positions,
@@ -608,9 +569,6 @@ int System::init() {
     if (apply_pbc_launch(arr.pos, arr.n, arr.S->h, st) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "apply_pbc failed");
     if (arr.kind != FMD_SYS_RIGID) {
         const int rc = tune_lj();
-        if (rc != FMD_OK) return rc;
-    } else {
-        const int rc = tune_rigid();
         if (rc != FMD_OK) return rc;
     }
     if (enqueue_forces(arr, st) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "force launch failed");
@@ -769,6 +727,12 @@ extern "C" int fmd_system_create_rigid(fmd_ctx* ctx, const fmd_run_params* p, in
     // beyond rmcut (LJ:320).
     if ((rc = s->alloc_lists(rmc, max_neigh, 0.0, 0, false)) != FMD_OK) return rc;
     s->rc2_a = rmc * rmc;
+    if (rigid_pair_fits(natom, max_neigh)) {
+        char* mem;
+        if (s->alloc(&mem, rigid_pair_bytes(n, natom, max_neigh), (const char*)nullptr))
+            return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
+        s->arr.rigid_pair = rigid_pair_layout(mem, n, natom, max_neigh);
+    }
     out[0] = new fmd_system{std::move(s)};
     return FMD_OK;
 }
@@ -1133,8 +1097,7 @@ extern "C" int fmd_system_kernel_ms(fmd_system* s, int stage, int reps, double* 
         switch (stage) {
             case 0:
                 if (a.kind == FMD_SYS_RIGID)
-                    return rigid_launch(a.precision, a.pos, a.qv, a.body, hh, a.cnt_a, a.list_a, a.cap_a, a.n,
-                                        a.natom, a.rmcut2, a.F, a.T, a.part_f1, st, a.rigid_lab, a.rigid_shape);
+                    return enqueue_rigid(a, st);
                 // Timed into the scratch accumulator (F itself is left alone).
                 return lj_gather_launch(a.kind == FMD_SYS_AIREBO ? FMD_FF_AIREBO : FMD_FF_MM, a.pos, hh, a.cnt_a,
                                         a.list_a, a.cap_a, a.in_cnt, a.in_list, a.in_cap, a.n, a.Facc, a.Facc,
@@ -1149,8 +1112,7 @@ extern "C" int fmd_system_kernel_ms(fmd_system* s, int stage, int reps, double* 
                     return rebo_slots_launch(a.pos, hh, a.cnt_b, a.list_b, a.cap_b, a.n, a.rebo_slots, a.Facc,
                                              a.part_f1, kForceBlocks, nullptr, 0, st, a.rebo_ids, a.rebo_phys != 0);
                 if (a.kind == FMD_SYS_MM) return mm_bonded_launch(a.topo, a.pos, hh, a.Facc, a.part_f1, st);
-                return rigid_launch(a.precision, a.pos, a.qv, a.body, hh, a.cnt_a, a.list_a, a.cap_a, a.n, a.natom,
-                                    a.rmcut2, a.F, a.T, a.part_f1, st, a.rigid_lab, a.rigid_shape);
+                return enqueue_rigid(a, st);
             case 2:
                 y.full_rows_stale = a.clus.on;
                 return y.enqueue_rebuild(st);

@@ -69,7 +69,6 @@ struct System {
     int tune_lj_pruned(bool run_tuner, bool* pending);
     LJShape pick_lj_shape(bool pruned, int& rc);
     void set_lj_blocks();
-    int tune_rigid();
     int capture(bool rebuild, bool phase, bool judge = false);
     void drop_graphs();
     int use_surrogate(fmd_sg* model, int judge_every, double rmse_max);
