@@ -234,7 +234,10 @@ __global__ void __launch_bounds__(kPB) k_begin_kick(StepArrays a, StepParams p) 
     int* dst = reinterpret_cast<int*>(&sS);
     for (int k = threadIdx.x; k < kWords; k += blockDim.x) dst[k] = src[k];
     __syncthreads();
-    if (threadIdx.x == 0) begin_body(&sS, a.kind, p);
+    if (threadIdx.x == 0) {
+        begin_body(&sS, a.kind, p);
+        sS.kick_done = 0u;                     // a block that starts late has copied other blocks' tickets
+    }
     __syncthreads();
     kick_body(a, p.dt, blockIdx.x, gridDim.x, &sS);
     __syncthreads();
@@ -242,7 +245,7 @@ __global__ void __launch_bounds__(kPB) k_begin_kick(StepArrays a, StepParams p) 
     __syncthreads();
     if (!last) return;
     int* out = reinterpret_cast<int*>(a.S);
-    for (int k = threadIdx.x; k < kWords; k += blockDim.x) out[k] = dst[k];   // kick_done: 0 again
+    for (int k = threadIdx.x; k < kWords; k += blockDim.x) out[k] = dst[k];
 }
 
 __global__ void __launch_bounds__(kPB) k_ke_partial(StepArrays a) {
