@@ -327,7 +327,7 @@ int upload_scal(fmd_ctx* ctx, const double* h, const double* hi, const double* W
 int alloc_partials(fmd_ctx* ctx, StepArrays& a) {
     int rc = up<double>(ctx, S_PART1, nullptr, (size_t)std::max(kForceBlocks, a.n) * kNV, &a.part_f1);
     if (!rc) rc = up<double>(ctx, S_PART2, nullptr, (size_t)kLJMaxBlocks * kNV, &a.part_f2);
-    a.lj_blocks = lj_gather_blocks(a.kind == FMD_SYS_MM ? FMD_FF_MM : FMD_FF_AIREBO, a.precision, a.lj_shape, 0);
+    a.lj_blocks = lj_gather_blocks(a.kind == FMD_SYS_MM ? FMD_FF_MM : FMD_FF_AIREBO, a.precision, a.lj_shape, 0, a.n);
     if (!rc) rc = up<double>(ctx, S_PART3, nullptr, (size_t)kForceBlocks, &a.part_f3);
     if (!rc) rc = up<double>(ctx, S_PARTKE, nullptr, (size_t)kForceBlocks * 2, &a.part_ke);
     return rc;
@@ -468,7 +468,7 @@ static int atom_term(fmd_ctx* ctx, int term, int ff, const double* pos, const do
     }
     double* red;
     if ((rc = up<double>(ctx, S_PART3, nullptr, 16, &red))) return rc;
-    if (reduce_partials(part, term == 0 ? kForceBlocks : lj_gather_blocks(ff, ctx->precision, LJShape{}, 0), kNV, red,
+    if (reduce_partials(part, term == 0 ? kForceBlocks : lj_gather_blocks(ff, ctx->precision, LJShape{}, 0, na), kNV, red,
                         ctx->stream) != cudaSuccess)
         return ctx->fail(FMD_ERR_CUDA, "reduce launch failed");
     double r[kNV];

@@ -825,6 +825,11 @@ cudaError_t rebo_launch_gated(const double* pos, const double* hh, const int* cn
     return cudaGetLastError();
 }
 
+// Eight slots an atom (three bonds and the second neighbours that thermal motion
+// brings inside the list radius; half as many blocks cost a second pass), a thread
+// each; a system with more per atom takes them in the grid's stride.
+int rebo_slot_blocks(int na) { return std::max(1, std::min(kForceBlocks, (8 * na + 255) / 256)); }
+
 cudaError_t rebo_slots_launch(const double* pos, const double* hh, const int* cnt, const int* list, int cap,
                               int na, double* slots, double* F, double* part, int nblocks, const int* gate,
                               int want, cudaStream_t st, const int* ids, bool phys) {
@@ -832,7 +837,7 @@ cudaError_t rebo_slots_launch(const double* pos, const double* hh, const int* cn
     SlotBO* bo = reinterpret_cast<SlotBO*>(slots + (size_t)na * cap * 8);
     cudaError_t e;
     if (ids) {
-        if ((e = launch_pdl(k_rebo_geo_bo, dim3(kForceBlocks), dim3(256), 0, st, pos, hh, cnt, list, cap, sl, bo,
+        if ((e = launch_pdl(k_rebo_geo_bo, dim3(rebo_slot_blocks(na)), dim3(256), 0, st, pos, hh, cnt, list, cap, sl, bo,
                             gate, want, ids)) != cudaSuccess)
             return e;
     } else {
@@ -943,6 +948,9 @@ cudaError_t rebo_ids_build(const int* cnt, const int* list, int cap, int n, int*
 
 namespace {
 
+// Blocks that give every atom a warp: more would only add empty records.
+int lj_warp_blocks(int na, int threads) { return std::max(1, (na + threads / 32 - 1) / (threads / 32)); }
+
 // Resident blocks per SM of one LJ gather instantiation (queried once).
 template <bool FV, bool F32, int U, bool PIPE, int NT>
 int lj_occupancy() {
@@ -960,7 +968,7 @@ template <bool FV, bool F32, int U, bool PIPE, int NT>
 int lj_dispatch(bool launch, const double* pos, const double* hh, const int* cnt, const int* list, int cap,
                 const int* in_cnt, const int* in_list, int in_cap, int na, double* F, double* Facc, const LJP& p,
                 double* part, cudaStream_t st, const LJPruneOut& po, int nrec, int contig) {
-    const int nb = std::min(kLJMaxBlocks, lj_occupancy<FV, F32, U, PIPE, NT>() * kSMs);
+    const int nb = std::min({kLJMaxBlocks, lj_occupancy<FV, F32, U, PIPE, NT>() * kSMs, lj_warp_blocks(na, NT)});
     if (launch)
         launch_pdl(k_lj_gather<FV, F32, U, PIPE, NT>, dim3(nb), dim3(NT), 0, st, pos, hh, in_cnt, in_list, in_cap, na,
                    F, Facc, p, part, po, nrec, contig);
@@ -990,7 +998,7 @@ int lj_dispatch_staged(bool launch, const double* pos, const double* hh, const i
         it = occ.emplace(in_cap, b).first;
     }
     if (it->second < 1) return 0;
-    const int nb = std::min(kLJMaxBlocks, it->second * kSMs);
+    const int nb = std::min({kLJMaxBlocks, it->second * kSMs, lj_warp_blocks(na, NT)});
     if (launch)
         launch_pdl(k_lj_gather_staged<FV, F32, U, NT>, dim3(nb), dim3(NT), smem, st, pos, hh, in_cnt, in_list, in_cap,
                    na, F, Facc, p, part, err, po, nrec, contig);
@@ -1035,8 +1043,8 @@ int lj_select(bool launch, int ff, int precision, const LJShape& sh, const doubl
 
 }  // namespace
 
-int lj_gather_blocks(int ff, int precision, const LJShape& sh, int in_cap) {
-    return lj_select(false, ff, precision, sh, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, in_cap, 0,
+int lj_gather_blocks(int ff, int precision, const LJShape& sh, int in_cap, int na) {
+    return lj_select(false, ff, precision, sh, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, in_cap, na,
                      nullptr, nullptr, nullptr, nullptr);
 }
 

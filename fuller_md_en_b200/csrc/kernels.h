@@ -90,6 +90,7 @@ cudaError_t rebo_launch_gated(const double* pos, const double* hh, const int* cn
 // na * cap bond-order records; device scratch owned by the caller); otherwise
 // as rebo_launch_gated (gate may be null).
 constexpr int kReboSlotDoubles = 16;
+int rebo_slot_blocks(int na);   // a grid for the occupied slots of na atoms
 // ids (may be null): the occupied slots in atom-major order packed into
 // 32-lane bins (no atom's slots cross a bin; unused lanes -1), ids[0] the
 // padded length and ids[1 + k] the slot i * cap + jn, then at
@@ -160,7 +161,8 @@ int rebo_ids_scratch(int n);
 // and the row feed (pipe 0: loads as used, 1: software-pipelined loads,
 // 2: rows staged in shared memory by bulk asynchronous copies, needs
 // in_cap % 4 == 0 and an error word); the grid is one full wave of the
-// instantiation (resident blocks per SM x SMs, at most kLJMaxBlocks) and
+// instantiation (resident blocks per SM x SMs, at most kLJMaxBlocks and a warp
+// per atom) and
 // writes that many partial records -- lj_gather_blocks returns it (0: the
 // shape cannot run with this row stride).  po.cnt non-null: a pruning
 // gather, which also writes per atom i the entries of its row with
@@ -190,7 +192,7 @@ struct LJPruneOut {
     const double* hb = nullptr;
     double delta = 0.0, rc = 0.0;
 };
-int lj_gather_blocks(int ff, int precision, const LJShape& shape, int in_cap);
+int lj_gather_blocks(int ff, int precision, const LJShape& shape, int in_cap, int na);
 
 // Cluster rows of the atomistic LJ gather (ljclus.cu): kClusG atoms of one
 // molecule share one pruned row, each entry naming a partner atom, the
@@ -291,6 +293,7 @@ struct MMTopoOut {
 // molecule's term k with every index offset by m natom, copies in order,
 // each term kind molecule-major.  `mol` holds one molecule's terms.
 cudaError_t mm_replicate_launch(const MMTopoDev& mol, int nmol, int natom, const MMTopoOut& out, cudaStream_t st);
+int mm_bonded_blocks(const MMTopoDev& t);   // partial records
 cudaError_t mm_bonded_launch(const MMTopoDev& t, const double* pos, const double* hh, double* Facc,
                              double* part, cudaStream_t st);
 // Cut Coulomb (a15), all pairs of different molecules: adds into Facc; {Ecoul} partials.

@@ -25,14 +25,20 @@ __host__ __device__ inline unsigned long long lj_rows_tag(unsigned long long kin
 // gather and the step's reduction evaluate it on the same, unchanged inputs.
 __device__ __forceinline__ bool lj_prune_needed(const unsigned long long* words, const double* hh, const double* hb,
                                                 double delta, double rc, unsigned long long kind) {
-    if (words[1] != lj_rows_tag(kind, delta)) return true;
+    // every load first, so that they cost one latency together
+    const unsigned long long tag = words[1];
     const double u = __longlong_as_double((long long)words[0]);
+    double h[9], b[9];
+#pragma unroll
+    for (int a = 0; a < 9; a++) { h[a] = hh[a]; b[a] = hb[a]; }
     double k = 0.0;
-    for (int a = 0; a < 3; a++) k = fmax(k, fabs(hh[4 * a] - hb[4 * a]) / fabs(hb[4 * a]));
-    const bool diag = hh[1] == 0.0 && hh[2] == 0.0 && hh[3] == 0.0 && hh[5] == 0.0 && hh[6] == 0.0 &&
-                      hh[7] == 0.0 && hb[1] == 0.0 && hb[2] == 0.0 && hb[3] == 0.0 && hb[5] == 0.0 &&
-                      hb[6] == 0.0 && hb[7] == 0.0;
-    return !(diag && k * (rc + delta) + 2.0 * u < delta - 1e-6);
+#pragma unroll
+    for (int a = 0; a < 3; a++) k = fmax(k, fabs(h[4 * a] - b[4 * a]) / fabs(b[4 * a]));
+    bool diag = true;
+#pragma unroll
+    for (int a = 0; a < 9; a++)
+        if (a % 4 != 0) diag = diag && h[a] == 0.0 && b[a] == 0.0;
+    return tag != lj_rows_tag(kind, delta) || !(diag && k * (rc + delta) + 2.0 * u < delta - 1e-6);
 }
 
 }  // namespace fmd

@@ -254,9 +254,14 @@ cudaError_t mm_replicate_launch(const MMTopoDev& mol, int nmol, int natom, const
     return cudaGetLastError();
 }
 
+int mm_bonded_blocks(const MMTopoDev& t) {
+    const long long terms = (long long)t.nb + t.nang + t.ndih + t.nimp;
+    return (int)std::max(1LL, std::min<long long>(kForceBlocks, (terms + 127) / 128));
+}
+
 cudaError_t mm_bonded_launch(const MMTopoDev& t, const double* pos, const double* hh, double* Facc,
                              double* part, cudaStream_t st) {
-    k_mm_bonded<<<kForceBlocks, 128, 0, st>>>(t, pos, hh, Facc, part);
+    k_mm_bonded<<<mm_bonded_blocks(t), 128, 0, st>>>(t, pos, hh, Facc, part);
     return cudaGetLastError();
 }
 

@@ -123,7 +123,24 @@ __device__ __forceinline__ void quat_step(double* q, double wx, double wy, doubl
 
 }  // namespace
 
-__device__ void kick_body(const StepArrays& a, double dt, int blk, int nblk, const SysScal* sc = nullptr) {
+// What the first kick reads of particle i.
+struct KickIn {
+    double v[3], F[3], p[3], m, sb[3];
+};
+__device__ __forceinline__ KickIn kick_load(const StepArrays& a, int i) {
+    KickIn k;
+    k.m = a.mass != nullptr ? a.mass[i] : 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        k.v[c] = a.vel[3 * i + c]; k.F[c] = a.F[3 * i + c]; k.p[c] = a.pos[3 * i + c];
+        k.sb[c] = a.prune_sb ? a.prune_sb[3 * i + c] : 0.0;
+    }
+    return k;
+}
+
+// in: the thread's first particle, already loaded.
+__device__ void kick_body(const StepArrays& a, double dt, int blk, int nblk, const SysScal* sc = nullptr,
+                          const KickIn* in = nullptr) {
     const SysScal* S = sc ? sc : a.S;
     const double hdt = 0.5 * dt, sc_v = S->sc_v, sc_nh = S->sc_nh;
     const double* hi = S->hi_old;
@@ -132,12 +149,16 @@ __device__ void kick_body(const StepArrays& a, double dt, int blk, int nblk, con
     const double cF = rigid ? kConv / a.Mmol : kConv / kMC, cT = rigid ? kConv / a.I0 : 0.0;
     double u2 = 0.0;   // largest squared displacement since the last LJ prune
     for (int i = blk * blockDim.x + threadIdx.x; i < a.n; i += nblk * blockDim.x) {
-        const double mi = (a.mass != nullptr) ? kConv / a.mass[i] : cF;
-        double v[3], p[3];
+        KickIn k;
+        if (in) k = *in;
+        else k = kick_load(a, i);
+        in = nullptr;
+        const double mi = (a.mass != nullptr) ? kConv / k.m : cF;
+        double v[3];
+        const double* p = k.p;
         for (int c = 0; c < 3; c++) {
-            v[c] = a.vel[3 * i + c] * sc_v + hdt * a.F[3 * i + c] * mi;
+            v[c] = k.v[c] * sc_v + hdt * k.F[c] * mi;
             a.vel[3 * i + c] = v[c];
-            p[c] = a.pos[3 * i + c];
         }
         double sx = hi[0] * p[0] + hi[1] * p[1] + hi[2] * p[2];
         double sy = hi[3] * p[0] + hi[4] * p[1] + hi[5] * p[2];
@@ -152,7 +173,7 @@ __device__ void kick_body(const StepArrays& a, double dt, int blk, int nblk, con
         a.pos[3 * i + 2] = h[6] * sx + h[7] * sy + h[8] * sz;
         if (a.prune_sb) {
             // nearest-image fractional displacement, measured in the new cell
-            double ex = sx - a.prune_sb[3 * i], ey = sy - a.prune_sb[3 * i + 1], ez = sz - a.prune_sb[3 * i + 2];
+            double ex = sx - k.sb[0], ey = sy - k.sb[1], ez = sz - k.sb[2];
             const double kx = rint(ex), ky = rint(ey), kz = rint(ez);
             ex -= kx; ey -= ky; ez -= kz;
             if (a.clus.on) {
@@ -234,12 +255,16 @@ __global__ void __launch_bounds__(kPB) k_begin_kick(StepArrays a, StepParams p) 
     int* dst = reinterpret_cast<int*>(&sS);
     for (int k = threadIdx.x; k < kWords; k += blockDim.x) dst[k] = src[k];
     __syncthreads();
+    // the particles' loads wait beside thread 0's scalars
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    KickIn in;
+    if (i0 < a.n) in = kick_load(a, i0);
     if (threadIdx.x == 0) {
         begin_body(&sS, a.kind, p);
         sS.kick_done = 0u;                     // a block that starts late has copied other blocks' tickets
     }
     __syncthreads();
-    kick_body(a, p.dt, blockIdx.x, gridDim.x, &sS);
+    kick_body(a, p.dt, blockIdx.x, gridDim.x, &sS, &in);
     __syncthreads();
     if (threadIdx.x == 0) last = atomicAdd(&a.S->kick_done, 1u) == gridDim.x - 1;
     __syncthreads();
@@ -300,53 +325,96 @@ __global__ void __launch_bounds__(kPB) k_rescale(StepArrays a) {
     rescale_body(a, blockIdx.x, gridDim.x, sm);
 }
 
-// One pass over every partial array: each thread sums its strided records
-// (fixed order), then one CTA reduction for all fields.  Layout of t[]:
-// [0,10) part_f1 fields, [10,20) part_f2 fields, [20] part_f3, [21,23) kinetic.
+// Sums of the partial records, t[]: [0,10) part_f1 fields, [10,20) part_f2
+// fields, [20] part_f3, [21,23) kinetic; valid in every thread.  The record
+// arrays are read as they lie, element by element across the threads (a thread
+// stride that is a multiple of the record width keeps a thread on one field),
+// the first loads of all arrays before any is used; then a warp sums the
+// threads of a field.  Fixed order.  The step's end is one block's latency, so
+// code and waits are kept short: k_kick2_end takes 7.6 us at 1,920 atoms and
+// 9.5 us at 30,000, against 12.0 and 13.2 us when a thread walked whole records
+// 80 bytes from its neighbour's, 23 fields were summed over the block one
+// after the other and one thread did all scalar work.
 constexpr int kRedFields = 23;
+constexpr int kRedShared = 4 * kRedThreads + kRedFields + 1;
 
-__device__ void reduce_all(const StepArrays& a, int nblk_f1, int nblk_ke, bool forces, bool kinetic,
-                           double* sm, double (&t)[kRedFields], int nblk_f2) {
-    double acc[kRedFields];
-#pragma unroll
-    for (int k = 0; k < kRedFields; k++) acc[k] = 0.0;
-    // L2 loads (__ldcg): the fused second kick reduces records that other
-    // blocks of the same launch have just written.
-    if (forces) {
-        // record widths as compile-time constants so each thread's loads issue together
-        if (a.kind == FMD_SYS_MM) {
-            for (int b = threadIdx.x; b < nblk_f1; b += blockDim.x)
-#pragma unroll
-                for (int k = 0; k < kMMNV; k++) acc[k] += __ldcg(a.part_f1 + (size_t)b * kMMNV + k);
-        } else {
-            for (int b = threadIdx.x; b < nblk_f1; b += blockDim.x)
-#pragma unroll
-                for (int k = 0; k < kNV; k++) acc[k] += __ldcg(a.part_f1 + (size_t)b * kNV + k);
-        }
-        if (a.kind != FMD_SYS_RIGID)
-            for (int b = threadIdx.x; b < nblk_f2; b += blockDim.x) {
-#pragma unroll
-                for (int k = 0; k < kNV; k++) acc[10 + k] += __ldcg(a.part_f2 + (size_t)b * kNV + k);
-            }
-        if (a.kind == FMD_SYS_MM && a.has_charge)
-            for (int b = threadIdx.x; b < kForceBlocks; b += blockDim.x) acc[20] += __ldcg(a.part_f3 + b);
-        // the switched-LJ correction belongs to the LJ term
-        if (a.kind == FMD_SYS_AIREBO && (a.rebo2_flags & FMD_REBO2_LJ_SWITCH))
-            for (int b = threadIdx.x; b < kForceBlocks; b += blockDim.x) {
-#pragma unroll
-                for (int k = 0; k < kNV; k++) acc[10 + k] += __ldcg(a.part_sw + (size_t)b * kNV + k);
-            }
+// Threads that read an array of this record width.
+__device__ __forceinline__ int red_stride(int width) {
+    const bool half = blockDim.x == 256;
+    return width == 10 ? (half ? 250 : 510) : (width == 7 ? (half ? 252 : 511) : (int)blockDim.x);
+}
+
+// One array's sum by threads: NU loads, then the rest NU at a time.
+template <int NU>
+struct FlatSum {
+    const double* part;
+    int stride, n, e;
+    double v[NU];
+    __device__ __forceinline__ FlatSum(const double* p, int nrec, int width)
+        : part(p), stride(red_stride(width)), n((int)threadIdx.x < stride ? nrec * width : 0), e(threadIdx.x) {
+        load();
     }
-    if (kinetic)
-        for (int b = threadIdx.x; b < nblk_ke; b += blockDim.x) {
-            acc[21] += __ldcg(a.part_ke + 2 * b);
-            acc[22] += __ldcg(a.part_ke + 2 * b + 1);
+    __device__ __forceinline__ void load() {               // L2: other blocks of the launch wrote them
+#pragma unroll
+        for (int u = 0; u < NU; u++) v[u] = e + u * stride < n ? __ldcg(part + e + u * stride) : 0.0;
+        e += NU * stride;
+    }
+    __device__ __forceinline__ double sum() {
+        double acc = 0.0;
+        for (;;) {
+#pragma unroll
+            for (int u = 0; u < NU; u++) acc += v[u];
+            if (e >= n) return acc;
+            load();
         }
-    block_sum_store<kRedFields>(acc, sm, t);   // result valid in thread 0
+    }
+};
+
+__device__ void reduce_all(const StepArrays& a, int nblk_f1, int nblk_ke, bool forces, bool kinetic, double* sm,
+                           const double*& t, int nblk_f2) {
+    const int nt = blockDim.x, w1 = a.kind == FMD_SYS_MM ? kMMNV : kNV;
+    {
+        FlatSum<2> k(a.part_ke, kinetic ? nblk_ke : 0, 2);
+        FlatSum<8> f1(a.part_f1, forces ? nblk_f1 : 0, w1), f2(a.part_f2, forces && a.kind != FMD_SYS_RIGID ? nblk_f2 : 0, kNV);
+        sm[3 * nt + threadIdx.x] = k.sum();
+        sm[threadIdx.x] = f1.sum();
+        double v2 = f2.sum(), v3 = 0.0;
+        if (forces && a.kind == FMD_SYS_MM && a.has_charge) v3 = FlatSum<2>(a.part_f3, kForceBlocks, 1).sum();
+        // the switched-LJ correction belongs to the LJ term
+        if (forces && a.kind == FMD_SYS_AIREBO && (a.rebo2_flags & FMD_REBO2_LJ_SWITCH))
+            v2 += FlatSum<8>(a.part_sw, kForceBlocks, kNV).sum();
+        sm[nt + threadIdx.x] = v2;
+        sm[2 * nt + threadIdx.x] = v3;
+    }
+    __syncthreads();
+    double* out = sm + 4 * kRedThreads;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    constexpr int kRounds = 3;                             // of 8 (16) warps
+    double x[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; r++) {
+        const int f = w + r * (nt >> 5);
+        const int arr = f < 10 ? 0 : (f < 20 ? 1 : (f < 21 ? 2 : 3));
+        const int width = arr == 0 ? w1 : (arr == 1 ? kNV : (arr == 2 ? 1 : 2));
+        const int k = f < 20 ? f - 10 * arr : (f < 21 ? 0 : f - 21), end = red_stride(width);
+        x[r] = 0.0;
+        if (f < kRedFields && k < width)
+            for (int q = lane * width + k; q < end; q += 32 * width) x[r] += sm[arr * nt + q];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < kRounds; r++) x[r] += __shfl_xor_sync(kFull, x[r], o);
+    if (lane == 0)
+#pragma unroll
+        for (int r = 0; r < kRounds; r++)
+            if (w + r * (nt >> 5) < kRedFields) out[w + r * (nt >> 5)] = x[r];
+    __syncthreads();
+    t = out;
 }
 
 // Thread 0: kinetic energies from the reduced sums into S (a.S or a copy).
-__device__ void kinetic_from_sums(SysScal* S, const StepArrays& a, const double (&t)[kRedFields]) {
+__device__ void kinetic_from_sums(SysScal* S, const StepArrays& a, const double* t) {
     if (a.kind == FMD_SYS_RIGID) {
         S->kt = 0.5 * a.Mmol * t[21] / kConv;     // LJ:411
         S->kr = 0.5 * a.I0 * t[22] / kConv;       // LJ:420
@@ -356,50 +424,54 @@ __device__ void kinetic_from_sums(SysScal* S, const StepArrays& a, const double 
     }
 }
 
-// Thread 0: virial and energies (program grouping) from the reduced sums
-// into S (a.S or a copy).
-__device__ void forces_from_sums(SysScal* S, const StepArrays& a, const double (&t)[kRedFields]) {
-    double e[8] = {0, 0, 0, 0, 0, 0, 0, 0}, w[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (a.kind == FMD_SYS_RIGID) {
-        e[0] = t[0];
-        for (int q = 0; q < 9; q++) w[q] = t[1 + q];
-    } else if (a.kind == FMD_SYS_AIREBO) {
-        e[1] = t[0]; e[2] = t[10]; e[0] = e[1] + e[2];
-        for (int q = 0; q < 9; q++) w[q] = t[1 + q] + t[11 + q];
-    } else {
-        for (int q = 0; q < 4; q++) e[q] = t[q];
-        e[4] = t[10];
-        e[5] = a.has_charge ? t[20] : 0.0;
-        e[6] = e[0] + e[1] + e[2] + e[3] + e[4] + e[5];
-        const int d[3] = {0, 4, 8};
-        for (int q = 0; q < 3; q++) w[d[q]] = t[4 + q] + t[11 + d[q]];
-    }
-    for (int q = 0; q < 9; q++) S->W9[q] = w[q];
-    for (int q = 0; q < 8; q++) S->E[q] = e[q];
+// Virial entry q and energy q (program grouping) from the reduced sums.
+__device__ __forceinline__ double virial_of(int kind, const double* t, int q) {
+    if (kind == FMD_SYS_RIGID) return t[1 + q];
+    if (kind == FMD_SYS_AIREBO) return t[1 + q] + t[11 + q];
+    return q % 4 == 0 ? t[4 + q / 4] + t[11 + q] : 0.0;
+}
+__device__ __forceinline__ double energy_of(const StepArrays& a, const double* t, int q) {
+    if (a.kind == FMD_SYS_RIGID) return q == 0 ? t[0] : 0.0;
+    if (a.kind == FMD_SYS_AIREBO) return q == 0 ? t[0] + t[10] : (q == 1 ? t[0] : (q == 2 ? t[10] : 0.0));
+    const double ec = a.has_charge ? t[20] : 0.0;
+    return q < 4 ? t[q] : (q == 4 ? t[10] : (q == 5 ? ec : (q == 6 ? t[0] + t[1] + t[2] + t[3] + t[10] + ec : 0.0)));
 }
 
-// Observables, averages and the monitor record (LJ:874-897, AI:896-912, MM:1215-1236).
-__device__ void record(SysScal* S, int kind, const StepParams& p) {
+// Threads 32.. of the block: virial and energies into S (a.S or a copy).
+__device__ __forceinline__ void forces_from_sums(SysScal* S, const StepArrays& a, const double* t) {
+    const int q = (int)threadIdx.x - 32;
+    if (q >= 0 && q < 9) S->W9[q] = virial_of(a.kind, t, q);
+    if (q >= 32 && q < 40) S->E[q - 32] = energy_of(a, t, q - 32);
+}
+
+// Observables, averages and the monitor record (LJ:874-897, AI:896-912,
+// MM:1215-1236), by threads of one block on S: thread 0 temperature, pressure,
+// lattice constant and kinetic energy, eight threads from first the energies,
+// each its own (e: energy q, d: the energy of the q-th average).
+__device__ __forceinline__ void record_state(SysScal* S, const StepParams& p) {
     const int g = S->gstep;
     const double an = S->h[0] / p.nc;
     S->an = an;
     if (g >= p.gavg_from && g <= p.gavg_to) {
         fmd_avg& A = S->avg;
         A.sT += S->Tn; A.sP += S->Pn; A.sa += an;
-        if (kind == FMD_SYS_RIGID) {
-            A.sE[0] += S->E[0] / p.nmol;
-        } else if (kind == FMD_SYS_AIREBO) {
-            A.sE[0] += S->E[1] / p.nmol; A.sE[1] += S->E[2] / p.nmol; A.sE[2] += S->E[0] / p.nmol;
-        } else {
-            A.sE[0] += S->E[0] / p.nmol; A.sE[1] += S->E[1] / p.nmol;
-            A.sE[2] += (S->E[2] + S->E[3]) / p.nmol; A.sE[3] += S->E[4] / p.nmol;
-            A.sE[4] += S->E[6] / p.nmol;
-        }
         A.n++;
     }
     fmd_obs& o = S->obs;
     o.step = g; o.T = S->Tn; o.P = S->Pn; o.a = an; o.KE = S->KE;
-    for (int q = 0; q < 8; q++) o.E[q] = S->E[q];
+}
+// The energy of the program's q-th average: rigid {Ep}; AIREBO {REBO, LJ,
+// total}; MM {bond, angle, dihedral + improper, LJ, total}.
+__device__ __forceinline__ double average_energy(int kind, const double* E, int q) {
+    if (kind == FMD_SYS_RIGID) return E[0];
+    if (kind == FMD_SYS_AIREBO) return E[q == 2 ? 0 : q + 1];
+    return q == 2 ? E[2] + E[3] : E[q < 2 ? q : (q == 3 ? 4 : 6)];
+}
+__device__ __forceinline__ void record_energy(SysScal* S, int kind, const StepParams& p, const double* E, int q) {
+    const int g = S->gstep;
+    if (g >= p.gavg_from && g <= p.gavg_to && q < (kind == FMD_SYS_RIGID ? 1 : (kind == FMD_SYS_AIREBO ? 3 : 5)))
+        S->avg.sE[q] += average_energy(kind, E, q) / p.nmol;
+    S->obs.E[q] = E[q];
 }
 
 }  // namespace
@@ -411,7 +483,7 @@ __device__ void record(SysScal* S, int kind, const StepParams& p) {
 __device__ void lj_prune_commit(const StepArrays& a, const double* hh) {
     if (!a.prune_hb || !(a.prune_delta > 0.0)) return;
     if (!a.prune_walk) {
-        a.prune_stats[0] += 1ull;
+        atomicAdd(&a.prune_stats[0], 1ull);
         return;
     }
     const bool pruned = a.clus.on ? lj_clus_mode(a.clus, a.prune_umax, hh, a.prune_hb, a.prune_delta, a.prune_rc) ==
@@ -422,37 +494,50 @@ __device__ void lj_prune_commit(const StepArrays& a, const double* hh) {
         a.prune_umax[0] = 0ull;
         a.prune_umax[1] = lj_rows_tag(a.clus.on ? kRowsClusters : kRowsAtoms, a.prune_delta);
         for (int q = 0; q < 9; q++) a.prune_hb[q] = hh[q];
-        a.prune_stats[1] += 1ull;
+        atomicAdd(&a.prune_stats[1], 1ull);
     }
-    a.prune_stats[0] += 1ull;
+    atomicAdd(&a.prune_stats[0], 1ull);
 }
 
-// Thread 0 of the step end: prune commit, energies, virial and kinetic
-// energy from the reduced sums, the thermostat/barostat second half and the
-// driver's observables, on the scalars S.
-__device__ void end_scalars(const StepArrays& a, const StepParams& p, const double (&t)[kRedFields], SysScal* S) {
-    lj_prune_commit(a, S->h);
-    forces_from_sums(S, a, t);
+// The scalar end of a step on the copy S, by the block's threads: thread 0 the
+// kinetic energy, the thermostat/barostat second half and the driver's
+// temperature and pressure; others the virial and the energies with their
+// averages meanwhile.
+__device__ void end_scalars(const StepArrays& a, const StepParams& p, const double* t, SysScal* S) {
+    const bool rigid = a.kind == FMD_SYS_RIGID;
+    const int g = S->gstep;
+    const bool phase = g <= p.coldstart || g <= p.coldstart + p.warmup;
+    const bool rec = p.schedule && !phase;
+    if (threadIdx.x != 0) {
+        forces_from_sums(S, a, t);
+        const int q = (int)threadIdx.x - 64;
+        if (rec && q >= 0 && q < 8) {
+            double E[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) E[k] = energy_of(a, t, k);
+            record_energy(S, a.kind, p, E, q);
+        }
+        return;
+    }
+    double W[9];
+#pragma unroll
+    for (int q = 0; q < 9; q += 4) W[q] = virial_of(a.kind, t, q);
     kinetic_from_sums(S, a, t);
     const double hdt = 0.5 * p.dt;
-    const bool rigid = a.kind == FMD_SYS_RIGID;
-    const double V2 = fabs(det9(S->h));
-    if (rigid) npt_half(S->npt, hdt, S->KE, S->kt, S->W9, V2, 0.1, 0.01);
-    else npt_half(S->npt, hdt, S->KE, S->KE, S->W9, V2, 0.05, 0.005);
+    const double V = fabs(det9(S->h));
+    if (rigid) npt_half(S->npt, hdt, S->KE, S->kt, W, V, 0.1, 0.01);
+    else npt_half(S->npt, hdt, S->KE, S->KE, W, V, 0.05, 0.005);
     if (!p.schedule) return;
     // Driver observables after step_npt (LJ:874-876, AI:896, MM:1215-1219).
-    const double V = fabs(det9(S->h));
     S->Tn = inst_T(S->KE, S->npt.Nf);
-    S->Pn = inst_P(S->W9, rigid ? S->kt : S->KE, V);
-    const int g = S->gstep;
-    const bool phase = (g <= p.coldstart || g <= p.coldstart + p.warmup);
+    S->Pn = inst_P(W, rigid ? S->kt : S->KE, V);
     S->do_rescale = 0;
     if (phase && S->Tn > 0.1) {                                      // LJ:879-894
         const double tgt = (g <= p.coldstart) ? p.T_cold : S->npt.Tt;
         S->scale = sqrt(fmax(tgt, 0.1) / S->Tn);
         S->do_rescale = 1;
     }
-    if (!phase) record(S, a.kind, p);
+    if (rec) record_state(S, p);
 }
 
 // The end of a step in one block: the block copies the step scalars into
@@ -467,13 +552,12 @@ __device__ void end_body(const StepArrays& a, const StepParams& p, int nblk_f1, 
     int* gS = reinterpret_cast<int*>(a.S);
     int* cS = reinterpret_cast<int*>(sS);
     for (int k = threadIdx.x; k < kWords; k += blockDim.x) cS[k] = __ldcg(gS + k);
-    __syncthreads();
-    double t[kRedFields];
+    // the prune bookkeeping reads only the cell: beside the reduction
+    if (threadIdx.x == blockDim.x - 32) lj_prune_commit(a, a.S->h);
+    const double* t;
     reduce_all(a, nblk_f1, nblk_ke, true, true, sm, t, nblk_f2);
-    if (threadIdx.x == 0) {
-        end_scalars(a, p, t, sS);
-        sS->kick2_done = 0u;
-    }
+    end_scalars(a, p, t, sS);
+    if (threadIdx.x == 0) sS->kick2_done = 0u;
     __syncthreads();
     for (int k = threadIdx.x; k < kWords; k += blockDim.x) gS[k] = cS[k];
 }
@@ -481,17 +565,24 @@ __device__ void end_body(const StepArrays& a, const StepParams& p, int nblk_f1, 
 __device__ void rescale_end_body(const StepArrays& a, const StepParams& p, int nblk_ke, double* sm) {
     SysScal* S = a.S;
     const bool doit = S->do_rescale != 0;
-    double t[kRedFields];
+    const double* t;
     if (doit) reduce_all(a, 0, nblk_ke, false, true, sm, t, 0);
-    if (threadIdx.x != 0) return;
-    if (doit) {
-        kinetic_from_sums(S, a, t);
-        S->Tn = inst_T(S->KE, S->npt.Nf);
-        S->npt.xi = 0;
-        if (S->gstep <= p.coldstart)
-            for (int k = 0; k < 9; k++) S->npt.Vg[k] = 0;
+    if (threadIdx.x == 0) {
+        if (doit) {
+            kinetic_from_sums(S, a, t);
+            S->Tn = inst_T(S->KE, S->npt.Nf);
+            S->npt.xi = 0;
+            if (S->gstep <= p.coldstart)
+                for (int k = 0; k < 9; k++) S->npt.Vg[k] = 0;
+        }
+        record_state(S, p);
     }
-    record(S, a.kind, p);
+    const int q = (int)threadIdx.x - 64;
+    if (q >= 0 && q < 8) {
+        double E[8];
+        for (int k = 0; k < 8; k++) E[k] = S->E[k];
+        record_energy(S, a.kind, p, E, q);
+    }
 }
 
 namespace {
@@ -502,7 +593,7 @@ namespace {
 // the result does not depend on which block is last) and resets the ticket.
 __global__ void __launch_bounds__(kPB) k_kick2_end(StepArrays a, StepParams p, int nblk_f1) {
     FMD_PDL_WAIT();
-    __shared__ double sm[32 * kRedFields];
+    __shared__ double sm[kRedShared];
     __shared__ SysScal sS;
     __shared__ bool last;
     kick2_body(a, p.dt, blockIdx.x, gridDim.x, sm);
@@ -520,7 +611,7 @@ __global__ void __launch_bounds__(kPB) k_kick2_end(StepArrays a, StepParams p, i
 // kinetic record.
 __global__ void __launch_bounds__(kPB) k_rigid_kick2_end(StepArrays a, StepParams p) {
     FMD_PDL_WAIT();
-    __shared__ double sm[32 * kRedFields];
+    __shared__ double sm[kRedShared];
     __shared__ SysScal sS;
     __shared__ bool last;
     const int lane = threadIdx.x & 31;
@@ -563,13 +654,13 @@ __global__ void __launch_bounds__(kPB) k_rigid_kick2_end(StepArrays a, StepParam
 
 __global__ void __launch_bounds__(kRedThreads) k_rescale_end(StepArrays a, StepParams p, int nblk_ke) {
     FMD_PDL_WAIT();
-    __shared__ double sm[32 * kRedFields];
+    __shared__ double sm[kRedShared];
     rescale_end_body(a, p, nblk_ke, sm);
 }
 
 __global__ void __launch_bounds__(kRedThreads) k_ke_final(StepArrays a, int nblk_ke) {
-    __shared__ double sm[32 * kRedFields];
-    double t[kRedFields];
+    __shared__ double sm[kRedShared];
+    const double* t;
     reduce_all(a, 0, nblk_ke, false, true, sm, t, 0);
     if (threadIdx.x == 0) kinetic_from_sums(a.S, a, t);
 }
@@ -599,7 +690,7 @@ __global__ void __launch_bounds__(kPB) k_b_rescale(BatchDev b) {
 }
 
 __global__ void __launch_bounds__(256) k_b_end(BatchDev b) {
-    __shared__ double sm[32 * kRedFields];
+    __shared__ double sm[kRedShared];
     __shared__ SysScal sS;
     const int r = blockIdx.x;
     end_body(b.A[r], b.P[r], b.off_f1[r + 1] - b.off_f1[r], b.off_atom[r + 1] - b.off_atom[r],
@@ -607,26 +698,24 @@ __global__ void __launch_bounds__(256) k_b_end(BatchDev b) {
 }
 
 __global__ void __launch_bounds__(256) k_b_rescale_end(BatchDev b) {
-    __shared__ double sm[32 * kRedFields];
+    __shared__ double sm[kRedShared];
     const int r = blockIdx.x;
     rescale_end_body(b.A[r], b.P[r], b.off_atom[r + 1] - b.off_atom[r], sm);
 }
 
 __global__ void __launch_bounds__(kRedThreads) k_force_final(StepArrays a, int nblk_f1) {
-    __shared__ double sm[32 * kRedFields];
-    double t[kRedFields];
+    __shared__ double sm[kRedShared];
+    const double* t;
     reduce_all(a, nblk_f1, 0, true, false, sm, t, a.lj_blocks);
-    if (threadIdx.x == 0) {
-        forces_from_sums(a.S, a, t);
-        lj_prune_commit(a, a.S->h);
-    }
+    forces_from_sums(a.S, a, t);
+    if (threadIdx.x == 0) lj_prune_commit(a, a.S->h);
 }
 
 }  // namespace
 
 int force_partial_blocks(const StepArrays& a) {
     if (a.kind == FMD_SYS_RIGID && a.rigid_pair.on) return rigid_pair_records(a.n);
-    return a.kind == FMD_SYS_RIGID ? rigid_grid(a.n) : (a.kind == FMD_SYS_AIREBO ? a.rebo_blocks : kForceBlocks);
+    return a.kind == FMD_SYS_RIGID ? rigid_grid(a.n) : (a.kind == FMD_SYS_AIREBO ? a.rebo_blocks : mm_bonded_blocks(a.topo));
 }
 
 // LJ term of an atomistic system: the gather over the full rows, or with
@@ -672,7 +761,7 @@ cudaError_t enqueue_forces(const StepArrays& a, cudaStream_t st, bool judge, boo
         else if (a.sg) e = sg_enqueue_rebo(*a.sg, a, judge, st);
         else if (a.rebo_slots)
             e = rebo_slots_launch(a.pos, hh, a.cnt_b, a.list_b, a.cap_b, a.n, a.rebo_slots, a.Facc, a.part_f1,
-                                  kForceBlocks, nullptr, 0, st, a.rebo_ids, a.rebo_phys != 0);
+                                  a.rebo_blocks, nullptr, 0, st, a.rebo_ids, a.rebo_phys != 0);
         else e = rebo_launch(a.pos, hh, a.cnt_b, a.list_b, a.cap_b, a.n, a.Facc, a.part_f1, st);
         if (e != cudaSuccess) return e;
         e = enqueue_lj(a, FMD_FF_AIREBO, st);

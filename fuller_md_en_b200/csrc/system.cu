@@ -394,7 +394,7 @@ LJShape System::pick_lj_shape(bool pruned, int& rc) {
         if (arr.kind == FMD_SYS_MM) return mm_bonded_launch(arr.topo, arr.pos, hh, arr.Facc, arr.part_f1, st);
         if (arr.rebo_slots)
             return rebo_slots_launch(arr.pos, hh, arr.cnt_b, arr.list_b, arr.cap_b, arr.n, arr.rebo_slots, arr.Facc,
-                                     arr.part_f1, kForceBlocks, nullptr, 0, st, arr.rebo_ids, arr.rebo_phys != 0);
+                                     arr.part_f1, arr.rebo_blocks, nullptr, 0, st, arr.rebo_ids, arr.rebo_phys != 0);
         return rebo_launch(arr.pos, hh, arr.cnt_b, arr.list_b, arr.cap_b, arr.n, arr.Facc, arr.part_f1, st);
     };
     const LJPruneOut walk = pruned ? lj_prune_out(prune) : LJPruneOut{};
@@ -419,7 +419,7 @@ LJShape System::pick_lj_shape(bool pruned, int& rc) {
         for (int u : {2, 4})
             for (int pipe : {0, 1, 2}) {
                 const LJShape sh{nt, u, pipe, contig};
-                if (lj_gather_blocks(ff, arr.precision, sh, arr.in_cap) < 1) continue;
+                if (lj_gather_blocks(ff, arr.precision, sh, arr.in_cap, arr.n) < 1) continue;
                 time_one(sh, walk, 0);           // untimed: first launch of this shape
                 float tot = 0.f;
                 for (int r = 0; r < 3; r++) tot += time_one(sh, walk, r);
@@ -447,8 +447,8 @@ void System::set_lj_blocks() {
         arr.lj_blocks = lj_clus_blocks(ff, arr.precision);
         return;
     }
-    arr.lj_blocks = std::max(lj_gather_blocks(ff, arr.precision, arr.lj_shape, arr.in_cap),
-                             lj_gather_blocks(ff, arr.precision, arr.lj_shape_p, arr.in_cap));
+    arr.lj_blocks = std::max(lj_gather_blocks(ff, arr.precision, arr.lj_shape, arr.in_cap, arr.n),
+                             lj_gather_blocks(ff, arr.precision, arr.lj_shape_p, arr.in_cap, arr.n));
 }
 
 // Launch shape of the atomistic LJ gather over the full rows: every candidate
@@ -473,7 +473,7 @@ int System::tune_lj() {
                 return false;
             sh.pipe = feed & 3;
             sh.contig = feed >> 2;
-            return lj_gather_blocks(ff, arr.precision, sh, arr.in_cap) > 0;
+            return lj_gather_blocks(ff, arr.precision, sh, arr.in_cap, arr.n) > 0;
         };
         LJShape sh, shp;
         const char* second = std::strchr(env, ';');
@@ -748,7 +748,8 @@ extern "C" int fmd_system_create_airebo(fmd_ctx* ctx, const fmd_run_params* p, i
     s->arr.kind = FMD_SYS_AIREBO;
     s->arr.n = na;
     s->arr.precision = p->precision;
-    s->arr.lj_blocks = lj_gather_blocks(FMD_FF_AIREBO, p->precision, s->arr.lj_shape, 0);
+    s->arr.lj_blocks = lj_gather_blocks(FMD_FF_AIREBO, p->precision, s->arr.lj_shape, 0, na);
+    s->arr.rebo_blocks = rebo_slot_blocks(na);
     int rc = s->alloc_common(pos, vel, h, npt);
     if (rc != FMD_OK) return rc;
     double* m; int* mid;
@@ -776,7 +777,7 @@ int create_mm(fmd_ctx* ctx, const fmd_run_params* p, int na, const double* pos, 
     s->arr.kind = FMD_SYS_MM;
     s->arr.n = na;
     s->arr.precision = p->precision;
-    s->arr.lj_blocks = lj_gather_blocks(FMD_FF_MM, p->precision, s->arr.lj_shape, 0);
+    s->arr.lj_blocks = lj_gather_blocks(FMD_FF_MM, p->precision, s->arr.lj_shape, 0, na);
     int rc = s->alloc_common(pos, vel, h, npt);
     if (rc != FMD_OK) return rc;
     int* mid;
@@ -1110,7 +1111,7 @@ extern "C" int fmd_system_kernel_ms(fmd_system* s, int stage, int reps, double* 
                     return sg_enqueue_rebo(*a.sg, a, false, st);
                 if (a.kind == FMD_SYS_AIREBO)
                     return rebo_slots_launch(a.pos, hh, a.cnt_b, a.list_b, a.cap_b, a.n, a.rebo_slots, a.Facc,
-                                             a.part_f1, kForceBlocks, nullptr, 0, st, a.rebo_ids, a.rebo_phys != 0);
+                                             a.part_f1, a.rebo_blocks, nullptr, 0, st, a.rebo_ids, a.rebo_phys != 0);
                 if (a.kind == FMD_SYS_MM) return mm_bonded_launch(a.topo, a.pos, hh, a.Facc, a.part_f1, st);
                 return enqueue_rigid(a, st);
             case 2:
@@ -1194,7 +1195,7 @@ extern "C" int fmd_system_set_lj_shape(fmd_system* s, int threads, int unroll, i
         return y.ctx->fail(FMD_ERR_ARG, "fmd_system_set_lj_shape: bad shape");
     const LJShape sh{threads, unroll, feed & 3, feed >> 2};
     const int ff = y.arr.kind == FMD_SYS_AIREBO ? FMD_FF_AIREBO : FMD_FF_MM;
-    const int nb = lj_gather_blocks(ff, y.arr.precision, sh, y.arr.in_cap);
+    const int nb = lj_gather_blocks(ff, y.arr.precision, sh, y.arr.in_cap, y.arr.n);
     if (nb < 1) return y.ctx->fail(FMD_ERR_ARG, "fmd_system_set_lj_shape: shape cannot run with this list");
     if (cudaStreamSynchronize(y.ctx->stream) != cudaSuccess) return y.ctx->fail(FMD_ERR_CUDA, "sync failed");
     y.drop_graphs();                     // captured graphs hold the old launch
@@ -1345,7 +1346,7 @@ int fmd::System::use_surrogate(fmd_sg* model, int judge_every, double rmse_max) 
     drop_graphs();                       // captured graphs hold the old REBO term
     if (!model) {
         arr.sg = nullptr;
-        arr.rebo_blocks = kForceBlocks;
+        arr.rebo_blocks = rebo_slot_blocks(arr.n);
     } else {
         if (arr.rebo2_flags & FMD_REBO2_BOND_ORDER)
             return ctx->fail(FMD_ERR_ARG, "fmd_system_use_surrogate: the system uses the REBO-II bond order");
