@@ -24,6 +24,7 @@
 #include <tuple>
 #include <vector>
 
+#include "mmmol.h"
 #include "molnlist.h"
 #include "step.h"
 #include "system.h"
@@ -43,8 +44,9 @@ struct Tune {
     double lj_ms = 0, f1_ms = 0;
 };
 
-std::map<std::tuple<int, int, long long>, Tune>& tune_cache() {
-    static std::map<std::tuple<int, int, long long>, Tune> m;
+using TuneKey = std::tuple<int, int, long long, bool>;
+std::map<TuneKey, Tune>& tune_cache() {
+    static std::map<TuneKey, Tune> m;
     return m;
 }
 
@@ -259,7 +261,7 @@ struct fmd_batch {
 
     int autotune() {
         const int dev = ctx->device;
-        const auto key = std::make_tuple(dev, R, natoms);
+        const auto key = std::make_tuple(dev, R, natoms, bd.mol_smem > 0);
         auto it = tune_cache().find(key);
         if (it != tune_cache().end()) {
             tune = it->second;
@@ -297,13 +299,15 @@ struct fmd_batch {
             best.f1_ms = 1e30;
             Tune b2 = best;
             for (int nt : {128, 256})
-                for (int tpb : {256, 512, 1024, 2048}) {
+                for (int tpb : {256, 512, 1024, 2048, 4096, 8192}) {
+                    if (bd.mol_smem ? nt != 256 : tpb > 2048) continue;
                     Tune t = b2;
                     t.f1_threads = nt; t.f1_tpb = tpb;
                     int rc = set_offsets(t);
                     if (rc) return rc;
                     const double ms = time_ms(3, [&]() {
-                        return batch_mm_bonded_launch(dA, bd.off_f1, R, bd.nblk_f1, nt, st);
+                        return bd.mol_smem ? batch_mm_mol_launch(dA, bd.off_f1, R, bd.nblk_f1, bd.mol_smem, st)
+                                           : batch_mm_bonded_launch(dA, bd.off_f1, R, bd.nblk_f1, nt, st);
                     });
                     if (ms < best.f1_ms) { best.f1_threads = nt; best.f1_tpb = tpb; best.f1_ms = ms; }
                 }
@@ -498,7 +502,13 @@ extern "C" int fmd_batch_create(fmd_ctx* ctx, int R, fmd_system* const* systems,
     std::vector<StepParams> P(R);
     // the batch's gather walks cluster rows where every replica's does, else full rows
     b->bd.lj_clus = 1;
-    for (System* s : b->sys) b->bd.lj_clus &= s->arr.clus.on;
+    bool molecules = true;
+    for (System* s : b->sys) {
+        b->bd.lj_clus &= s->arr.clus.on;
+        molecules = molecules && s->arr.topo.tpl.nmol > 0;
+    }
+    if (molecules)
+        for (System* s : b->sys) b->bd.mol_smem = std::max(b->bd.mol_smem, mm_mol_shared(s->arr.topo.tpl));
     for (int r = 0; r < R; r++) {
         A[r] = b->sys[r]->arr;
         A[r].prune_walk = b->bd.lj_clus;

@@ -271,7 +271,21 @@ cudaError_t rigid_pair_launch(const RigidPair& r, int precision, const double* p
 cudaError_t rigid_pair_reduce(const RigidPair& r, const int* cnt, const int* list, int cap, int n, double* F,
                               double* T, double* part, cudaStream_t st);
 
-// MM bonded terms (a10-a13): atomics into Facc; partials {E_b,E_a,E_d,E_i, W00,W11,W22}
+// The terms of one molecule of a system of nmol equal ones, copies in order
+// (mmmol.cu): torsions (dihedrals, then impropers) {a1..a4}, {V, cos gamma,
+// sin gamma, multiplicity}; angles {i, j, k}, {k, th0}; bonds {i, j}, {k, r0}.
+// A term's force on its r-th atom of n goes to slot kind base + r * terms +
+// term; inc[inc_off[a] ..) lists atom a's slots, filled up with slot `slots`
+// (no force) to whole groups of 16.  nmol 0: none.
+struct MMTpl {
+    int nmol = 0, natom = 0, ntor = 0, ndih = 0, nang = 0, nb = 0, slots = 0, ninc = 0;
+    const ushort4* id = nullptr;           // atoms of the torsions, then angles, then bonds
+    const double4* torp = nullptr;
+    const double2 *angp = nullptr, *bondp = nullptr;
+    const int* inc_off = nullptr;
+    const ushort4* inc = nullptr;
+};
+// MM bonded terms (a10-a13): by molecules with tpl, else atomics into Facc; partials {E_b,E_a,E_d,E_i, W00,W11,W22}
 struct MMTopoDev {
     int nb, nang, ndih, nimp;
     const int *b_i0, *b_i1; const double *b_kb, *b_r0;
@@ -279,6 +293,7 @@ struct MMTopoDev {
     const int *d_i0, *d_i1, *d_i2, *d_i3; const double *d_vn; const int *d_mult; const double *d_gamma;
     const int *m_i0, *m_i1, *m_i2, *m_i3; const double *m_ki, *m_gamma;
     int physical;                 // 1: bond and angle forces as -grad E (FMD_PHYS_MM_BONDED)
+    MMTpl tpl;
 };
 constexpr int kMMNV = 7;
 // Writable view of a system's topology arrays (the replication's output).

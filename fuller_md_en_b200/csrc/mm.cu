@@ -1,7 +1,9 @@
 // mm.cu -- molecular-mechanics bonded terms and cut Coulomb (MM:378-709,
 // MM:766-786).
 //
-// Bonded terms: one thread per term over the concatenated index space
+// Bonded terms of a system of equal molecules: mmmol.cu.  Any other topology
+// (terms in another order, molecules that differ, too many terms for a block's
+// shared memory) and the host-pointer calls: one thread per term over the concatenated index space
 // [bonds | angles | dihedrals | impropers]; forces scattered with FP64
 // atomics into an accumulator that the LJ gather kernel folds into F and
 // clears.  Sign conventions follow the reference exactly, including the bond
@@ -19,6 +21,7 @@
 #include <cmath>
 #include "kernels.h"
 #include "geom.cuh"
+#include "mmmol.h"
 #include "step.h"
 
 namespace fmd {
@@ -255,12 +258,14 @@ cudaError_t mm_replicate_launch(const MMTopoDev& mol, int nmol, int natom, const
 }
 
 int mm_bonded_blocks(const MMTopoDev& t) {
+    if (t.tpl.nmol) return mm_mol_blocks(t.tpl);
     const long long terms = (long long)t.nb + t.nang + t.ndih + t.nimp;
     return (int)std::max(1LL, std::min<long long>(kForceBlocks, (terms + 127) / 128));
 }
 
 cudaError_t mm_bonded_launch(const MMTopoDev& t, const double* pos, const double* hh, double* Facc,
                              double* part, cudaStream_t st) {
+    if (t.tpl.nmol) return mm_mol_launch(t.tpl, t.physical, pos, hh, Facc, part, st);
     k_mm_bonded<<<mm_bonded_blocks(t), 128, 0, st>>>(t, pos, hh, Facc, part);
     return cudaGetLastError();
 }

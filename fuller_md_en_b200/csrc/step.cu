@@ -26,6 +26,7 @@
 #include <cmath>
 #include "step.h"
 #include "ljprune.h"
+#include "mmmol.h"
 #include "ljprune.cuh"
 #include "ljclus.cuh"
 #include "geom.cuh"
@@ -816,7 +817,9 @@ cudaError_t enqueue_batch_step(const BatchDev& b, bool rescale_phase, cudaStream
     cudaError_t e;
     k_b_begin<<<b.R, 32, 0, st>>>(b);
     k_b_kick<<<b.nblk_atom, kPB, 0, st>>>(b);
-    if (b.kind == FMD_SYS_MM)
+    if (b.mol_smem) {
+        if ((e = batch_mm_mol_launch(b.A, b.off_f1, b.R, b.nblk_f1, b.mol_smem, st)) != cudaSuccess) return e;
+    } else if (b.kind == FMD_SYS_MM)
         if ((e = batch_mm_bonded_launch(b.A, b.off_f1, b.R, b.nblk_f1, b.f1_threads, st)) != cudaSuccess) return e;
     if (b.lj_clus) {
         if ((e = batch_lj_clus_launch(b.A, b.off_lj, b.R, b.nblk_lj, b.precision, st)) != cudaSuccess) return e;

@@ -140,6 +140,7 @@ struct BatchDev {
     int lj_threads = 256, lj_unroll = 4, f1_threads = 128;
     int lj_staged_in_cap = 0;        // > 0: LJ rows staged in shared memory
     int lj_clus = 0;                 // 1: cluster rows (every replica's clus.on)
+    size_t mol_smem = 0;             // > 0: bonded terms by molecules (every replica's topo.tpl)
     int kind = FMD_SYS_MM, ff = FMD_FF_MM, precision = FMD_PREC_FP64;
 };
 // LJ gather / MM bonded terms over all replicas in one launch each.

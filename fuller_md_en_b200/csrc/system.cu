@@ -14,6 +14,7 @@
 #include <tuple>
 #include "ljclus.h"
 #include "ljprune.cuh"
+#include "mmmol.h"
 #include "step.h"
 #include "system.h"
 #include "sg_host.h"
@@ -783,7 +784,7 @@ int create_mm(fmd_ctx* ctx, const fmd_run_params* p, int na, const double* pos, 
     int* mid;
     if (s->alloc(&mid, na, mol_id)) return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
     s->arr.mol_id = mid;
-    if ((rc = t ? s->upload_topology(t) : s->replicate_topology(t1, nmol, natom_mol)) != FMD_OK) return rc;
+    if ((rc = t ? s->upload_topology(t, mol_id) : s->replicate_topology(t1, nmol, natom_mol)) != FMD_OK) return rc;
     bool has_charge = false;
     if (charge)
         for (int i = 0; i < na && !has_charge; i++) has_charge = std::fabs(charge[i]) > 1e-10;   // MM:1110
@@ -863,10 +864,11 @@ int fmd::System::replicate_topology(const fmd_mm_topology* t, int nmol, int nato
     d.d_gamma = o.d_gamma;
     d.m_i0 = o.m_i0; d.m_i1 = o.m_i1; d.m_i2 = o.m_i2; d.m_i3 = o.m_i3; d.m_ki = o.m_ki; d.m_gamma = o.m_gamma;
     arr.topo = d;
-    return ctx->sync_check("topology replication");
+    const int rc = ctx->sync_check("topology replication");
+    return rc != FMD_OK ? rc : upload_template(t, 1, nmol, natom);
 }
 
-int fmd::System::upload_topology(const fmd_mm_topology* t) {
+int fmd::System::upload_topology(const fmd_mm_topology* t, const int* mol_id) {
     // Topology indices address device arrays: check them before any launch.
     auto ok = [&](const int* a, int m) {
         if (m > 0 && !a) return false;
@@ -879,7 +881,30 @@ int fmd::System::upload_topology(const fmd_mm_topology* t) {
         !ok(t->dih_i0, t->ndih) || !ok(t->dih_i1, t->ndih) || !ok(t->dih_i2, t->ndih) || !ok(t->dih_i3, t->ndih) ||
         !ok(t->imp_i0, t->nimp) || !ok(t->imp_i1, t->nimp) || !ok(t->imp_i2, t->nimp) || !ok(t->imp_i3, t->nimp))
         return ctx->fail(FMD_ERR_ARG, "MM topology: index out of range");
-    return upload_topology_arrays(t);
+    const int rc = upload_topology_arrays(t), natom = mm_copies(*t, arr.n, mol_id);
+    return rc != FMD_OK || natom == 0 ? rc : upload_template(t, arr.n / natom, arr.n / natom, natom);
+}
+
+// The plan of the bonded terms by molecules, where one can be had, for nmol
+// molecules of natom atoms; t holds copies of one molecule's terms.
+int fmd::System::upload_template(const fmd_mm_topology* t, int copies, int nmol, int natom) {
+    MMTplHost o;
+    if (!mm_tpl_build(*t, copies, natom, o)) return FMD_OK;
+    MMTpl d = o.dims;
+    d.nmol = nmol;
+    ushort4* id;
+    double4* torp;
+    double2 *angp, *bondp;
+    int* off;
+    ushort4* inc;
+    if (alloc(&id, o.id.size(), o.id.data()) || alloc(&torp, o.torp.size(), o.torp.data()) ||
+        alloc(&angp, o.angp.size(), o.angp.data()) || alloc(&bondp, o.bondp.size(), o.bondp.data()) ||
+        alloc(&off, o.inc_off.size(), o.inc_off.data()) || alloc(&inc, o.inc.size(), o.inc.data()))
+        return ctx->fail(FMD_ERR_CUDA, "topology upload failed");
+    d.id = id; d.torp = torp; d.angp = angp; d.bondp = bondp;
+    d.inc_off = off; d.inc = inc;
+    arr.topo.tpl = d;
+    return ctx->sync_check("molecule template");   // the host's copy goes
 }
 
 // Copies the topology arrays of t to the device as the system's topology

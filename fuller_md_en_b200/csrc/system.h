@@ -46,7 +46,8 @@ struct System {
     cudaError_t ensure_full_rows(cudaStream_t st);
     void set_clus(bool allowed);
     int retune_lj();
-    int upload_topology(const fmd_mm_topology* t);
+    int upload_topology(const fmd_mm_topology* t, const int* mol_id);
+    int upload_template(const fmd_mm_topology* t, int copies, int nmol, int natom);
     int upload_topology_arrays(const fmd_mm_topology* t);
     // One molecule's topology t (indices within the molecule) replicated on
     // the device over nmol contiguous molecules of natom atoms.
