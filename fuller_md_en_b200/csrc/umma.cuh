@@ -94,6 +94,26 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     for (int q = 0; q < 16; q++) v[q] = __uint_as_float(r[q]);
 }
 
+// Two such loads with one wait.
+__device__ __forceinline__ void tmem_ld16x2(uint32_t ta, uint32_t tb, float* a, float* b) {
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]),
+          "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]),
+          "=&r"(r[15]), "=&r"(r[16]), "=&r"(r[17]), "=&r"(r[18]), "=&r"(r[19]), "=&r"(r[20]), "=&r"(r[21]),
+          "=&r"(r[22]), "=&r"(r[23]), "=&r"(r[24]), "=&r"(r[25]), "=&r"(r[26]), "=&r"(r[27]), "=&r"(r[28]),
+          "=&r"(r[29]), "=&r"(r[30]), "=&r"(r[31])
+        : "r"(ta), "r"(tb)
+        : "memory");
+#pragma unroll
+    for (int q = 0; q < 16; q++) { a[q] = __uint_as_float(r[q]); b[q] = __uint_as_float(r[16 + q]); }
+}
+
 // The store of the same shape: thread t of the warp writes lane (lane base +
 // t), 16 consecutive columns.  tmem_wait_st() waits for this thread's stores.
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
@@ -123,6 +143,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* m, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// The one arrival of this phase, which then also waits for `bytes` of copies.
+__device__ __forceinline__ void mbar_expect(uint64_t* m, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(m)), "r"(bytes) : "memory");
+}
+// Copy of `bytes` (a multiple of 16, both ends 16-byte aligned) from global to
+// shared memory, counted by *m.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* m) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(smem_u32(m))
+                 : "memory");
+}
 __device__ __forceinline__ uint64_t globaltimer_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -139,10 +170,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* m, uint32_t parity) {
     return false;
 }
 
+// Two values as BF16 (nearest), a in the low half: one conversion.
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-    const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16_rn(a));
-    const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16_rn(b));
-    return lo | (hi << 16);
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
 }
 
 }  // namespace umma
