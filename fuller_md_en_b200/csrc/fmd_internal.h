@@ -2,6 +2,7 @@
 // launch helpers, error plumbing).  Not part of the public C-ABI.
 #pragma once
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 #include <map>
@@ -70,20 +71,41 @@ struct fmd_ctx {
     // Device blocks released by systems of this context, by size: the next
     // system of the same size takes them instead of mapping fresh memory
     // (cudaMalloc of a few hundred MB costs milliseconds and varies with the
-    // process's allocation history).  Freed with the context.
+    // process's allocation history).  At most kCacheMax bytes; given back when
+    // an allocation fails, and with the context.
+    static constexpr size_t kCacheMax = (size_t)16 << 30;
     std::multimap<size_t, void*> mem_cache;
+    size_t cached = 0;
+    void drop_cache() {
+        for (auto& b : mem_cache) cudaFree(b.second);
+        mem_cache.clear();
+        cached = 0;
+    }
     cudaError_t dev_alloc(void** p, size_t bytes) {
         auto it = mem_cache.find(bytes);
         if (it != mem_cache.end()) {
             *p = it->second;
             mem_cache.erase(it);
+            cached -= bytes;
             return cudaSuccess;
         }
-        return cudaMalloc(p, bytes);
+        cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation && !mem_cache.empty()) {
+            cudaGetLastError();
+            drop_cache();
+            e = cudaMalloc(p, bytes);
+        }
+        return e;
     }
     // The caller has synchronised every stream that used the block.
     void dev_release(void* p, size_t bytes) {
-        if (p) mem_cache.emplace(bytes, p);
+        if (!p) return;
+        if (bytes > kCacheMax - std::min(cached, kCacheMax)) {
+            cudaFree(p);
+            return;
+        }
+        mem_cache.emplace(bytes, p);
+        cached += bytes;
     }
 
     int fail(int code, const std::string& m) {

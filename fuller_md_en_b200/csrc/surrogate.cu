@@ -537,14 +537,15 @@ __global__ void k_sg_pack(const double* __restrict__ P, uint16_t* __restrict__ i
 
 }  // namespace
 
-cudaError_t work_alloc(Work& w, int na, int cap) {
+cudaError_t work_alloc(Work& w, int na, int cap, cudaStream_t st, const DevAlloc& alloc) {
     if (na <= w.na_cap && cap == w.cap) return cudaSuccess;
     work_free(w);
     const int rcap = ((na * cap + TILE - 1) / TILE) * TILE;
     cudaError_t e = cudaSuccess;
     auto A = [&](void** p, size_t bytes) {
-        if (e == cudaSuccess) e = cudaMalloc(p, bytes);
+        if (e == cudaSuccess) e = alloc(p, bytes);
     };
+    w.lent = alloc.fn != nullptr;
     A((void**)&w.acnt, sizeof(int) * (size_t)na);
     A((void**)&w.aoff, sizeof(int) * ((size_t)na + 1));
     A((void**)&w.row_i, sizeof(int) * (size_t)rcap);
@@ -558,7 +559,7 @@ cudaError_t work_alloc(Work& w, int na, int cap) {
     A((void**)&w.err, sizeof(int) * 4);
     A((void**)&w.bsum, sizeof(int) * ((size_t)na / 256 + 2));
     A((void**)&w.boff, sizeof(int) * ((size_t)na / 256 + 3));
-    if (e == cudaSuccess) e = cudaMemset(w.err, 0, sizeof(int) * 4);
+    if (e == cudaSuccess) e = cudaMemsetAsync(w.err, 0, sizeof(int) * 4, st);
     if (e != cudaSuccess) {
         work_free(w);
         return e;
@@ -570,6 +571,10 @@ cudaError_t work_alloc(Work& w, int na, int cap) {
 }
 
 void work_free(Work& w) {
+    if (w.lent) {
+        w = Work{};
+        return;
+    }
     cudaFree(w.acnt); cudaFree(w.aoff); cudaFree(w.row_i); cudaFree(w.row_s); cudaFree(w.rowid);
     cudaFree(w.partner); cudaFree(w.X); cudaFree(w.b); cudaFree(w.gx); cudaFree(w.part); cudaFree(w.err);
     cudaFree(w.bsum); cudaFree(w.boff);

@@ -13,6 +13,7 @@
 #include <cstdint>
 
 #include "fmd_internal.h"
+#include "kernels.h"
 
 namespace fmd {
 namespace sg {
@@ -51,9 +52,12 @@ struct Work {
     int* err = nullptr;       // [4] kernel status words
     int* bsum = nullptr;      // [na / 256 + 1] rows per block of 256 atoms
     int* boff = nullptr;      // [na / 256 + 2] their exclusive scan
+    bool lent = false;        // the arrays belong to the allocator they came from
 };
 
-cudaError_t work_alloc(Work& w, int na, int cap);
+// Arrays for na atoms, from cudaMalloc or from alloc, which keeps them; st
+// orders the zeroing of the status words.
+cudaError_t work_alloc(Work& w, int na, int cap, cudaStream_t st = nullptr, const DevAlloc& alloc = DevAlloc());
 void work_free(Work& w);
 
 // Packs the FP64 master parameters into the BF16 images and FP32 vectors.

@@ -1377,7 +1377,7 @@ int fmd::System::use_surrogate(fmd_sg* model, int judge_every, double rmse_max) 
             return ctx->fail(FMD_ERR_ARG, "fmd_system_use_surrogate: the system uses the REBO-II bond order");
         if (!sg) {
             auto g = std::make_unique<SgStep>();
-            if (sg::work_alloc(g->work, arr.n, arr.cap_b) != cudaSuccess)
+            if (sg::work_alloc(g->work, arr.n, arr.cap_b, st, owned_alloc()) != cudaSuccess)
                 return ctx->fail(FMD_ERR_CUDA, "fmd_system_use_surrogate: workspace allocation failed");
             if (alloc(&g->Fj, 3 * (size_t)arr.n, (const double*)nullptr) ||
                 alloc(&g->part_j, (size_t)sg::kRowBlocks * kNV, (const double*)nullptr)) {
