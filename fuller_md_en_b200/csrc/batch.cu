@@ -122,6 +122,7 @@ struct fmd_batch {
             return ctx->fail(FMD_ERR_CUDA, "batch: upload failed");
         mb.reps = dReps;
         mb.R = R;
+        mb.atoms = ntot;
         mb.off_w = dMolOff;
         mb.off_rows = dMolOff + (R + 1);
         mb.off_in = dMolOff + 2 * (R + 1);

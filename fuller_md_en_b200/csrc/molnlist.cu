@@ -22,6 +22,7 @@
 // partners than the table holds (a disintegrating crystal), the system falls
 // back to the cell-grid builder (nlist.cu) for that rebuild: a device flag
 // gates the two paths inside one CUDA graph.
+#include <algorithm>
 #include <cmath>
 
 #include "geom.cuh"
@@ -66,8 +67,8 @@ __device__ __forceinline__ bool pair_in(const double* __restrict__ pos, int i, i
 
 // Centre (mean of the minimum images relative to the first atom) and radius
 // (largest minimum-image distance of an atom from the centre) per molecule,
-// and the FP32 copy of the positions; one warp per molecule.  Resets the
-// partner-overflow flag.
+// and the FP32 copy of the positions, each atom's image nearest the centre;
+// one warp per molecule.  Resets the partner-overflow flag.
 __device__ __forceinline__ void mol_centre_body(const double* __restrict__ pos, const double* __restrict__ hh,
                                                 const int* __restrict__ off, int M, double* __restrict__ cen,
                                                 double* __restrict__ rad, float4* __restrict__ pos32,
@@ -82,9 +83,6 @@ __device__ __forceinline__ void mol_centre_body(const double* __restrict__ pos, 
     double sx = 0.0, sy = 0.0, sz = 0.0;
     for (int a = a0 + lane; a < a1; a += 32) {
         double dx = pos[3 * a] - pos[3 * a0], dy = pos[3 * a + 1] - pos[3 * a0 + 1], dz = pos[3 * a + 2] - pos[3 * a0 + 2];
-        const double x = pos[3 * a], y = pos[3 * a + 1], z = pos[3 * a + 2];
-        const bool small = fabs(x) < kScreenMax && fabs(y) < kScreenMax && fabs(z) < kScreenMax;
-        pos32[a] = make_float4((float)x, (float)y, (float)z, small ? 1.0f : 0.0f);
         mimg(dx, dy, dz, hi, h);
         sx += dx; sy += dy; sz += dz;
     }
@@ -96,6 +94,9 @@ __device__ __forceinline__ void mol_centre_body(const double* __restrict__ pos, 
         double dx = pos[3 * a] - cx, dy = pos[3 * a + 1] - cy, dz = pos[3 * a + 2] - cz;
         mimg(dx, dy, dz, hi, h);
         r2 = fmax(r2, dx * dx + dy * dy + dz * dz);
+        const double x = cx + dx, y = cy + dy, z = cz + dz;
+        const bool small = fabs(x) < kScreenMax && fabs(y) < kScreenMax && fabs(z) < kScreenMax;
+        pos32[a] = make_float4((float)x, (float)y, (float)z, small ? 1.0f : 0.0f);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) r2 = fmax(r2, __shfl_xor_sync(kFull, r2, o));
@@ -262,23 +263,16 @@ k_mol_rows(const double* __restrict__ pos, const double* __restrict__ hh, int n,
 // and truncation as k_mol_rows<0>.  k div S is (k + 0.5) * fl(1/S) truncated:
 // the quotient's fractional part stays 0.5/S from an integer, and the FP32
 // product's relative error (<= 2^-23) cannot cross that for k < 4e6.
-// PAIRED (32 <= S <= 64): the walk goes by partner instead, two 32-lane
-// slices per partner (atoms 0-31, 32-63; lanes past S idle), kFlatU / 2
-// partners at a time -- no quotient per candidate -- and the ballot of the
-// kept entries of slice h of the p-th higher partner is stored as word 2 p + h
-// of the atom's candidate bitmap, bm[(A * 2 pmax + 2 p + h) * S + i - off[A]],
-// from which k_mol_incoming forms the full rows.
 constexpr int kFlatU = 4;
 constexpr int kFlatWarps = 8;
 
-template <bool PAIRED>
 __device__ __forceinline__ void mol_half_flat_body(const double* __restrict__ pos, const double* __restrict__ hh,
                                                    int n, const int* __restrict__ off, const int* __restrict__ amol,
                                                    const int* __restrict__ npart, const int* __restrict__ part,
                                                    int pmax, int S, const float4* __restrict__ pos32, double rc2,
                                                    int cap, int* __restrict__ cnt, int* __restrict__ list,
-                                                   int* __restrict__ dropped, const int* __restrict__ flag,
-                                                   unsigned* __restrict__ bm, int blk, int nblk) {
+                                                   int* __restrict__ dropped, const int* __restrict__ flag, int blk,
+                                                   int nblk) {
     if (flag[0] == 0) return;
     __shared__ double s_hh[18];
     __shared__ int s_start[kFlatWarps][kMolPartners];
@@ -311,23 +305,16 @@ __device__ __forceinline__ void mol_half_flat_body(const double* __restrict__ po
         const bool screen = sc.on && pi.w != 0.0f;
         int* row = list + (size_t)i * cap;
         int emitted = 0;
-        unsigned* bmA = PAIRED ? bm + (size_t)A * 2 * pmax * S + (i - off[A]) : nullptr;
-        const int nit = PAIRED ? nup : ncand;
-        for (int k0 = 0; k0 < nit; k0 += PAIRED ? kFlatU / 2 : 32 * kFlatU) {
+        for (int k0 = 0; k0 < ncand; k0 += 32 * kFlatU) {
             int jj[kFlatU];
             float4 q[kFlatU];
 #pragma unroll
             for (int u = 0; u < kFlatU; u++) {
                 jj[u] = -1;
-                if (PAIRED) {
-                    const int p = k0 + (u >> 1), a = ((u & 1) << 5) + lane;
-                    if (p < nup && a < S) jj[u] = st[p] + a;
-                } else {
-                    const int k = k0 + 32 * u + lane;
-                    if (k < ncand) {
-                        const int pk = (int)(((float)k + 0.5f) * invS);
-                        jj[u] = st[pk] + (k - pk * S);
-                    }
+                const int k = k0 + 32 * u + lane;
+                if (k < ncand) {
+                    const int pk = (int)(((float)k + 0.5f) * invS);
+                    jj[u] = st[pk] + (k - pk * S);
                 }
             }
 #pragma unroll
@@ -353,12 +340,6 @@ __device__ __forceinline__ void mol_half_flat_body(const double* __restrict__ po
                 const unsigned m = __ballot_sync(kFull, ok);
                 const int kk = emitted + __popc(m & below);
                 if (ok && kk < cap) row[kk] = jj[u];
-                if (PAIRED) {
-                    // the slice's entries that fit in the row (row position < cap)
-                    const unsigned kept = __ballot_sync(kFull, ok && kk < cap);
-                    const int p = k0 + (u >> 1);
-                    if (lane == 0 && p < nup) bmA[(size_t)(2 * p + (u & 1)) * S] = kept;
-                }
                 emitted += __popc(m);
             }
         }
@@ -370,15 +351,204 @@ __device__ __forceinline__ void mol_half_flat_body(const double* __restrict__ po
     }
 }
 
-template <bool PAIRED>
 __global__ void __launch_bounds__(32 * kFlatWarps, 3)
 k_mol_half_flat(const double* __restrict__ pos, const double* __restrict__ hh, int n, const int* __restrict__ off,
                 const int* __restrict__ amol, const int* __restrict__ npart, const int* __restrict__ part, int pmax,
                 int S, const float4* __restrict__ pos32, double rc2, int cap, int* __restrict__ cnt,
-                int* __restrict__ list, int* __restrict__ dropped, const int* __restrict__ flag,
+                int* __restrict__ list, int* __restrict__ dropped, const int* __restrict__ flag) {
+    mol_half_flat_body(pos, hh, n, off, amol, npart, part, pmax, S, pos32, rc2, cap, cnt, list, dropped, flag,
+                       blockIdx.x, gridDim.x);
+}
+
+// The half rows and candidate bitmaps of molecules of S atoms, 32 <= S <= 64.
+// A warp takes G consecutive atoms of a molecule.  Its lanes first test
+// the centres of 32 partners against the atoms: a partner further than rc + R
+// from an atom (about half of them: partners are within rc + R + R of the
+// molecule) holds none of its candidates.  Then the warp goes by partner, two
+// 32-lane slices each (atoms 0-31, 32-63; lanes past S idle): a slice's
+// positions are loaded and shifted to the image once and tested for every
+// atom that the partner is near.  The ballot of an atom's kept entries of
+// slice h of the p-th higher partner is word 2 p + h of the atom's candidate
+// bitmap, bm[(A * 2 pmax + 2 p + h) * S + i - off[A]], from which
+// k_mol_incoming forms the full rows and the cluster gather its own.
+// Same tests, order and truncation as k_mol_rows<0>.  It is bound by issue.
+// An atom a warp, every partner and an image per pair -> this one (B200, C60
+// crystals): 30,000 atoms 168 -> 84 us, 122,880 664 -> 314 us, 32 replicas of
+// 430,000 in all 2,644 -> 1,002 us.  G is kQuad when that gives every resident
+// warp a group, else 1 (mol_atoms_per_warp).
+//
+// One image serves a partner when every edge exceeds 2 (rc + R_A + R_B + 1):
+// pos32 holds each atom's image nearest its molecule's centre, and only the
+// image that the centres are nearest in can then bring two atoms within rc.
+constexpr int kQuad = 4;
+constexpr int kQuadWarps = 8;
+
+// pair_in out of line: it runs for few slices, and eight copies of it would
+// spread the walk's code.
+__device__ __noinline__ bool pair_in_far(const double* __restrict__ pos, int i, int j, const double* hh, double rc2) {
+    return pair_in(pos, i, j, hh, hh + 9, diag_cell(hh, hh + 9), rc2);
+}
+
+struct QuadShared {
+    double hh[18];
+    float4 part[kQuadWarps][kMolPartners];     // partner: image offset, first atom
+    int what[kQuadWarps][kMolPartners];        // p | atoms near << 16
+};
+
+template <int G>
+__device__ __forceinline__ void mol_half_quad_body(const double* __restrict__ pos, const double* __restrict__ hh,
+                                                   int M, const int* __restrict__ off, const int* __restrict__ npart,
+                                                   const int* __restrict__ part, const double* __restrict__ cen,
+                                                   const double* __restrict__ rad, int pmax, int S,
+                                                   const float4* __restrict__ pos32, double rc2, int cap,
+                                                   int* __restrict__ cnt, int* __restrict__ list,
+                                                   int* __restrict__ dropped, const int* __restrict__ flag,
+                                                   unsigned* __restrict__ bm, int blk, int nblk, QuadShared& sh) {
+    if (flag[0] == 0) return;
+    if (threadIdx.x < 18) sh.hh[threadIdx.x] = hh[threadIdx.x];
+    __syncthreads();
+    const double* h = sh.hh;
+    const double* hi = sh.hh + 9;
+    const bool diag = diag_cell(h, hi);
+    const Screen sc = make_screen(h, hi, diag, rc2);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    const int gpm = (S + G - 1) / G;
+    const float rcf = (float)sqrt(rc2);
+    const float half = 0.5f * fminf(fabsf(sc.L[0]), fminf(fabsf(sc.L[1]), fabsf(sc.L[2])));
+    for (int k = blk * kQuadWarps + w; k < M * gpm; k += nblk * kQuadWarps) {
+        const int A = k / gpm, a0 = (k - A * gpm) * G, ng = min(G, S - a0), i0 = off[A] + a0;
+        float px[G], py[G], pz[G];
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            const float4 q = pos32[i0 + min(g, ng - 1)];
+            px[g] = sc.on && q.w != 0.0f ? q.x : __int_as_float(0x7fffffff);     // NaN: every test is exact
+            py[g] = q.y; pz[g] = q.z;
+        }
+        const int np = npart[A];
+        const int* pa = part + (size_t)A * pmax;
+        unsigned* bmA = bm + (size_t)A * 2 * pmax * S + a0;
+        const float cx = (float)cen[3 * A], cy = (float)cen[3 * A + 1], cz = (float)cen[3 * A + 2], ra = (float)rad[A];
+        int nup = 0, ns = 0;
+        bool wide = true;                      // one image serves each partner
+        for (int q0 = 0; q0 < np; q0 += 32) {
+            const int q = q0 + lane;
+            const int B = q < np ? pa[q] : -1;
+            const bool up = B > A;
+            int near = 0;
+            float4 at = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (up) {
+                const double bx = cen[3 * B], by = cen[3 * B + 1], bz = cen[3 * B + 2];
+                const bool small = fabs(bx) < kScreenMax && fabs(by) < kScreenMax && fabs(bz) < kScreenMax;
+                const float x = (float)bx, y = (float)by, z = (float)bz, rb = (float)rad[B];
+                wide = wide && half > (rcf + ra + rb) * 1.0001f + 1.0f;
+                // FP32 coordinates below kScreenMax: distances to better than 0.001 A
+                const float lim = (rcf + rb) * 1.0001f + 0.01f, lim2 = lim * lim;
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    float dx = x - px[g], dy = y - py[g], dz = z - pz[g];
+                    dx = fmaf(-sc.L[0], rintf(dx * sc.Li[0]), dx);
+                    dy = fmaf(-sc.L[1], rintf(dy * sc.Li[1]), dy);
+                    dz = fmaf(-sc.L[2], rintf(dz * sc.Li[2]), dz);
+                    const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                    near |= g < ng && !(small && d2 > lim2) ? 1 << g : 0;
+                }
+                at.x = sc.L[0] * rintf((x - cx) * sc.Li[0]);
+                at.y = sc.L[1] * rintf((y - cy) * sc.Li[1]);
+                at.z = sc.L[2] * rintf((z - cz) * sc.Li[2]);
+                at.w = __int_as_float(off[B]);
+            }
+            const unsigned mu = __ballot_sync(kFull, up), mn = __ballot_sync(kFull, near != 0);
+            const int p = nup + __popc(mu & below);
+            if (near != 0) {
+                const int t = ns + __popc(mn & below);
+                sh.part[w][t] = at;
+                sh.what[w][t] = p | near << 16;
+            } else if (up) {
+                for (int g = 0; g < ng; g++) bmA[(size_t)(2 * p) * S + g] = bmA[(size_t)(2 * p + 1) * S + g] = 0u;
+            }
+            nup += __popc(mu);
+            ns += __popc(mn);
+        }
+        wide = __all_sync(kFull, wide);
+        __syncwarp();
+        int emitted[G];
+#pragma unroll
+        for (int g = 0; g < G; g++) emitted[g] = 0;
+        const bool low = lane < S, high = lane + 32 < S;
+        int* row = list + (size_t)i0 * cap;
+        float4 q[2], qn[2];
+        auto load = [&](int t) {
+            const int j0 = t < ns ? __float_as_int(sh.part[w][t].w) : i0;
+            qn[0] = pos32[j0 + (low ? lane : 0)];
+            qn[1] = pos32[j0 + (high ? lane + 32 : 0)];
+        };
+        load(0);
+        for (int t = 0; t < ns; t++) {
+            q[0] = qn[0]; q[1] = qn[1];
+            load(t + 1);
+            const float4 at = sh.part[w][t];
+            const int what = sh.what[w][t], j0 = __float_as_int(at.w), p = what & 0xffff;
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const bool valid = u ? high : low;
+                const int j = j0 + 32 * u + lane;
+                if (q[u].w == 0.0f) q[u].x = __int_as_float(0x7fffffff);         // NaN: exact
+                if (wide) { q[u].x -= at.x; q[u].y -= at.y; q[u].z -= at.z; }
+                unsigned word = 0u;
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    if (!(what >> (16 + g) & 1)) continue;                       // the same for the warp
+                    float dx = q[u].x - px[g], dy = q[u].y - py[g], dz = q[u].z - pz[g];
+                    if (!wide) {
+                        dx = fmaf(-sc.L[0], rintf(dx * sc.Li[0]), dx);
+                        dy = fmaf(-sc.L[1], rintf(dy * sc.Li[1]), dy);
+                        dz = fmaf(-sc.L[2], rintf(dz * sc.Li[2]), dz);
+                    }
+                    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                    bool ok = valid && r2 < sc.lo2;
+                    // the exact test only where some lane is in the band or without an FP32 copy
+                    const bool exact = valid && !(r2 < sc.lo2) && !(r2 > sc.hi2);
+                    if (__any_sync(kFull, exact)) {
+                        const bool in = pair_in_far(pos, i0 + g, exact ? j : i0 + g, sh.hh, rc2);
+                        ok = ok || (exact && in);
+                    }
+                    const unsigned m = __ballot_sync(kFull, ok);
+                    const int kk = emitted[g] + __popc(m & below);
+                    const bool fits = ok && kk < cap;
+                    if (fits) row[(size_t)g * cap + kk] = j;
+                    emitted[g] += __popc(m);
+                    // the slice's entries that fit in the row
+                    const unsigned kept = emitted[g] <= cap ? m : __ballot_sync(kFull, fits);
+                    if (lane == g) word = kept;
+                }
+                if (lane < ng) bmA[(size_t)(2 * p + u) * S + lane] = word;
+            }
+        }
+        __syncwarp();                              // the tables are refilled for the next atoms
+#pragma unroll
+        for (int g = 0; g < G; g++)
+            if (lane == g && g < ng) {
+                cnt[i0 + g] = emitted[g] < cap ? emitted[g] : cap;
+                if (emitted[g] > cap && dropped) atomicAdd(dropped, emitted[g] - cap);
+            }
+    }
+}
+
+// Atoms per warp for a build of n atoms.  1 / 4: 1,920 atoms 17 / 44 us, 6,480 27 /
+// 46, 15,360 55 / 54, 30,000 98 / 85, 51,840 162 / 144 us.
+int mol_atoms_per_warp(long long n) { return n >= kQuad * kSMs * 3 * kQuadWarps ? kQuad : 1; }
+
+template <int G>
+__global__ void __launch_bounds__(32 * kQuadWarps, G == 1 ? 4 : 3)
+k_mol_half_quad(const double* __restrict__ pos, const double* __restrict__ hh, int M, const int* __restrict__ off,
+                const int* __restrict__ npart, const int* __restrict__ part, const double* __restrict__ cen,
+                const double* __restrict__ rad, int pmax, int S, const float4* __restrict__ pos32, double rc2, int cap,
+                int* __restrict__ cnt, int* __restrict__ list, int* __restrict__ dropped, const int* __restrict__ flag,
                 unsigned* __restrict__ bm) {
-    mol_half_flat_body<PAIRED>(pos, hh, n, off, amol, npart, part, pmax, S, pos32, rc2, cap, cnt, list, dropped, flag,
-                               bm, blockIdx.x, gridDim.x);
+    __shared__ QuadShared sh;
+    mol_half_quad_body<G>(pos, hh, M, off, npart, part, cen, rad, pmax, S, pos32, rc2, cap, cnt, list, dropped, flag, bm,
+                       blockIdx.x, gridDim.x, sh);
 }
 
 // First index of a partner >= key in an ascending partner list.
@@ -422,7 +592,7 @@ __global__ void k_mol_rev(int M, const int* __restrict__ npart, const int* __res
 }
 
 // Full LJ rows from the candidate bitmaps of the partner-aligned walk
-// (k_mol_half_flat<true>), for equal molecules of S atoms (32 <= S <= 64,
+// (k_mol_half_quad), for equal molecules of S atoms (32 <= S <= 64,
 // off[A] = A S): atom j = B S + jb is in the kept row of i = A S + ia (A < B)
 // iff bit jb mod 32 of word 2 rev[B][q] + jb div 32 of i's bitmap is set.
 // Two blocks per molecule B, one per half of its atoms (jb < 32, jb >= 32):
@@ -610,13 +780,15 @@ __global__ void k_b_mol_cond(const MolRep* __restrict__ reps, int R, cudaGraphCo
     if (__syncthreads_or(need) && threadIdx.x == 0) cudaGraphSetConditional(cond, 1u);
 }
 
-__global__ void __launch_bounds__(32 * kFlatWarps, 3)
-k_b_mol_half_flat(const MolRep* __restrict__ reps, const int* __restrict__ off, int R) {
+template <int G>
+__global__ void __launch_bounds__(32 * kQuadWarps, G == 1 ? 4 : 2)
+k_b_mol_half_quad(const MolRep* __restrict__ reps, const int* __restrict__ off, int R) {
+    __shared__ QuadShared sh;
     const int r = rep_of(off, R, blockIdx.x);
     const MolRep& q = reps[r];
-    mol_half_flat_body<true>(q.pos, q.hh, q.m.n, q.m.off, q.m.amol, q.m.npart, q.m.part, q.m.pmax, q.m.usize,
-                             q.m.pos32, q.rc2, q.cap, q.cnt, q.list, q.dropped, q.m.flag, q.m.bm,
-                             blockIdx.x - off[r], off[r + 1] - off[r]);
+    mol_half_quad_body<G>(q.pos, q.hh, q.m.M, q.m.off, q.m.npart, q.m.part, q.m.cen, q.m.rad, q.m.pmax, q.m.usize,
+                          q.m.pos32, q.rc2, q.cap, q.cnt, q.list, q.dropped, q.m.flag, q.m.bm, blockIdx.x - off[r],
+                          off[r + 1] - off[r], sh);
 }
 
 __global__ void __launch_bounds__(32 * kInWarps)
@@ -653,7 +825,8 @@ cudaError_t mol_rebuild_batch_pre(const MolBatch& b, cudaGraphConditionalHandle 
 
 cudaError_t mol_rebuild_batch_rows(const MolBatch& b, cudaStream_t st) {
     if (b.R < 1) return cudaSuccess;
-    k_b_mol_half_flat<<<b.nblk_rows, 32 * kFlatWarps, 0, st>>>(b.reps, b.off_rows, b.R);
+    auto k = mol_atoms_per_warp(b.atoms) == 1 ? k_b_mol_half_quad<1> : k_b_mol_half_quad<kQuad>;
+    k<<<b.nblk_rows, 32 * kQuadWarps, 0, st>>>(b.reps, b.off_rows, b.R);
     k_b_mol_incoming<<<b.nblk_in, 32 * kInWarps, 0, st>>>(b.reps, b.off_in, b.R);
     return cudaGetLastError();
 }
@@ -750,15 +923,17 @@ cudaError_t mol_rows_intra(const MolLists& m, const double* pos, const double* h
 cudaError_t mol_rows_half(const MolLists& m, const double* pos, const double* hh, double rc2, int cap, int* cnt,
                           int* list, int* dropped, cudaStream_t st) {
     if (m.masks) {
-        k_mol_half_flat<true><<<kRowBlocksMol, 32 * kFlatWarps, 0, st>>>(pos, hh, m.n, m.off, m.amol, m.npart,
-                                                                         m.part, m.pmax, m.usize, m.pos32, rc2, cap,
-                                                                         cnt, list, dropped, m.flag, m.bm);
+        const int quads = m.M * ((m.usize + kQuad - 1) / kQuad), g = mol_atoms_per_warp(m.n);
+        const int blocks = std::min(kRowBlocksMol, ((g == 1 ? m.n : quads) + kQuadWarps - 1) / kQuadWarps);
+        auto k = g == 1 ? k_mol_half_quad<1> : k_mol_half_quad<kQuad>;
+        k<<<blocks, 32 * kQuadWarps, 0, st>>>(pos, hh, m.M, m.off, m.npart, m.part, m.cen, m.rad, m.pmax, m.usize,
+                                              m.pos32, rc2, cap, cnt, list, dropped, m.flag, m.bm);
         return cudaGetLastError();
     }
     if (m.usize > 0) {
-        k_mol_half_flat<false><<<kRowBlocksMol, 32 * kFlatWarps, 0, st>>>(pos, hh, m.n, m.off, m.amol, m.npart,
-                                                                          m.part, m.pmax, m.usize, m.pos32, rc2, cap,
-                                                                          cnt, list, dropped, m.flag, nullptr);
+        k_mol_half_flat<<<kRowBlocksMol, 32 * kFlatWarps, 0, st>>>(pos, hh, m.n, m.off, m.amol, m.npart, m.part, m.pmax,
+                                                                   m.usize, m.pos32, rc2, cap, cnt, list, dropped,
+                                                                   m.flag);
         return cudaGetLastError();
     }
     k_mol_rows<0><<<kRowBlocksMol, 256, 0, st>>>(pos, hh, m.n, m.off, m.amol, m.npart, m.part, m.pmax, m.pos32, rc2,

@@ -81,6 +81,7 @@ struct MolBatch {
     const int* off_rows = nullptr;
     const int* off_in = nullptr;
     int nblk_w = 0, nblk_rows = 0, nblk_in = 0;
+    long long atoms = 0;      // of all replicas
 };
 // The molecule-path rebuild of every replica of a batch, one launch per
 // phase, for equal molecules of 32-64 atoms (the candidate-bitmap path).
