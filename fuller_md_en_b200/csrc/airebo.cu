@@ -23,7 +23,8 @@
 #include "ljpair.cuh"
 #include "ljprune.cuh"
 #include "ljrow.cuh"
-#include "rebo_fn.cuh"
+#include "rebo_row.cuh"
+#include "rebomol.h"
 #include "step.h"
 #include "umma.cuh"
 #include "pdl.cuh"
@@ -32,64 +33,6 @@ namespace fmd {
 namespace {
 
 using namespace rebo;
-
-// Sum over the centre's other neighbours of fc * G(cos theta) (AI:301-309).
-__device__ double bo_sum(const double* __restrict__ pos, const int* __restrict__ cnt,
-                         const int* __restrict__ list, int cap, const double* h, const double* hi,
-                         int c, int skip, double bx, double by, double bz, double rb) {
-    double gs = 0.0;
-    const int m = cnt[c];
-    for (int kn = 0; kn < m; kn++) {
-        const int k = list[(size_t)c * cap + kn];
-        if (k == skip) continue;
-        double kx, ky, kz;
-        bond_vec(pos, c, k, h, hi, kx, ky, kz);
-        const double rk = sqrt(norm2_rn(kx, ky, kz));
-        if (rk > DMAX_CC) continue;
-        const double fk = sw_fc(rk);
-        if (fk < 1e-15) continue;
-        const double ct = clamp1((bx * kx + by * ky + bz * kz) / (rb * rk));
-        gs += fk * ang_g(ct);
-    }
-    return gs;
-}
-
-// Reference three-body forces on the neighbours of centre c (AI:361-419).
-// b = (1+gs)^-1/2 is passed in, so db/dgs = -1/2 (1+gs)^-3/2 = -b / (2 (1+gs)).
-__device__ __forceinline__ void bo_three_body(double* __restrict__ F, const double* __restrict__ pos,
-                              const int* __restrict__ cnt, const int* __restrict__ list, int cap,
-                              const double* h, const double* hi, int c, int skip, double bx, double by,
-                              double bz, double rb, double ux, double uy, double uz, double gs, double b,
-                              double fcut, double va) {
-    if (!(fabs(gs) > 1e-20 && va > 1e-20)) return;
-    const double dbp = -BO_DELTA * b / (1.0 + gs);
-    const double vh = 0.5 * fcut * va;
-    const double coeff = -vh * dbp;
-    const int m = cnt[c];
-    double fcx = 0.0, fcy = 0.0, fcz = 0.0;
-    for (int kn = 0; kn < m; kn++) {
-        const int k = list[(size_t)c * cap + kn];
-        if (k == skip) continue;
-        double kx, ky, kz;
-        bond_vec(pos, c, k, h, hi, kx, ky, kz);
-        const double rk = sqrt(norm2_rn(kx, ky, kz));
-        if (rk > DMAX_CC) continue;
-        const double fck = sw_fc(rk);
-        if (fck < 1e-15) continue;
-        const double dfck = sw_dfc(rk);
-        const double rki = 1.0 / rk;
-        const double rx = kx * rki, ry = ky * rki, rz = kz * rki;
-        const double ct = clamp1((bx * kx + by * ky + bz * kz) / (rb * rk));
-        const double gv = ang_g(ct), dgv = ang_dg(ct);
-        const double a1 = coeff * dfck * gv, a2 = coeff * fck * dgv;
-        const double fx = a1 * rx + a2 * ((ux - ct * rx) * rki);
-        const double fy = a1 * ry + a2 * ((uy - ct * ry) * rki);
-        const double fz = a1 * rz + a2 * ((uz - ct * rz) * rki);
-        atomic_add3(F, k, fx, fy, fz);
-        fcx -= fx; fcy -= fy; fcz -= fz;
-    }
-    atomic_add3(F, c, fcx, fcy, fcz);
-}
 
 // Four threads per atom share its row (slots jn, jn+4, jn+8): a fullerene
 // atom has three bonds, so one bond per thread; this gives ~4x the
@@ -112,48 +55,9 @@ k_rebo(const double* __restrict__ pos, const double* __restrict__ hh, const int*
     const long long total = (long long)na * kReboLanes;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t / kReboLanes), lane = (int)(t % kReboLanes);
-        const int m = cnt[i];
-        double fix = 0.0, fiy = 0.0, fiz = 0.0;
-        for (int jn = lane; jn < m; jn += kReboLanes) {
-            const int j = list[(size_t)i * cap + jn];
-            if (j <= i) continue;
-            double dx, dy, dz;
-            bond_vec(pos, i, j, h, hi, dx, dy, dz);
-            const double rij = sqrt(norm2_rn(dx, dy, dz));
-            if (rij > DMAX_CC) continue;
-            const double fcut = sw_fc(rij), dfcut = sw_dfc(rij);
-            if (fcut < 1e-15 && dfcut == 0) continue;
-            // V_R, V_A and derivatives (AI:173-183)
-            const double ea = A_CC * exp(-ALPHA_CC * rij);
-            const double vr = (1.0 + Q_CC / rij) * ea;
-            const double dvr = (-Q_CC / (rij * rij)) * ea + (1.0 + Q_CC / rij) * (-ALPHA_CC) * ea;
-            const double e1 = exp(-BETA1_CC * rij), e2 = exp(-BETA2_CC * rij), e3 = exp(-BETA3_CC * rij);
-            const double va = B1_CC * e1 + B2_CC * e2 + B3_CC * e3;
-            const double dva = -BETA1_CC * B1_CC * e1 - BETA2_CC * B2_CC * e2 - BETA3_CC * B3_CC * e3;
-            const double rinv = 1.0 / rij;
-            const double ux = dx * rinv, uy = dy * rinv, uz = dz * rinv;
-            const double gij = bo_sum(pos, cnt, list, cap, h, hi, i, j, dx, dy, dz, rij);
-            const double gji = bo_sum(pos, cnt, list, cap, h, hi, j, i, -dx, -dy, -dz, rij);
-            // (1+g)^-1/2 (AI:310, 323) as a reciprocal square root
-            const double bij = 1.0 / sqrt(1.0 + gij), bji = 1.0 / sqrt(1.0 + gji);
-            const double bbar = 0.5 * (bij + bji);
-            acc[0] += fcut * (vr - bbar * va);
-            const double fpair = (dfcut * (vr - bbar * va) + fcut * (dvr - bbar * dva)) * rinv;
-            fix += fpair * dx; fiy += fpair * dy; fiz += fpair * dz;
-            atomic_add3(F, j, -fpair * dx, -fpair * dy, -fpair * dz);
-            const double d[3] = {dx, dy, dz};
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int b = 0; b < 3; b++) acc[1 + a * 3 + b] -= d[a] * fpair * d[b];
-            bo_three_body(F, pos, cnt, list, cap, h, hi, i, j, dx, dy, dz, rij, ux, uy, uz, gij, bij, fcut, va);
-            bo_three_body(F, pos, cnt, list, cap, h, hi, j, i, -dx, -dy, -dz, rij, -ux, -uy, -uz, gji, bji, fcut,
-                          va);
-        }
-        if (fix != 0.0 || fiy != 0.0 || fiz != 0.0) atomic_add3(F, i, fix, fiy, fiz);
+        rebo_row<false>(pos, h, hi, cnt, list, cap, (int)(t / kReboLanes), (int)(t % kReboLanes), kReboLanes, F, acc);
     }
-    block_sum_store<kNV>(acc, sm, part + (size_t)blockIdx.x * kNV);
+    block_sum_fields<kNV>(acc, sm, part + (size_t)blockIdx.x * kNV);
 }
 
 // ------------------------------------------------- REBO on slot records --
@@ -196,12 +100,6 @@ k_rebo_slots(const double* __restrict__ pos, const double* __restrict__ hh, cons
     }
 }
 
-__device__ __forceinline__ void ang_g_dg(double x, double& g, double& dg) {
-    const double c2 = G_C0 * G_C0, d2 = G_D0 * G_D0, hh = 1.0 + x, inv = 1.0 / (d2 + hh * hh);
-    g = G_A0 * (1.0 + c2 / d2 - c2 * inv);
-    dg = G_A0 * 2.0 * c2 * hh * inv * inv;
-}
-
 // Sum over centre c's other slots of f_c G(cos) for the bond in slot skip_kn
 // of c's row (-1: the bond is not in c's row) whose vector is s*(bx,by,bz)
 // with s = +-1 (AI:301-309).  Rows hold no atom twice, so skipping the slot is
@@ -230,24 +128,6 @@ __device__ __forceinline__ double bo_sum_sl(const Slot* __restrict__ sl, int cap
 struct SlotBO {
     double b, g, coeff, vr, dvr, va, dva, ok;
 };
-
-__device__ __forceinline__ void rebo_pair_fn(double r, double rinv, double& vr, double& dvr, double& va,
-                                             double& dva) {
-    const double ea = A_CC * exp(-ALPHA_CC * r);
-    const double qr = Q_CC * rinv;
-    vr = (1.0 + qr) * ea;
-    dvr = (-qr * rinv) * ea + (1.0 + qr) * (-ALPHA_CC) * ea;
-    const double e1 = exp(-BETA1_CC * r), e2 = exp(-BETA2_CC * r), e3 = exp(-BETA3_CC * r);
-    va = B1_CC * e1 + B2_CC * e2 + B3_CC * e3;
-    dva = -BETA1_CC * B1_CC * e1 - BETA2_CC * B2_CC * e2 - BETA3_CC * B3_CC * e3;
-}
-
-// Three-body coefficient of centre c for a bond with f_c and V_A.
-__device__ __forceinline__ double three_body_coeff(double gs, double b, double fcut, double va) {
-    if (!(fabs(gs) > 1e-20 && va > 1e-20)) return 0.0;
-    const double dbp = -BO_DELTA * b / (1.0 + gs);
-    return -(0.5 * fcut * va) * dbp;
-}
 
 __global__ void __launch_bounds__(256)
 k_rebo_bo(const Slot* __restrict__ sl, const int* __restrict__ cnt, const int* __restrict__ list, int cap, int na,
@@ -533,7 +413,7 @@ k_rebo_force(const Slot* __restrict__ sl, const SlotBO* __restrict__ bo, const i
         seg_sum3(fcx, fcy, fcz, seg, lane, span);
         if (lead && valid && (fcx != 0.0 || fcy != 0.0 || fcz != 0.0)) atomic_add3(F, i, fcx, fcy, fcz);
     }
-    block_sum_store<kNV>(acc, sm, part + (size_t)blockIdx.x * kNV);
+    block_sum_fields<kNV>(acc, sm, part + (size_t)blockIdx.x * kNV);
 }
 
 LJP lj_params(int ff) { return lj_params_dev(ff); }
@@ -605,7 +485,7 @@ __device__ __forceinline__ void lj_gather_body(const double* __restrict__ pos, c
         lj_atom_done(i, fx, fy, fz, px, py, pz, hi, F, Facc, po, pc, lane, fa);
     }
     lj_virial_mirror<FULL_VIRIAL>(acc);
-    block_sum_store<kNV>(acc, sm, part + (size_t)blk * kNV);
+    block_sum_fields<kNV>(acc, sm, part + (size_t)blk * kNV);
 }
 
 // The rows of this evaluation: with po.words set, the full rows and pruned-
@@ -740,7 +620,7 @@ __device__ __forceinline__ void lj_gather_staged_body(const double* __restrict__
     // after an early exit, the copy issued for the next atom may still be in flight
     if (pending) umma::mbar_wait(&mb[cur ^ 1], (cur ^ 1) ? ph1 : ph0);
     lj_virial_mirror<FULL_VIRIAL>(acc);
-    block_sum_store<kNV>(acc, sm, part + (size_t)blk * kNV);
+    block_sum_fields<kNV>(acc, sm, part + (size_t)blk * kNV);
 }
 
 template <bool FULL_VIRIAL, bool F32, int U, int NT>
@@ -832,7 +712,8 @@ int rebo_slot_blocks(int na) { return std::max(1, std::min(kForceBlocks, (8 * na
 
 cudaError_t rebo_slots_launch(const double* pos, const double* hh, const int* cnt, const int* list, int cap,
                               int na, double* slots, double* F, double* part, int nblocks, const int* gate,
-                              int want, cudaStream_t st, const int* ids, bool phys) {
+                              int want, cudaStream_t st, const int* ids, bool phys, const ReboMol& mol) {
+    if (mol.M) return rebo_mol_launch(mol, pos, hh, cnt, list, cap, F, part, nblocks, gate, want, phys, st);
     Slot* sl = reinterpret_cast<Slot*>(slots);
     SlotBO* bo = reinterpret_cast<SlotBO*>(slots + (size_t)na * cap * 8);
     cudaError_t e;

@@ -110,4 +110,45 @@ __device__ __forceinline__ void block_sum_store(double (&v)[NV], double* sm, dou
     __syncthreads();
 }
 
+// One step of the warp's sum of NV fields: the lane keeps half of them (those
+// from `at` on if its bit O is clear, the rest otherwise) and hands the other
+// half over; the lane's fields are at .. end - 1.
+template <int NV, int O>
+__device__ __forceinline__ void fold_fields(double* v, int lane, int& at, int& end) {
+    if constexpr (NV > 1) {
+        constexpr int H = (NV + 1) / 2;
+        const bool hi = lane & O;
+#pragma unroll
+        for (int k = 0; k < H; k++) {
+            const double up = k + H < NV ? v[k + H] : 0.0;
+            const double send = hi ? v[k] : up;
+            v[k] = (hi ? up : v[k]) + __shfl_xor_sync(kFull, send, O);
+        }
+        if (hi) at += H;
+        else end = at + H < end ? at + H : end;
+        if constexpr (O > 1) fold_fields<H, O / 2>(v, lane, at, end);
+    } else {
+        v[0] += __shfl_xor_sync(kFull, v[0], O);
+        if constexpr (O > 1) fold_fields<1, O / 2>(v, lane, at, end);
+    }
+}
+
+// As block_sum_store, with 12 shuffles for 10 fields instead of 50 and the
+// warps' sums added by a thread per field (0.6 us of a block's end in the
+// cluster gather); out is global or shared memory.
+template <int NV>
+__device__ __forceinline__ void block_sum_fields(double (&v)[NV], double* sm, double* out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int at = 0, end = NV;
+    fold_fields<NV, 16>(v, lane, at, end);
+    if (at < end) sm[warp * NV + at] = v[0];
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        double t = 0.0;
+        for (int w = 0; w < nw; w++) t += sm[w * NV + threadIdx.x];
+        out[threadIdx.x] = t;
+    }
+    __syncthreads();
+}
+
 }  // namespace fmd

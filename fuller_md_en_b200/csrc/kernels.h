@@ -90,6 +90,13 @@ cudaError_t rebo_launch_gated(const double* pos, const double* hh, const int* cn
 // na * cap bond-order records; device scratch owned by the caller); otherwise
 // as rebo_launch_gated (gate may be null).
 constexpr int kReboSlotDoubles = 16;
+// Molecules (contiguous atoms off[m] .. off[m + 1]) whose atoms' REBO rows stay
+// within them: the term then goes by molecules (rebomol.cu), without slots or
+// ids.  M 0: none.
+struct ReboMol {
+    int M = 0, max_atoms = 0;
+    const int* off = nullptr;
+};
 int rebo_slot_blocks(int na);   // a grid for the occupied slots of na atoms
 // ids (may be null): the occupied slots in atom-major order packed into
 // 32-lane bins (no atom's slots cross a bin; unused lanes -1), ids[0] the
@@ -101,7 +108,8 @@ int rebo_slot_blocks(int na);   // a grid for the occupied slots of na atoms
 // three-body forces (FMD_PHYS_REBO).
 cudaError_t rebo_slots_launch(const double* pos, const double* hh, const int* cnt, const int* list, int cap,
                               int na, double* slots, double* F, double* part, int nblocks, const int* gate,
-                              int want, cudaStream_t st, const int* ids = nullptr, bool phys = false);
+                              int want, cudaStream_t st, const int* ids = nullptr, bool phys = false,
+                              const ReboMol& mol = ReboMol{});
 // REBO-II extension (rebo2.cu; no reference counterpart): bond order with
 // P_CC(N, 0), pi^rc_CC(N_ij, N_ji, N_conj) and the dihedral term
 // T_CC(...) sum (1 - cos^2 w) f_c f_c, and AIREBO's switched LJ.  Splines on

@@ -653,7 +653,7 @@ __device__ __forceinline__ void lj_clus_body(const LJClus& c, const double* __re
     if (lane == 0)
 #pragma unroll
         for (int k = 0; k < kNV; k++) acc[k] += sh.extra[w][k];
-    block_sum_store<kNV>(acc, sh.sm, part + (size_t)blk * kNV);
+    block_sum_fields<kNV>(acc, sh.sm, part + (size_t)blk * kNV);
 }
 
 template <bool FV, bool F32>

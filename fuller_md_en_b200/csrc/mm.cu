@@ -140,7 +140,7 @@ __device__ __forceinline__ void mm_bonded_body(const MMTopoDev& t, const double*
                               t.m_gamma[p], sg);
         }
     }
-    block_sum_store<kMMNV>(acc, sm, part + (size_t)blk * kMMNV);
+    block_sum_fields<kMMNV>(acc, sm, part + (size_t)blk * kMMNV);
 }
 
 __global__ void __launch_bounds__(128)

@@ -490,7 +490,7 @@ k_rebo2_bonds(const double* __restrict__ pos, const double* __restrict__ hh, con
     }
 #pragma unroll
     for (int q = 0; q < 9; q++) acc[1 + q] = w[q];
-    block_sum_store<kNV>(acc, sm, part + (size_t)blockIdx.x * kNV);
+    block_sum_fields<kNV>(acc, sm, part + (size_t)blockIdx.x * kNV);
 }
 
 // The LJ pairs closer than 2^(1/6) sigma (where the switch acts), compacted
@@ -568,7 +568,7 @@ k_lj_switch(const double* __restrict__ pos, const double* __restrict__ hh, const
     }
 #pragma unroll
     for (int q = 0; q < 9; q++) acc[1 + q] = w[q];
-    block_sum_store<kNV>(acc, sm, part + (size_t)blockIdx.x * kNV);
+    block_sum_fields<kNV>(acc, sm, part + (size_t)blockIdx.x * kNV);
 }
 
 // Cubic Hermite basis on [0,1] as polynomial coefficients of u^0..u^3:

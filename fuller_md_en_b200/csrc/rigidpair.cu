@@ -471,7 +471,7 @@ k_rigid_sum(RigidPair rp, const int* __restrict__ cnt, const int* __restrict__ l
             T[3 * i] = v[3]; T[3 * i + 1] = v[4]; T[3 * i + 2] = v[5];
         }
     }
-    block_sum_store<kNV>(tot, sm, part + (size_t)blockIdx.x * kNV);
+    block_sum_fields<kNV>(tot, sm, part + (size_t)blockIdx.x * kNV);
 }
 
 // Warps per molecule: about one own pair each (21) at 108 molecules, four at

@@ -641,7 +641,7 @@ __global__ void __launch_bounds__(kPB) k_rigid_kick2_end(StepArrays a, StepParam
     acc[kNV] = vv;
     acc[kNV + 1] = ww;
     __shared__ double rec[kNV + 2];
-    block_sum_store<kNV + 2>(acc, sm, rec);
+    block_sum_fields<kNV + 2>(acc, sm, rec);
     if (threadIdx.x < kNV) a.part_f1[(size_t)blockIdx.x * kNV + threadIdx.x] = rec[threadIdx.x];
     else if (threadIdx.x < kNV + 2) a.part_ke[2 * blockIdx.x + threadIdx.x - kNV] = rec[threadIdx.x];
     __threadfence();                      // this block's records before its ticket
@@ -760,9 +760,9 @@ cudaError_t enqueue_forces(const StepArrays& a, cudaStream_t st, bool judge, boo
             e = rebo2_launch(a.rebo2, a.pos, hh, a.cnt_b, a.list_b, a.cap_b, a.n, a.Facc, a.part_f1, a.rebo_blocks,
                              st);
         else if (a.sg) e = sg_enqueue_rebo(*a.sg, a, judge, st);
-        else if (a.rebo_slots)
+        else if (a.rebo_slots || a.rebo_mol.M)
             e = rebo_slots_launch(a.pos, hh, a.cnt_b, a.list_b, a.cap_b, a.n, a.rebo_slots, a.Facc, a.part_f1,
-                                  a.rebo_blocks, nullptr, 0, st, a.rebo_ids, a.rebo_phys != 0);
+                                  a.rebo_blocks, nullptr, 0, st, a.rebo_ids, a.rebo_phys != 0, a.rebo_mol);
         else e = rebo_launch(a.pos, hh, a.cnt_b, a.list_b, a.cap_b, a.n, a.Facc, a.part_f1, st);
         if (e != cudaSuccess) return e;
         e = enqueue_lj(a, FMD_FF_AIREBO, st);

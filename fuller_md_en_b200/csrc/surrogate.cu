@@ -501,7 +501,7 @@ k_sg_force(const double* __restrict__ pos, const double* __restrict__ hh, const 
         }
         if (fix != 0.0 || fiy != 0.0 || fiz != 0.0) atomic_add3(F, i, fix, fiy, fiz);
     }
-    block_sum_store<kNV>(acc, smr, part + (size_t)blockIdx.x * kNV);
+    block_sum_fields<kNV>(acc, smr, part + (size_t)blockIdx.x * kNV);
 }
 
 __global__ void k_sg_pack(const double* __restrict__ P, uint16_t* __restrict__ img, float* __restrict__ vec) {

@@ -15,6 +15,7 @@
 #include "ljclus.h"
 #include "ljprune.cuh"
 #include "mmmol.h"
+#include "rebomol.h"
 #include "step.h"
 #include "system.h"
 #include "sg_host.h"
@@ -127,14 +128,6 @@ int System::alloc_lists(double rc_list_a, int cap_a_, double rc_list_b, int cap_
         cudaMemsetAsync(lst, 0, sizeof(int) * (size_t)n * cap_b_, ctx->stream);
         arr.cnt_b = cnt; arr.list_b = lst;
         if (cells_alloc(cells_b, n, h0, rc_b, 1, owned_alloc()) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "cell allocation failed");
-        if (alloc(&arr.rebo_slots, (size_t)n * cap_b_ * kReboSlotDoubles, (const double*)nullptr))
-            return ctx->fail(FMD_ERR_CUDA, "list allocation failed");
-        int* ids;
-        if (alloc(&ids, 1 + (size_t)kIdsLanes * n + (size_t)n * cap_b_, (const int*)nullptr) ||
-            alloc(&rebo_bsum, (size_t)rebo_ids_scratch(n), (const int*)nullptr))
-            return ctx->fail(FMD_ERR_CUDA, "list allocation failed");
-        cudaMemsetAsync(ids, 0, sizeof(int), ctx->stream);
-        arr.rebo_ids = ids;
     }
     if (transpose) {
         arr.in_cap = kInCap + cap_a_;   // full rows: incoming entries then the row itself
@@ -146,6 +139,32 @@ int System::alloc_lists(double rc_list_a, int cap_a_, double rc_list_b, int cap_
 }
 
 // Rebuild of every list this kind uses, as the driver does at gstep % nlup == 0.
+// The REBO term goes by molecules where they are contiguous and fit a block,
+// else over slot records and their index.
+int System::alloc_rebo() {
+    if (mol.ok && mol.max_atoms <= kReboMolAtoms) {
+        arr.rebo_mol.M = mol.M;
+        arr.rebo_mol.max_atoms = mol.max_atoms;
+        arr.rebo_mol.off = mol.off;
+        return FMD_OK;
+    }
+    const int n = arr.n;
+    int* ids;
+    if (alloc(&arr.rebo_slots, (size_t)n * arr.cap_b * kReboSlotDoubles, (const double*)nullptr) ||
+        alloc(&ids, 1 + (size_t)kIdsLanes * n + (size_t)n * arr.cap_b, (const int*)nullptr) ||
+        alloc(&rebo_bsum, (size_t)rebo_ids_scratch(n), (const int*)nullptr))
+        return ctx->fail(FMD_ERR_CUDA, "list allocation failed");
+    cudaMemsetAsync(ids, 0, sizeof(int), ctx->stream);
+    arr.rebo_ids = ids;
+    return FMD_OK;
+}
+
+// Partial records of the plain REBO term.
+int System::rebo_records() const {
+    const bool molecules = arr.rebo_mol.M && !(arr.rebo2_flags & FMD_REBO2_BOND_ORDER);
+    return molecules ? rebo_mol_blocks(arr.rebo_mol) : rebo_slot_blocks(arr.n);
+}
+
 int System::alloc_prune(double rc_lj) {
     if (!arr.in_list) return FMD_OK;
     const int n = arr.n;
@@ -393,9 +412,10 @@ LJShape System::pick_lj_shape(bool pruned, int& rc) {
     auto short_range = [&]() -> cudaError_t {
         const double* hh = arr.S->h;
         if (arr.kind == FMD_SYS_MM) return mm_bonded_launch(arr.topo, arr.pos, hh, arr.Facc, arr.part_f1, st);
-        if (arr.rebo_slots)
+        if (arr.rebo_slots || arr.rebo_mol.M)
             return rebo_slots_launch(arr.pos, hh, arr.cnt_b, arr.list_b, arr.cap_b, arr.n, arr.rebo_slots, arr.Facc,
-                                     arr.part_f1, arr.rebo_blocks, nullptr, 0, st, arr.rebo_ids, arr.rebo_phys != 0);
+                                     arr.part_f1, arr.rebo_blocks, nullptr, 0, st, arr.rebo_ids, arr.rebo_phys != 0,
+                                     arr.rebo_mol);
         return rebo_launch(arr.pos, hh, arr.cnt_b, arr.list_b, arr.cap_b, arr.n, arr.Facc, arr.part_f1, st);
     };
     const LJPruneOut walk = pruned ? lj_prune_out(prune) : LJPruneOut{};
@@ -750,7 +770,6 @@ extern "C" int fmd_system_create_airebo(fmd_ctx* ctx, const fmd_run_params* p, i
     s->arr.n = na;
     s->arr.precision = p->precision;
     s->arr.lj_blocks = lj_gather_blocks(FMD_FF_AIREBO, p->precision, s->arr.lj_shape, 0, na);
-    s->arr.rebo_blocks = rebo_slot_blocks(na);
     int rc = s->alloc_common(pos, vel, h, npt);
     if (rc != FMD_OK) return rc;
     double* m; int* mid;
@@ -760,7 +779,9 @@ extern "C" int fmd_system_create_airebo(fmd_ctx* ctx, const fmd_run_params* p, i
     const double rebo_rcut = 2.0 + 0.3;         // AI:116
     if ((rc = s->alloc_lists(lj_rcut + 2.0, 400, rebo_rcut, 12, true)) != FMD_OK) return rc;
     if (fmd::mol_lists_alloc(s->mol, na, mol_id, s->owned_alloc()) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "list allocation failed");
-    if ((rc = s->alloc_prune(lj_rcut)) != FMD_OK || (rc = s->alloc_clus(pos)) != FMD_OK) return rc;
+    if ((rc = s->alloc_rebo()) != FMD_OK || (rc = s->alloc_prune(lj_rcut)) != FMD_OK || (rc = s->alloc_clus(pos)) != FMD_OK)
+        return rc;
+    s->arr.rebo_blocks = s->rebo_records();
     out[0] = new fmd_system{std::move(s)};
     return FMD_OK;
 }
@@ -1030,7 +1051,7 @@ extern "C" int fmd_system_set_physics(fmd_system* s, int flags) {
         return y.ctx->fail(FMD_ERR_ARG, "fmd_system_set_physics: FMD_PHYS_QUAT needs a rigid system");
     if ((flags & FMD_PHYS_MM_BONDED) && y.arr.kind != FMD_SYS_MM)
         return y.ctx->fail(FMD_ERR_ARG, "fmd_system_set_physics: FMD_PHYS_MM_BONDED needs an MM system");
-    if ((flags & FMD_PHYS_REBO) && (y.arr.kind != FMD_SYS_AIREBO || !y.arr.rebo_slots))
+    if ((flags & FMD_PHYS_REBO) && y.arr.kind != FMD_SYS_AIREBO)
         return y.ctx->fail(FMD_ERR_ARG, "fmd_system_set_physics: FMD_PHYS_REBO needs an AIREBO system");
     y.arr.topo.physical = (flags & FMD_PHYS_MM_BONDED) ? 1 : 0;
     y.arr.rebo_phys = (flags & FMD_PHYS_REBO) ? 1 : 0;
@@ -1082,6 +1103,7 @@ extern "C" int fmd_system_set_rebo2(fmd_system* s, const fmd_rebo2_knots* kn, in
             return y.ctx->fail(FMD_ERR_CUDA, "fmd_system_set_rebo2: copy failed");
     }
     y.arr.rebo2_flags = flags;
+    y.arr.rebo_blocks = y.rebo_records();
     return y.ctx->sync_check("fmd_system_set_rebo2");
 }
 
@@ -1136,7 +1158,8 @@ extern "C" int fmd_system_kernel_ms(fmd_system* s, int stage, int reps, double* 
                     return sg_enqueue_rebo(*a.sg, a, false, st);
                 if (a.kind == FMD_SYS_AIREBO)
                     return rebo_slots_launch(a.pos, hh, a.cnt_b, a.list_b, a.cap_b, a.n, a.rebo_slots, a.Facc,
-                                             a.part_f1, a.rebo_blocks, nullptr, 0, st, a.rebo_ids, a.rebo_phys != 0);
+                                             a.part_f1, a.rebo_blocks, nullptr, 0, st, a.rebo_ids, a.rebo_phys != 0,
+                                             a.rebo_mol);
                 if (a.kind == FMD_SYS_MM) return mm_bonded_launch(a.topo, a.pos, hh, a.Facc, a.part_f1, st);
                 return enqueue_rigid(a, st);
             case 2:
@@ -1371,7 +1394,7 @@ int fmd::System::use_surrogate(fmd_sg* model, int judge_every, double rmse_max) 
     drop_graphs();                       // captured graphs hold the old REBO term
     if (!model) {
         arr.sg = nullptr;
-        arr.rebo_blocks = rebo_slot_blocks(arr.n);
+        arr.rebo_blocks = rebo_records();
     } else {
         if (arr.rebo2_flags & FMD_REBO2_BOND_ORDER)
             return ctx->fail(FMD_ERR_ARG, "fmd_system_use_surrogate: the system uses the REBO-II bond order");

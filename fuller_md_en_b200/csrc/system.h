@@ -40,6 +40,8 @@ struct System {
     DevAlloc owned_alloc() { return DevAlloc{this, &System::alloc_raw}; }
     int alloc_common(const double* pos, const double* vel, const double* h, const fmd_npt* npt);
     int alloc_lists(double rc_list_a, int cap_a, double rc_list_b, int cap_b, bool transpose);
+    int alloc_rebo();
+    int rebo_records() const;
     int alloc_prune(double rc_lj);
     int alloc_clus(const double* pos);
     double lazy_edge() const;
