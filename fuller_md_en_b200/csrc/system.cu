@@ -42,6 +42,7 @@ void System::drop_graphs() {
         for (auto& b : a)
             for (auto& g : b)
                 if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+    if (chain) { cudaGraphExecDestroy(chain); chain = nullptr; }
 }
 
 void System::release() {
@@ -625,14 +626,22 @@ int System::init() {
     return FMD_OK;
 }
 
+// Steps of a chain (rebuilds every 20 or 25 steps leave 3 or 4 of them between),
+// and those a system needs before one is captured.
+constexpr int kChain = 6, kChainSteps = 64;
+
 int System::capture(bool rebuild, bool phase, bool judge) {
-    cudaGraphExec_t& ge = graphs[rebuild ? 1 : 0][phase ? 1 : 0][judge ? 1 : 0];
+    return capture_steps(graphs[rebuild ? 1 : 0][phase ? 1 : 0][judge ? 1 : 0], 1, rebuild, phase, judge);
+}
+
+int System::capture_steps(cudaGraphExec_t& ge, int count, bool rebuild, bool phase, bool judge) {
     if (ge) return FMD_OK;
     cudaStream_t st = ctx->stream;
     cudaGraph_t graph;
     if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
         return ctx->fail(FMD_ERR_CUDA, "graph capture failed to start");
-    cudaError_t e = enqueue_variant(rebuild, phase, st, judge);
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < count && e == cudaSuccess; k++) e = enqueue_variant(rebuild, phase, st, judge);
     cudaError_t e2 = cudaStreamEndCapture(st, &graph);
     if (e != cudaSuccess || e2 != cudaSuccess)
         return ctx->fail(FMD_ERR_CUDA, std::string("graph capture failed: ") +
@@ -673,8 +682,25 @@ int System::enqueue(int first, int last) {
     cudaMemcpyAsync(&arr.S->gstep, &g0, sizeof(int), cudaMemcpyHostToDevice, st);
     // rows a batch left unbuilt, for a gather that needs them
     if (!arr.clus.on && ensure_full_rows(st) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "full rows failed");
+    // Between two graphs the GPU idles for about 3 us, a tenth of a small step:
+    // plain steps go kChain to a graph.  It is captured when the system's steps
+    // pay for it (it costs the host what some 20 gaps cost the GPU), behind steps
+    // already enqueued, so that the GPU does not wait for it.
+    const bool many = p.use_graphs && steps_done + (last - first + 1) >= kChainSteps;
+    auto plain = [&](int g) { return g % p.nlup != 0 && g > p.coldstart + p.warmup && !judge_step(g); };
     for (int g = first; g <= last; g++) {
         if (arr.clus.on && g % p.nlup == 0) full_rows_stale = true;
+        if (many && (chain || g - first >= kChain)) {
+            int k = 0;
+            while (k < kChain && g + k <= last && plain(g + k)) k++;
+            if (k == kChain) {
+                int rc = capture_steps(chain, kChain, false, false, false);
+                if (rc != FMD_OK) return rc;
+                if (cudaGraphLaunch(chain, st) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "graph launch failed");
+                g += kChain - 1;
+                continue;
+            }
+        }
         if (p.use_graphs) {
             const int r = (g % p.nlup) == 0, ph = g <= p.coldstart + p.warmup, j = judge_step(g);
             int rc = capture(r != 0, ph != 0, j != 0);
@@ -685,6 +711,7 @@ int System::enqueue(int first, int last) {
             if (enqueue_one(g, st) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "step launch failed");
         }
     }
+    steps_done += last - first + 1;
     return FMD_OK;
 }
 

@@ -31,6 +31,10 @@ struct System {
     bool lj_pinned = false;            // launch shape of the row gather pinned by the caller
     // one graph per {rebuild, cold/warm phase, judge of the learned REBO term}
     cudaGraphExec_t graphs[2][2][2] = {};
+    // several plain steps (no rebuild, phase or judge) in one graph, once the
+    // system has run, or is to run, enough of them (enqueue)
+    cudaGraphExec_t chain = nullptr;
+    long long steps_done = 0;
     std::vector<std::pair<void*, size_t>> owned;   // blocks from the context's cache, with their sizes
     std::unique_ptr<SgStep> sg;        // learned REBO term (AIREBO only), nullptr: plain
 
@@ -72,6 +76,7 @@ struct System {
     int tune_lj_pruned(bool run_tuner, bool* pending);
     LJShape pick_lj_shape(bool pruned, int& rc);
     void set_lj_blocks();
+    int capture_steps(cudaGraphExec_t& ge, int count, bool rebuild, bool phase, bool judge);
     int capture(bool rebuild, bool phase, bool judge = false);
     void drop_graphs();
     int use_surrogate(fmd_sg* model, int judge_every, double rmse_max);
