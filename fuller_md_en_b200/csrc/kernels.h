@@ -142,10 +142,11 @@ struct Rebo2Dev {
 void rebo2_coeffs(const double* knots, double* pcc, double* pirc, double* tcc);
 // N_k into t.ncoord.
 cudaError_t rebo2_coord_launch(const Rebo2Dev& t, const double* pos, const double* hh, const int* cnt,
-                               const int* list, int cap, int na, cudaStream_t st);
+                               const int* list, int cap, int na, bool bonds, cudaStream_t st);
 // REBO-II energy over the bonds i < j of the REBO rows: forces -grad E ADDED
 // into F, {E, W9} partials in part[nblk * kNV] (full virial).  Computes
 // t.ncoord first.
+int rebo2_blocks(int na);   // a grid for the bonds of na atoms
 cudaError_t rebo2_launch(const Rebo2Dev& t, const double* pos, const double* hh, const int* cnt, const int* list,
                          int cap, int na, double* F, double* part, int nblk, cudaStream_t st);
 // Switched-LJ correction over the LJ half rows (cnt_a, list_a): energy

@@ -387,79 +387,81 @@ __device__ V3 bo_grad(const Geo& g, double* __restrict__ F, double (&w)[9], int 
     return gd;
 }
 
-__global__ void __launch_bounds__(256)
-k_rebo2_coord(const double* __restrict__ pos, const double* __restrict__ hh, const int* __restrict__ cnt,
-              const int* __restrict__ list, int cap, int na, double* __restrict__ ncoord) {
-    FMD_PDL_WAIT();
-    __shared__ double s_hh[18];
-    if (threadIdx.x < 18) s_hh[threadIdx.x] = hh[threadIdx.x];
-    __syncthreads();
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < na; k += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int mn = 0; mn < cnt[k]; mn++) {
-            double x, y, z;
-            bond_vec(pos, k, list[(size_t)k * cap + mn], s_hh, s_hh + 9, x, y, z);
-            const double r = sqrt(x * x + y * y + z * z);
-            if (r < DMAX_CC) s += sw_fc(r);
-        }
-        ncoord[k] = s;
-    }
-}
-
-// Appends (i, j) to a compacted work list from every lane of the warp that
-// takes its entry (one atomic per warp); entries beyond cap are dropped and
-// reported in err.  The whole warp calls it.
-__device__ __forceinline__ void warp_append(bool take, int i, int j, int2* __restrict__ out, int* __restrict__ count,
-                                            int cap, DevErr* err) {
-    const unsigned m = __ballot_sync(kFull, take);
-    if (!m) return;
-    const int lane = threadIdx.x & 31, lead = __ffs(m) - 1;
-    int base = 0;
-    if (lane == lead) base = atomicAdd(count, __popc(m));
-    base = __shfl_sync(kFull, base, lead);
-    if (!take) return;
-    const int k = base + __popc(m & ((1u << lane) - 1u));
+// Entry k of a work list; entries beyond cap are dropped and reported in err.
+__device__ __forceinline__ void append_at(int k, int i, int j, int2* __restrict__ out, int cap, DevErr* err) {
     if (k < cap) out[k] = make_int2(i, j);
     else if (err && atomicCAS(&err->code, FMD_OK, FMD_ERR_CAPACITY) == FMD_OK) {
         err->where = K_REBO2; err->index = i; err->value = k + 1;
     }
 }
 
-// The bonds of the REBO rows: slot i -> j with j > i (the enumeration of
-// AI:286-290) and r < D_max, compacted (the rows are 12 wide and hold ~3).
-__global__ void __launch_bounds__(256)
-k_rebo2_scan(const double* __restrict__ pos, const double* __restrict__ hh, const int* __restrict__ cnt,
-             const int* __restrict__ list, int cap, int na, Rebo2Dev t) {
+// Coordination numbers, and with BONDS the list of bonds: row entries i -> j
+// with j > i (the enumeration of AI:286-290) and r < D_max (the rows are 12 wide
+// and hold ~3), a thread per row, one atomic per block.  4.1 us for the numbers
+// alone and 10.5 for a scan of every slot with a global atomic per warp before.
+constexpr int kCoordThreads = 256;
+
+template <bool BONDS>
+__global__ void __launch_bounds__(kCoordThreads)
+k_rebo2_coord(const double* __restrict__ pos, const double* __restrict__ hh, const int* __restrict__ cnt,
+              const int* __restrict__ list, int cap, int na, double* __restrict__ ncoord, int2* __restrict__ bonds,
+              int* __restrict__ nbonds) {
     FMD_PDL_WAIT();
     __shared__ double s_hh[18];
+    __shared__ int s_n[kCoordThreads / 32], s_base;
     if (threadIdx.x < 18) s_hh[threadIdx.x] = hh[threadIdx.x];
     __syncthreads();
-    const long long tot = (long long)na * cap, stride = (long long)gridDim.x * blockDim.x;
-    for (long long b = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); b < tot; b += stride) {
-        const long long s = b + (threadIdx.x & 31);
-        bool take = false;
-        int i = 0, j = 0;
-        if (s < tot) {
-            i = (int)(s / cap);
-            const int jn = (int)(s - (long long)i * cap);
-            if (jn < cnt[i]) {
-                j = list[s];
-                if (j > i) {
-                    double x, y, z;
-                    bond_vec(pos, i, j, s_hh, s_hh + 9, x, y, z);
-                    take = sqrt(x * x + y * y + z * z) < DMAX_CC;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int k0 = blockIdx.x * kCoordThreads; k0 < na; k0 += gridDim.x * kCoordThreads) {
+        const int k = k0 + threadIdx.x;
+        unsigned mine = 0u;                    // the row's first 32 entries that are bonds k -> j > k
+        if (k < na) {
+            double s = 0.0;
+            for (int mn = 0; mn < cnt[k]; mn++) {
+                const int j = list[(size_t)k * cap + mn];
+                double x, y, z;
+                bond_vec(pos, k, j, s_hh, s_hh + 9, x, y, z);
+                const double r = sqrt(x * x + y * y + z * z);
+                if (r < DMAX_CC) {
+                    s += sw_fc(r);
+                    if (!BONDS || j < k) continue;
+                    if (mn < 32) mine |= 1u << mn;
+                    else bonds[atomicAdd(nbonds, 1)] = make_int2(k, j);
                 }
             }
+            ncoord[k] = s;
         }
-        warp_append(take, i, j, t.bonds, &t.counts[0], na * cap, nullptr);
+        if (!BONDS) continue;
+        const int c = __popc(mine);
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) s_n[w] = incl;
+        __syncthreads();
+        int before = 0, total = 0;
+        for (int q = 0; q < kCoordThreads / 32; q++) {
+            if (q < w) before += s_n[q];
+            total += s_n[q];
+        }
+        if (threadIdx.x == 0) s_base = atomicAdd(nbonds, total);
+        __syncthreads();
+        int at = s_base + before + incl - c;
+        for (; mine; mine &= mine - 1u) bonds[at++] = make_int2(k, list[(size_t)k * cap + __ffs(mine) - 1]);
+        __syncthreads();
     }
 }
 
 // One thread per bond of the compacted list: the bond's energy, and forces
-// and virial of its gradient.  Capped at 128 registers (4 blocks per SM; some
-// spill to L1): the uncapped kernel held 254 registers at 7 warps per SM and
-// took 123 us at nc = 5, the capped one 97 us.
-__global__ void __launch_bounds__(128, 4)
+// and virial of its gradient.  Bound by the latency of a thread's chain (30,000
+// atoms have 45,000 bonds, 10 warps an SM), so registers go to the threads as
+// long as all bonds fit the GPU at once: 5 blocks of 64 per SM (204 registers)
+// 95 us, 4 of 128 (128 registers, spilling) 104, 8 of 64 101, 4 of 64 (two
+// rounds) 169 us.
+constexpr int kBondThreads = 64, kBondBlocks = 5;
+__global__ void __launch_bounds__(kBondThreads, kBondBlocks)
 k_rebo2_bonds(const double* __restrict__ pos, const double* __restrict__ hh, const int* __restrict__ cnt,
               const int* __restrict__ list, int cap, Rebo2Dev t, double* __restrict__ F, double* __restrict__ part) {
     FMD_PDL_WAIT();
@@ -494,7 +496,14 @@ k_rebo2_bonds(const double* __restrict__ pos, const double* __restrict__ hh, con
 }
 
 // The LJ pairs closer than 2^(1/6) sigma (where the switch acts), compacted
-// from the half rows.
+// from the half rows: a warp per atom, kScanU slices of 32 entries in flight.
+// The distance is FP32 (its square off by less than 0.006 A^2 where it is used:
+// cell edges below 2048 A, half the narrowest beyond the radius by 1 A) with a
+// margin: the switch is zero for the few pairs that the margin adds.  30,000
+// atoms: 42 us; 79 us with a thread per slot of the table (occupied or
+// not), a 64-bit division to find its atom and the FP64 image of every entry.
+constexpr int kScanU = 4;
+
 __global__ void __launch_bounds__(256)
 k_lj_switch_scan(const double* __restrict__ pos, const double* __restrict__ hh, const int* __restrict__ cnt_a,
                  const int* __restrict__ list_a, int cap_a, int na, Rebo2Dev t) {
@@ -502,24 +511,60 @@ k_lj_switch_scan(const double* __restrict__ pos, const double* __restrict__ hh, 
     __shared__ double s_hh[18];
     if (threadIdx.x < 18) s_hh[threadIdx.x] = hh[threadIdx.x];
     __syncthreads();
+    const double* h = s_hh;
+    const double* hi = s_hh + 9;
     const LJP lp = lj_params_dev(FMD_FF_AIREBO);
     const double rmax2 = kSwitchRmaxOverSigma2 * lp.sig2;
-    const long long tot = (long long)na * cap_a, stride = (long long)gridDim.x * blockDim.x;
-    for (long long b = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); b < tot; b += stride) {
-        const long long s = b + (threadIdx.x & 31);
-        bool take = false;
-        int i = 0, j = 0;
-        if (s < tot) {
-            i = (int)(s / cap_a);
-            const int jn = (int)(s - (long long)i * cap_a);
-            if (jn < cnt_a[i]) {
-                j = list_a[s];
-                double x, y, z;
-                bond_vec(pos, i, j, s_hh, s_hh + 9, x, y, z);
-                take = x * x + y * y + z * z < rmax2;
+    const bool diag = h[1] == 0.0 && h[2] == 0.0 && h[3] == 0.0 && h[5] == 0.0 && h[6] == 0.0 && h[7] == 0.0 &&
+                      hi[1] == 0.0 && hi[2] == 0.0 && hi[3] == 0.0 && hi[5] == 0.0 && hi[6] == 0.0 && hi[7] == 0.0;
+    const bool screen = diag && 0.5 * fmin(fabs(h[0]), fmin(fabs(h[4]), fabs(h[8]))) > sqrt(rmax2) + 1.0 &&
+                        fmax(fabs(h[0]), fmax(fabs(h[4]), fabs(h[8]))) < 2048.0;
+    const float L[3] = {(float)h[0], (float)h[4], (float)h[8]}, Li[3] = {(float)hi[0], (float)hi[4], (float)hi[8]};
+    const float far2 = (float)rmax2 + 0.01f;
+    const int lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
+    for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < na; i += nw) {
+        const int c = min(cnt_a[i], cap_a);
+        const int* row = list_a + (size_t)i * cap_a;
+        const double px = pos[3 * i], py = pos[3 * i + 1], pz = pos[3 * i + 2];
+        for (int b = 0; b < c; b += 32 * kScanU) {
+            int j[kScanU];
+            double x[kScanU], y[kScanU], z[kScanU];
+#pragma unroll
+            for (int u = 0; u < kScanU; u++) j[u] = b + 32 * u + lane < c ? row[b + 32 * u + lane] : -1;
+#pragma unroll
+            for (int u = 0; u < kScanU; u++) {
+                const int q = j[u] < 0 ? i : j[u];
+                x[u] = pos[3 * q]; y[u] = pos[3 * q + 1]; z[u] = pos[3 * q + 2];
+            }
+            unsigned m[kScanU];
+            int total = 0;
+#pragma unroll
+            for (int u = 0; u < kScanU; u++) {
+                float dx = (float)(x[u] - px), dy = (float)(y[u] - py), dz = (float)(z[u] - pz);
+                dx = fmaf(-L[0], rintf(dx * Li[0]), dx);
+                dy = fmaf(-L[1], rintf(dy * Li[1]), dy);
+                dz = fmaf(-L[2], rintf(dz * Li[2]), dz);
+                bool take = j[u] >= 0 && !(screen && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > far2);
+                if (!screen && take) {
+                    double ex, ey, ez;
+                    bond_vec(pos, i, j[u], h, hi, ex, ey, ez);
+                    take = ex * ex + ey * ey + ez * ez < rmax2;
+                }
+                m[u] = __ballot_sync(kFull, take);
+                total += __popc(m[u]);
+            }
+            if (total == 0) continue;
+            // one atomic for the slices together
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&t.counts[1], total);
+            at = __shfl_sync(kFull, at, 0);
+#pragma unroll
+            for (int u = 0; u < kScanU; u++) {
+                const int k = at + __popc(m[u] & ((1u << lane) - 1u));
+                if ((m[u] >> lane) & 1u) append_at(k, i, j[u], t.sw_pairs, t.sw_cap, t.err);
+                at += __popc(m[u]);
             }
         }
-        warp_append(take, i, j, t.sw_pairs, &t.counts[1], t.sw_cap, t.err);
     }
 }
 
@@ -577,21 +622,23 @@ constexpr double kHerm[4][4] = {{1, 0, -3, 2}, {0, 1, -2, 1}, {0, 0, 3, -2}, {0,
 
 }  // namespace
 
+int rebo2_blocks(int na) {
+    return std::max(1, std::min({(3 * na / 2 + kBondThreads - 1) / kBondThreads, kBondBlocks * kSMs, std::max(kForceBlocks, na)}));
+}
+
 cudaError_t rebo2_coord_launch(const Rebo2Dev& t, const double* pos, const double* hh, const int* cnt,
-                               const int* list, int cap, int na, cudaStream_t st) {
+                               const int* list, int cap, int na, bool bonds, cudaStream_t st) {
     const int nb = std::max(1, std::min((na + 255) / 256, kForceBlocks));
-    return launch_pdl(k_rebo2_coord, dim3(nb), dim3(256), 0, st, pos, hh, cnt, list, cap, na, t.ncoord);
+    auto k = bonds ? k_rebo2_coord<true> : k_rebo2_coord<false>;
+    return launch_pdl(k, dim3(nb), dim3(kCoordThreads), 0, st, pos, hh, cnt, list, cap, na, t.ncoord, t.bonds, t.counts);
 }
 
 cudaError_t rebo2_launch(const Rebo2Dev& t, const double* pos, const double* hh, const int* cnt, const int* list,
                          int cap, int na, double* F, double* part, int nblk, cudaStream_t st) {
     cudaError_t e;
     if ((e = cudaMemsetAsync(t.counts, 0, 2 * sizeof(int), st)) != cudaSuccess) return e;
-    if ((e = rebo2_coord_launch(t, pos, hh, cnt, list, cap, na, st)) != cudaSuccess) return e;
-    const int ns = std::max(1, std::min((int)(((long long)na * cap + 255) / 256), kForceBlocks));
-    if ((e = launch_pdl(k_rebo2_scan, dim3(ns), dim3(256), 0, st, pos, hh, cnt, list, cap, na, t)) != cudaSuccess)
-        return e;
-    return launch_pdl(k_rebo2_bonds, dim3(nblk), dim3(128), 0, st, pos, hh, cnt, list, cap, t, F, part);
+    if ((e = rebo2_coord_launch(t, pos, hh, cnt, list, cap, na, true, st)) != cudaSuccess) return e;
+    return launch_pdl(k_rebo2_bonds, dim3(nblk), dim3(kBondThreads), 0, st, pos, hh, cnt, list, cap, t, F, part);
 }
 
 cudaError_t lj_switch_launch(const Rebo2Dev& t, const double* pos, const double* hh, const int* cnt_b,
@@ -599,8 +646,8 @@ cudaError_t lj_switch_launch(const Rebo2Dev& t, const double* pos, const double*
                              double* F, double* part, int nblk, bool coord_ready, cudaStream_t st) {
     cudaError_t e;
     if ((e = cudaMemsetAsync(t.counts + 1, 0, sizeof(int), st)) != cudaSuccess) return e;
-    if (!coord_ready && (e = rebo2_coord_launch(t, pos, hh, cnt_b, list_b, cap_b, na, st)) != cudaSuccess) return e;
-    const int ns = std::max(1, std::min((int)(((long long)na * cap_a + 255) / 256), 4 * kForceBlocks));
+    if (!coord_ready && (e = rebo2_coord_launch(t, pos, hh, cnt_b, list_b, cap_b, na, false, st)) != cudaSuccess) return e;
+    const int ns = std::max(1, std::min((na + 7) / 8, 4 * kForceBlocks));
     if ((e = launch_pdl(k_lj_switch_scan, dim3(ns), dim3(256), 0, st, pos, hh, cnt_a, list_a, cap_a, na, t)) !=
         cudaSuccess)
         return e;

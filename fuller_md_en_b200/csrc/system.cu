@@ -160,10 +160,10 @@ int System::alloc_rebo() {
     return FMD_OK;
 }
 
-// Partial records of the plain REBO term.
+// Partial records of the REBO term (the learned one apart).
 int System::rebo_records() const {
-    const bool molecules = arr.rebo_mol.M && !(arr.rebo2_flags & FMD_REBO2_BOND_ORDER);
-    return molecules ? rebo_mol_blocks(arr.rebo_mol) : rebo_slot_blocks(arr.n);
+    if (arr.rebo2_flags & FMD_REBO2_BOND_ORDER) return rebo2_blocks(arr.n);
+    return arr.rebo_mol.M ? rebo_mol_blocks(arr.rebo_mol) : rebo_slot_blocks(arr.n);
 }
 
 int System::alloc_prune(double rc_lj) {
