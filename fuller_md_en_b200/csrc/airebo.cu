@@ -672,6 +672,7 @@ k_b_lj_gather(const StepArrays* __restrict__ As, const int* __restrict__ off, in
 }
 
 __global__ void k_reduce(const double* __restrict__ part, int nblk, int nv, double* __restrict__ out) {
+    FMD_PDL_WAIT();
     __shared__ double sm[32 * 16];
     double acc[16];
 #pragma unroll
@@ -975,8 +976,7 @@ cudaError_t batch_lj_launch(const StepArrays* As, const int* off, int R, int nbl
 }
 
 cudaError_t reduce_partials(const double* part, int nblk, int nv, double* out, cudaStream_t st) {
-    k_reduce<<<1, 256, 0, st>>>(part, nblk, nv, out);
-    return cudaGetLastError();
+    return launch_pdl(k_reduce, dim3(1), dim3(256), 0, st, part, nblk, nv, out);
 }
 
 }  // namespace fmd

@@ -17,6 +17,7 @@
 #include <cuda_bf16.h>
 
 #include "kernels.h"
+#include "pdl.cuh"
 #include "sg_dev.cuh"
 #include "sg_train.cuh"
 #include "umma.cuh"
@@ -31,6 +32,7 @@ using namespace dev;
 __global__ void __launch_bounds__(256)
 k_sg_lambda(const double* __restrict__ F, const double* __restrict__ Fref, int na, double wF,
             double* __restrict__ lamF, double* __restrict__ part) {
+    FMD_PDL_WAIT();
     __shared__ double sm[32];
     double acc[1] = {0.0};
     const double k = 2.0 * wF / (3.0 * na);
@@ -46,6 +48,7 @@ k_sg_lambda(const double* __restrict__ F, const double* __restrict__ Fref, int n
 __global__ void k_sg_loss(const double* __restrict__ sc, const double* __restrict__ ref,
                           const double* __restrict__ sumdf2, int na, double wE, double wF, double wW,
                           double* __restrict__ lam, double* __restrict__ loss_acc) {
+    FMD_PDL_WAIT();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const double n2 = (double)na * na;
     const double dE = sc[0] - ref[0];
@@ -67,6 +70,7 @@ k_sg_adjoint(const double* __restrict__ pos, const double* __restrict__ hh, cons
              const int* __restrict__ row_i, const int* __restrict__ row_s, const float* __restrict__ vec,
              const double* __restrict__ lamF, const double* __restrict__ lam, int r_cap,
              float* __restrict__ beta, uint16_t* __restrict__ U) {
+    FMD_PDL_WAIT();
     double h[9], hi[9];
     load_cell(hh, h, hi);
     const int R = aoff[na];
@@ -258,6 +262,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 k_sg_chain(const uint16_t* __restrict__ img, const float* __restrict__ vec, const int* __restrict__ nrows,
            const uint16_t* __restrict__ X, const uint16_t* __restrict__ Ut, const float* __restrict__ beta,
            OperandTiles out, float* __restrict__ dw4_glob, int* __restrict__ err) {
+    FMD_PDL_WAIT();
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ uint64_t mbar;
     __shared__ uint32_t tbase;
@@ -466,6 +471,7 @@ __device__ __forceinline__ void red_add4(float* p, const float* v) {
 __global__ void __launch_bounds__(kGThreads, 1)
 k_sg_wgrad(const int* __restrict__ nrows, const uint16_t* __restrict__ X, const uint16_t* __restrict__ Ut,
            OperandTiles in, float* __restrict__ grad, int* __restrict__ err) {
+    FMD_PDL_WAIT();
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ uint64_t full[kGStages], empty[kGStages], fin;
     __shared__ uint32_t tbase;
@@ -672,16 +678,24 @@ cudaError_t accumulate_grad(Work& w, TrainWork& tw, const uint16_t* img, const f
     if (e == cudaSuccess) e = rebo_forces(w, img, vec, pos, hh, cnt, list, cap, na, F, w.part, st);
     if (e == cudaSuccess) e = reduce_partials(w.part, kRowBlocks, kNV, tw.sc, st);           // sc[0..9] = E, W
     if (e != cudaSuccess) return e;
-    k_sg_lambda<<<kRowBlocks, 256, 0, st>>>(F, Fref, na, wF, tw.lamF, tw.part);
+    if ((e = launch_pdl(k_sg_lambda, dim3(kRowBlocks), dim3(256), 0, st, F, Fref, na, wF, tw.lamF,
+                        tw.part)) != cudaSuccess)
+        return e;
     e = reduce_partials(tw.part, kRowBlocks, 1, tw.sc + 10, st);                              // sc[10] = sum dF^2
     if (e != cudaSuccess) return e;
-    k_sg_loss<<<1, 32, 0, st>>>(tw.sc, ref10, tw.sc + 10, na, wE, wF, wW, tw.sc + 12, loss_acc);   // sc[12..21] = lambdas
-    k_sg_adjoint<<<kRowBlocks, 128, 0, st>>>(pos, hh, cnt, list, cap, na, w.aoff, w.row_i, w.row_s, vec, tw.lamF,
-                                             tw.sc + 12, w.r_cap, tw.beta, tw.U);
+    if ((e = launch_pdl(k_sg_loss, dim3(1), dim3(32), 0, st, tw.sc, ref10, tw.sc + 10, na, wE, wF, wW, tw.sc + 12,
+                        loss_acc)) != cudaSuccess)
+        return e;   // sc[12..21] = lambdas
+    if ((e = launch_pdl(k_sg_adjoint, dim3(kRowBlocks), dim3(128), 0, st, pos, hh, cnt, list, cap, na, w.aoff,
+                        w.row_i, w.row_s, vec, tw.lamF, tw.sc + 12, w.r_cap, tw.beta, tw.U)) != cudaSuccess)
+        return e;
     const int* nrows = w.aoff + w.na_used;
-    k_sg_chain<<<kSMs, kThreads, C_TOTAL, st>>>(img, vec, nrows, w.X, tw.U, tw.beta, tw.t,
-                                                grad + H * D + 2 * H * H, w.err);
-    k_sg_wgrad<<<kSMs, kGThreads, G_TOTAL, st>>>(nrows, w.X, tw.U, tw.t, grad, w.err);
+    if ((e = launch_pdl(k_sg_chain, dim3(kSMs), dim3(kThreads), C_TOTAL, st, img, vec, nrows, w.X, tw.U, tw.beta,
+                        tw.t, grad + H * D + 2 * H * H, w.err)) != cudaSuccess)
+        return e;
+    if ((e = launch_pdl(k_sg_wgrad, dim3(kSMs), dim3(kGThreads), G_TOTAL, st, nrows, w.X, tw.U, tw.t, grad,
+                        w.err)) != cudaSuccess)
+        return e;
     return cudaGetLastError();
 }
 

@@ -18,6 +18,7 @@
 #include <cuda_bf16.h>
 
 #include "kernels.h"
+#include "pdl.cuh"
 #include "rebo_fn.cuh"
 #include "sg_dev.cuh"
 #include "surrogate.cuh"
@@ -38,6 +39,7 @@ __global__ void __launch_bounds__(kScanBlock)
 k_sg_count(const double* __restrict__ pos, const double* __restrict__ hh, const int* __restrict__ cnt,
            const int* __restrict__ list, int cap, int na, int* __restrict__ acnt, const int* __restrict__ gate,
            int* __restrict__ aoff, int* __restrict__ bsum) {
+    FMD_PDL_WAIT();
     __shared__ int wsum[kScanBlock / 32];
     double h[9], hi[9];
     load_cell(hh, h, hi);
@@ -73,6 +75,7 @@ k_sg_count(const double* __restrict__ pos, const double* __restrict__ hh, const 
 
 // Exclusive scan of acnt[0..na) into aoff[0..na]; one block of 1024 threads.
 __global__ void __launch_bounds__(1024) k_sg_scan(const int* __restrict__ acnt, int na, int* __restrict__ aoff) {
+    FMD_PDL_WAIT();
     __shared__ int sm[1024];
     const int per = (na + 1023) / 1024;
     const int b0 = min((int)threadIdx.x * per, na), b1 = min(b0 + per, na);
@@ -98,6 +101,7 @@ __global__ void k_sg_rows(const double* __restrict__ pos, const double* __restri
                           const int* __restrict__ cnt, const int* __restrict__ list, int cap, int na,
                           int* __restrict__ aoff, int* __restrict__ row_i, int* __restrict__ row_s,
                           int* __restrict__ rowid, const int* __restrict__ gate, const int* __restrict__ boff) {
+    FMD_PDL_WAIT();
     // global offsets: block-local offset + the block's scanned total
     const int i = blockIdx.x * kScanBlock + threadIdx.x;
     const int nblk = (na + kScanBlock - 1) / kScanBlock;
@@ -132,6 +136,7 @@ __global__ void k_sg_desc(const double* __restrict__ pos, const double* __restri
                           const int* __restrict__ aoff, const int* __restrict__ row_i,
                           const int* __restrict__ row_s, const int* __restrict__ rowid, const float* __restrict__ vec,
                           int r_cap, uint16_t* __restrict__ X, int* __restrict__ partner, int* __restrict__ err) {
+    FMD_PDL_WAIT();
     double h[9], hi[9];
     load_cell(hh, h, hi);
     const int R = aoff[na];
@@ -262,6 +267,7 @@ __device__ __forceinline__ void epi_bwd(uint32_t ta, uint32_t td, unsigned char*
 __global__ void __launch_bounds__(kMlpThreads, 1)
 k_sg_mlp(const uint16_t* __restrict__ img, const float* __restrict__ vec, const int* __restrict__ nrows,
          const uint16_t* __restrict__ X, float* __restrict__ bout, float* __restrict__ gxout, int* __restrict__ err) {
+    FMD_PDL_WAIT();
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ uint64_t mbar;
     __shared__ uint32_t tbase;
@@ -416,6 +422,7 @@ k_sg_force(const double* __restrict__ pos, const double* __restrict__ hh, const 
            const int* __restrict__ row_i, const int* __restrict__ row_s, const int* __restrict__ partner,
            const float* __restrict__ b, const float* __restrict__ gx, const float* __restrict__ vec,
            double* __restrict__ F, double* __restrict__ part) {
+    FMD_PDL_WAIT();
     __shared__ double smr[32 * kNV];
     double h[9], hi[9];
     load_cell(hh, h, hi);
@@ -591,30 +598,42 @@ cudaError_t build_rows(Work& w, const float* vec, const double* pos, const doubl
     if (na > w.na_cap || cap != w.cap) return cudaErrorInvalidValue;
     w.na_used = na;
     const int nb = (na + kScanBlock - 1) / kScanBlock;
-    k_sg_count<<<nb, kScanBlock, 0, st>>>(pos, hh, cnt, list, cap, na, w.acnt, gate, w.aoff, w.bsum);
-    k_sg_scan<<<1, 1024, 0, st>>>(w.bsum, nb, w.boff);
-    k_sg_rows<<<nb, kScanBlock, 0, st>>>(pos, hh, cnt, list, cap, na, w.aoff, w.row_i, w.row_s, w.rowid, gate, w.boff);
-    k_sg_desc<<<kRowBlocks, 128, 0, st>>>(pos, hh, cnt, list, cap, na, w.aoff, w.row_i, w.row_s, w.rowid, vec,
-                                          w.r_cap, w.X, w.partner, w.err);
+    cudaError_t e;
+    if ((e = launch_pdl(k_sg_count, dim3(nb), dim3(kScanBlock), 0, st, pos, hh, cnt, list, cap, na, w.acnt, gate,
+                        w.aoff, w.bsum)) != cudaSuccess)
+        return e;
+    if ((e = launch_pdl(k_sg_scan, dim3(1), dim3(1024), 0, st, w.bsum, nb, w.boff)) != cudaSuccess)
+        return e;
+    if ((e = launch_pdl(k_sg_rows, dim3(nb), dim3(kScanBlock), 0, st, pos, hh, cnt, list, cap, na, w.aoff, w.row_i,
+                        w.row_s, w.rowid, gate, w.boff)) != cudaSuccess)
+        return e;
+    if ((e = launch_pdl(k_sg_desc, dim3(kRowBlocks), dim3(128), 0, st, pos, hh, cnt, list, cap, na, w.aoff, w.row_i,
+                        w.row_s, w.rowid, vec, w.r_cap, w.X, w.partner, w.err)) != cudaSuccess)
+        return e;
     return cudaGetLastError();
 }
 
 cudaError_t run_mlp(Work& w, const uint16_t* img, const float* vec, cudaStream_t st) {
     static bool attr = false;
+    cudaError_t e;
     if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_sg_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_TOTAL);
+        e = cudaFuncSetAttribute(k_sg_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_TOTAL);
         if (e != cudaSuccess) return e;
         attr = true;
     }
     // the row count stays on the device (aoff[na] of the last build)
-    k_sg_mlp<<<kSMs, kMlpThreads, SM_TOTAL, st>>>(img, vec, w.aoff + w.na_used, w.X, w.b, w.gx, w.err);
+    if ((e = launch_pdl(k_sg_mlp, dim3(kSMs), dim3(kMlpThreads), SM_TOTAL, st, img, vec, w.aoff + w.na_used, w.X,
+                        w.b, w.gx, w.err)) != cudaSuccess)
+        return e;
     return cudaGetLastError();
 }
 
 cudaError_t assemble(Work& w, const float* vec, const double* pos, const double* hh, const int* cnt,
                      const int* list, int cap, int na, double* F, double* part, cudaStream_t st) {
-    k_sg_force<<<kRowBlocks, 256, 0, st>>>(pos, hh, cnt, list, cap, na, w.aoff, w.row_i, w.row_s, w.partner, w.b,
-                                           w.gx, vec, F, part);
+    cudaError_t e;
+    if ((e = launch_pdl(k_sg_force, dim3(kRowBlocks), dim3(256), 0, st, pos, hh, cnt, list, cap, na, w.aoff, w.row_i,
+                        w.row_s, w.partner, w.b, w.gx, vec, F, part)) != cudaSuccess)
+        return e;
     return cudaGetLastError();
 }
 
