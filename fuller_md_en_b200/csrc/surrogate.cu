@@ -196,19 +196,22 @@ __global__ void k_sg_desc(const double* __restrict__ pos, const double* __restri
 }
 
 // ------------------------------------------------------------------ network
-// 16 warps: four per TMEM lane quadrant, each owning 32 of the 128 columns,
-// so the epilogues (TMEM -> SiLU -> BF16 tile) run on 512 threads.  Bound by
-// the serial chain of six GEMMs and epilogues of a tile; 368,640 rows: 170 us
-// (214 us with two BF16 conversions and four selections per pair of values).
-constexpr int kMlpThreads = 512;
+// Two CTAs of 8 warps per SM, so that one's tensor work and hand-offs overlap
+// the other's epilogues; each has two warps per TMEM lane quadrant (64 of the 128
+// columns a thread), 108 KB of shared memory and 256 TMEM columns: z1 and then
+// SiLU'(z1) in one half, every other accumulator in the second, SiLU'(z2) in
+// registers.  368,640 rows 145 us, 90,000 rows 45; one CTA of 16 warps, all
+// accumulators in TMEM: 170 and 48 us.
+constexpr int kMlpThreads = 256;
 constexpr int kColGroups = kMlpThreads / 128;      // column groups per row
-constexpr int kColsPerThread = H / kColGroups;      // 32
-// dynamic shared memory map (bytes)
-constexpr int SM_W1 = 0, SM_W2 = SM_W1 + H * D * 2, SM_W3 = SM_W2 + H * H * 2, SM_X = SM_W3 + H * H * 2,
-              SM_ACT = SM_X + TILE * D * 2, SM_W4 = SM_ACT + TILE * H * 2, SM_RED = SM_W4 + H * 4,
-              SM_TOTAL = SM_RED + kColGroups * TILE * 4;
+constexpr int kColsPerThread = H / kColGroups;      // 64
+constexpr int kSumCols = 32;                        // columns of a partial sum of the output layer
+// dynamic shared memory map (bytes); the descriptor tile lies where the
+// activations follow
+constexpr int SM_W1 = 0, SM_W2 = SM_W1 + H * D * 2, SM_W3 = SM_W2 + H * H * 2, SM_ACT = SM_W3 + H * H * 2,
+              SM_W4 = SM_ACT + TILE * H * 2, SM_RED = SM_W4 + H * 4, SM_TOTAL = SM_RED + H / kSumCols * TILE * 4;
 // TMEM columns
-constexpr uint32_t TM_Z1 = 0, TM_Z2 = 128, TM_Z3 = 256, TM_T = 384;
+constexpr uint32_t TM_Z1 = 0, TM_T = 128, TM_COLS = 256;
 
 // Forward epilogue of one hidden layer: each thread owns row q and
 // kColsPerThread columns from c0 of z (TMEM at ta).  Writes h = SiLU(z) as
@@ -241,14 +244,43 @@ __device__ __forceinline__ void epi_fwd(uint32_t ta, unsigned char* act, int q, 
     umma::tmem_wait_st();
 }
 
+// The same, SiLU'(z) to registers.
+__device__ __forceinline__ void epi_fwd_keep(uint32_t ta, unsigned char* act, int q, int c0, float* d) {
+#pragma unroll
+    for (int cc = 0; cc < kColsPerThread; cc += 16) {
+        float z[16];
+        umma::tmem_ld16(ta + c0 + cc, z);
+#pragma unroll
+        for (int e = 0; e < 16; e++) {
+            const float s = sigm(z[e]);
+            d[cc + e] = dsilu(z[e], s);
+            z[e] *= s;
+        }
+        if (c0 + cc + 16 == H) z[15] = 1.f;
+        st_tile16(act, q, c0 + cc, z);
+    }
+}
+
+// Gradient epilogue with SiLU'(z) in registers.
+__device__ __forceinline__ void epi_bwd_keep(uint32_t ta, const float* d, unsigned char* act, int q, int c0) {
+#pragma unroll
+    for (int cc = 0; cc < kColsPerThread; cc += 16) {
+        float v[16];
+        umma::tmem_ld16(ta + c0 + cc, v);
+#pragma unroll
+        for (int e = 0; e < 16; e++) v[e] *= d[cc + e];
+        if (c0 + cc + 16 == H) v[15] = 0.f;
+        st_tile16(act, q, c0 + cc, v);
+    }
+}
+
 // Gradient epilogue: g = t * SiLU'(z) from the t accumulator (ta) and the
 // SiLU'(z) the forward epilogue left at td; column 127 held at 0.
 __device__ __forceinline__ void epi_bwd(uint32_t ta, uint32_t td, unsigned char* act, int q, int c0) {
 #pragma unroll 1
     for (int cc = 0; cc < kColsPerThread; cc += 16) {
         float v[16], d[16];
-        umma::tmem_ld16(ta + c0 + cc, v);
-        umma::tmem_ld16(td + c0 + cc, d);
+        umma::tmem_ld16x2(ta + c0 + cc, td + c0 + cc, v, d);
 #pragma unroll
         for (int e = 0; e < 16; e++) v[e] *= d[e];
         if (c0 + cc + 16 == H) v[15] = 0.f;
@@ -264,7 +296,7 @@ __device__ __forceinline__ void epi_bwd(uint32_t ta, uint32_t td, unsigned char*
     }
 }
 
-__global__ void __launch_bounds__(kMlpThreads, 1)
+__global__ void __launch_bounds__(kMlpThreads, 2)
 k_sg_mlp(const uint16_t* __restrict__ img, const float* __restrict__ vec, const int* __restrict__ nrows,
          const uint16_t* __restrict__ X, float* __restrict__ bout, float* __restrict__ gxout, int* __restrict__ err) {
     FMD_PDL_WAIT();
@@ -287,7 +319,7 @@ k_sg_mlp(const uint16_t* __restrict__ img, const float* __restrict__ vec, const 
         for (int e = t; e < H; e += kMlpThreads) w4[e] = vec[V_W4 + e];
     }
     if (w == 0) {
-        umma::tmem_alloc(&tbase, 512);
+        umma::tmem_alloc(&tbase, TM_COLS);
         umma::tmem_relinquish();
     }
     if (t == 0) umma::mbar_init(&mbar, 1);
@@ -295,8 +327,7 @@ k_sg_mlp(const uint16_t* __restrict__ img, const float* __restrict__ vec, const 
     const uint32_t tm = tbase;
     const uint32_t tl = tm + ((uint32_t)(32 * (w & 3)) << 16);   // this warp's TMEM lanes
     const uint32_t sW1 = umma::smem_u32(sm + SM_W1), sW2 = umma::smem_u32(sm + SM_W2),
-                   sW3 = umma::smem_u32(sm + SM_W3), sX = umma::smem_u32(sm + SM_X),
-                   sA = umma::smem_u32(sm + SM_ACT);
+                   sW3 = umma::smem_u32(sm + SM_W3), sA = umma::smem_u32(sm + SM_ACT);
     unsigned char* act = sm + SM_ACT;
     const float* w4 = reinterpret_cast<const float*>(sm + SM_W4);
     float* red = reinterpret_cast<float*>(sm + SM_RED);
@@ -304,10 +335,15 @@ k_sg_mlp(const uint16_t* __restrict__ img, const float* __restrict__ vec, const 
     uint32_t ph = 0;
     bool ok = true;
 
-    // The descriptor tile of the next 128 rows: 8 KB, one 16-byte piece per
-    // thread, loaded into a register while the current tile is computed.
-    static_assert(TILE * D * 2 / 16 == kMlpThreads, "one 16-byte piece of the descriptor tile per thread");
-    uint4 xnext = reinterpret_cast<const uint4*>(X + (size_t)blockIdx.x * TILE * D)[t];
+    // The descriptor tile of 128 rows, 8 KB in the operand layout already: two
+    // 16-byte pieces per thread, the next tile's loaded behind the last GEMM.
+    static_assert(TILE * D * 2 / 16 == 2 * kMlpThreads, "two 16-byte pieces of the descriptor tile per thread");
+    uint4* xs = reinterpret_cast<uint4*>(act);
+    {
+        const uint4* x = reinterpret_cast<const uint4*>(X + (size_t)blockIdx.x * TILE * D);
+        xs[t] = x[t];
+        xs[t + kMlpThreads] = x[t + kMlpThreads];
+    }
 
     // Wait for the MMAs of this step, then (after the epilogue) hand the new
     // operand tile to the issuing thread; a wait that ran out ends every
@@ -326,26 +362,25 @@ k_sg_mlp(const uint16_t* __restrict__ img, const float* __restrict__ vec, const 
     } while (0)
 
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        reinterpret_cast<uint4*>(sm + SM_X)[t] = xnext;                // operand layout already
+        float d2[kColsPerThread];                                     // SiLU'(z2)
         SG_HANDOFF();
-        if (t == 0) issue(tm + TM_Z1, sX, D, false, sW1, D, false, H, D / 16, &mbar);
+        if (t == 0) issue(tm + TM_Z1, sA, D, false, sW1, D, false, H, D / 16, &mbar);
         SG_WAIT();
-        if (tile + (int)gridDim.x < ntiles)                           // X is free once z1 is done
-            xnext = reinterpret_cast<const uint4*>(X + (size_t)(tile + gridDim.x) * TILE * D)[t];
         epi_fwd(tl + TM_Z1, act, q, c0);                              // h1, SiLU'(z1) -> TM_Z1
         SG_HANDOFF();
-        if (t == 0) issue(tm + TM_Z2, sA, H, false, sW2, H, false, H, H / 16, &mbar);
+        if (t == 0) issue(tm + TM_T, sA, H, false, sW2, H, false, H, H / 16, &mbar);
         SG_WAIT();
-        epi_fwd(tl + TM_Z2, act, q, c0);                              // h2, SiLU'(z2) -> TM_Z2
+        epi_fwd_keep(tl + TM_T, act, q, c0, d2);                      // h2
         SG_HANDOFF();
-        if (t == 0) issue(tm + TM_Z3, sA, H, false, sW3, H, false, H, H / 16, &mbar);
+        if (t == 0) issue(tm + TM_T, sA, H, false, sW3, H, false, H, H / 16, &mbar);
         SG_WAIT();
         {   // output layer and g3 = bs * w4 * SiLU'(z3)
-            float y = 0.f;
+            float y = 0.f;                                            // sums of kSumCols columns
 #pragma unroll 1
             for (int cc = 0; cc < kColsPerThread; cc += 16) {
+                if (cc % kSumCols == 0) y = 0.f;
                 float z[16];
-                umma::tmem_ld16(tl + TM_Z3 + c0 + cc, z);
+                umma::tmem_ld16(tl + TM_T + c0 + cc, z);
                 float g[16];
 #pragma unroll
                 for (int e = 0; e < 16; e++) {
@@ -364,8 +399,8 @@ k_sg_mlp(const uint16_t* __restrict__ img, const float* __restrict__ vec, const 
                     o.w = umma::pack_bf16(g[8 * h8 + 6], g[8 * h8 + 7]);
                     *reinterpret_cast<uint4*>(act + umma::il_off(q, c0 + cc + 8 * h8, H)) = o;
                 }
+                if (cc % kSumCols == kSumCols - 16) red[(c0 + cc) / kSumCols * TILE + q] = y;
             }
-            red[(w >> 2) * TILE + q] = y;
         }
         SG_HANDOFF();
         {
@@ -373,20 +408,28 @@ k_sg_mlp(const uint16_t* __restrict__ img, const float* __restrict__ vec, const 
             if (c0 == 0 && row < R) {
                 float y = 0.f;
 #pragma unroll
-                for (int g = 0; g < kColGroups; g++) y += red[g * TILE + q];
+                for (int g = 0; g < H / kSumCols; g++) y += red[g * TILE + q];
                 bout[row] = b0 + bs * y;
             }
         }
         if (t == 0) issue(tm + TM_T, sA, H, false, sW3, H, true, H, H / 16, &mbar);   // t2 = g3 W3^T
         SG_WAIT();
-        epi_bwd(tl + TM_T, tl + TM_Z2, act, q, c0);                   // g2
+        epi_bwd_keep(tl + TM_T, d2, act, q, c0);                      // g2
         SG_HANDOFF();
         if (t == 0) issue(tm + TM_T, sA, H, false, sW2, H, true, H, H / 16, &mbar);   // t1 = g2 W2^T
         SG_WAIT();
         epi_bwd(tl + TM_T, tl + TM_Z1, act, q, c0);                   // g1
         SG_HANDOFF();
         if (t == 0) issue(tm + TM_T, sA, H, false, sW1, D, true, D, H / 16, &mbar);   // gx = g1 W1^T
+        const bool more = tile + (int)gridDim.x < ntiles;
+        uint4 xn[2];
+        if (more) {
+            const uint4* x = reinterpret_cast<const uint4*>(X + (size_t)(tile + gridDim.x) * TILE * D);
+            xn[0] = x[t];
+            xn[1] = x[t + kMlpThreads];
+        }
         SG_WAIT();
+        if (more) { xs[t] = xn[0]; xs[t + kMlpThreads] = xn[1]; }     // the activations are done with
         if ((w >> 2) < D / 16) {                // gx has D = 32 columns: two groups of 16
             const int row = tile * TILE + q;
             const int cg = 16 * (w >> 2);
@@ -410,7 +453,7 @@ done:
     }
     umma::fence_before();
     __syncthreads();
-    if (w == 0) umma::tmem_dealloc(tm, 512);
+    if (w == 0) umma::tmem_dealloc(tm, TM_COLS);
 #undef SG_WAIT
 #undef SG_HANDOFF
 }
@@ -622,7 +665,7 @@ cudaError_t run_mlp(Work& w, const uint16_t* img, const float* vec, cudaStream_t
         attr = true;
     }
     // the row count stays on the device (aoff[na] of the last build)
-    if ((e = launch_pdl(k_sg_mlp, dim3(kSMs), dim3(kMlpThreads), SM_TOTAL, st, img, vec, w.aoff + w.na_used, w.X,
+    if ((e = launch_pdl(k_sg_mlp, dim3(2 * kSMs), dim3(kMlpThreads), SM_TOTAL, st, img, vec, w.aoff + w.na_used, w.X,
                         w.b, w.gx, w.err)) != cudaSuccess)
         return e;
     return cudaGetLastError();
