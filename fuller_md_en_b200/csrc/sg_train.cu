@@ -160,12 +160,11 @@ k_sg_adjoint(const double* __restrict__ pos, const double* __restrict__ hh, cons
 // 16 warps: four per TMEM lane quadrant, each owning 32 of the 128 columns.
 // The sigmoid of z1 and z2 is evaluated twice per element: in the forward
 // pass, and where SiLU' and SiLU'' are first needed together; there SiLU'(z)
-// replaces z in TMEM for the later stages.  A thread keeps its row's part of
-// dL/dw4 for its columns in registers through all tiles.  The kernel is bound
-// by the serial chain of ten GEMMs and epilogues of a tile (22 us; its special
-// functions alone, six sigmoids an element, take 7).  90,000 rows: 107 us; 243
-// us with 8 warps, ten sigmoids an element, and dL/dw4 reduced over the rows
-// in every tile.
+// replaces z in TMEM for the later stages.  The kernel is bound
+// by the serial chain of ten GEMMs and epilogues of a tile (21 us; its special
+// functions alone, six sigmoids an element, take 7).  90,000 rows: 102 us; 243
+// us with 8 warps, ten sigmoids an element and 160 shuffles per 32 columns of
+// dL/dw4.
 constexpr int kThreads = 512;
 constexpr int kCols = TILE * H / kThreads;   // columns per thread
 static_assert(kCols == 32, "two slices of 16 columns per thread");
@@ -184,6 +183,22 @@ struct ChainThread {
     uint32_t tl;
     int q, c0;
 };
+
+// Sums 32 columns over the warp's rows (one per lane) and adds column k's to
+// acc[k]: each exchange hands half of the columns over, so lane l ends with
+// column l (31 shuffles instead of 160).
+__device__ __forceinline__ void add_columns(float (&v)[kCols], float* acc, int lane) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool hi = lane & o;
+#pragma unroll
+        for (int k = 0; k < o; k++) {
+            const float send = hi ? v[k] : v[k + o];
+            v[k] = (hi ? v[k + o] : v[k]) + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    atomicAdd(&acc[lane], v[0]);
+}
 
 // h = SiLU(z) (column 127: 1) to the operand tile and to out.
 __device__ __forceinline__ void chain_forward(const ChainThread& c, uint32_t tz, unsigned char* act, unsigned char* out) {
@@ -293,9 +308,8 @@ k_sg_chain(const uint16_t* __restrict__ img, const float* __restrict__ vec, cons
     unsigned char* E2 = sm + C_E2;
     const float* w4 = reinterpret_cast<const float*>(sm + C_W4);
     const float bs = vec[V_BS];
-    float dw[kCols];                       // dL/dw4 of this row so far
-#pragma unroll
-    for (int k = 0; k < kCols; k++) dw[k] = 0.f;
+    float* dw4 = reinterpret_cast<float*>(sm + C_DW4);
+    float dw[kCols];                       // a stage's part of dL/dw4, this row
     uint32_t ph = 0;
     bool ok = true;
 
@@ -352,12 +366,13 @@ k_sg_chain(const uint16_t* __restrict__ img, const float* __restrict__ vec, cons
             for (int e = 0; e < 16; e++) {
                 const bool last = e == 15 && cc + 16 == H;
                 const float s = sigm(z[e]);
-                dw[k + e] += ybar * (last ? 1.f : z[e] * s);
+                dw[k + e] = ybar * (last ? 1.f : z[e] * s);
                 z[e] = last ? 0.f : bs * w4[cc + e] * dsilu(z[e], s);
             }
             st_tile16(act, c.q, cc, z);
             st_tile16(gtile(out.g3, tile), c.q, cc, z);
         }
+        add_columns(dw, dw4 + c.c0, lane);
         // ---- gradient network
         SG_HANDOFF();
         if (t == 0) issue(tm + T_T, sA, H, false, sW3, H, true, H, H / 16, &mbar);        // t2 = g3 W3^T
@@ -388,12 +403,13 @@ k_sg_chain(const uint16_t* __restrict__ img, const float* __restrict__ vec, cons
             for (int e = 0; e < 16; e++) {
                 const bool last = e == 15 && cc + 16 == H;
                 const float s = sigm(z[e]), d = dsilu(z[e], s);
-                dw[k + e] += last ? 0.f : bs * gb[e] * d;
+                dw[k + e] = last ? 0.f : bs * gb[e] * d;
                 z[e] = last ? 0.f : gb[e] * bs * w4[cc + e] * d2silu(z[e], s) + ybar * w4[cc + e] * d;
             }
             st_tile16(act, c.q, cc, z);
             st_tile16(gtile(out.z3, tile), c.q, cc, z);
         }
+        add_columns(dw, dw4 + c.c0, lane);
         // ---- adjoint of the forward network
         SG_HANDOFF();
         if (t == 0) issue(tm + T_T, sA, H, false, sW3, H, true, H, H / 16, &mbar);        // hb2 = zb3 W3^T
@@ -413,20 +429,10 @@ done:
         // chance to land before TMEM is released
         umma::mbar_wait(&mbar, ph);
     }
-    {   // rows of a warp, then of the block
-        float* dw4 = reinterpret_cast<float*>(sm + C_DW4);
-#pragma unroll
-        for (int k = 0; k < kCols; k++) {
-            float x = dw[k];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-            if (lane == 0) atomicAdd(&dw4[c.c0 + k], x);
-        }
-        umma::fence_before();
-        __syncthreads();
-        if (ok)
-            for (int e = t; e < H; e += kThreads) atomicAdd(&dw4_glob[e], dw4[e]);
-    }
+    umma::fence_before();
+    __syncthreads();
+    if (ok)
+        for (int e = t; e < H; e += kThreads) atomicAdd(&dw4_glob[e], dw4[e]);
     if (w == 0) umma::tmem_dealloc(tm, 512);
 #undef SG_WAIT
 #undef SG_HANDOFF
@@ -438,9 +444,9 @@ done:
 // dW3^T = z3^T h2 + g3^T tb2), summed in TMEM over the CTA's tiles.  One
 // thread copies the pairs into a ring of stages, one issues the MMAs as they
 // arrive.  It is bound by the reading of the operand tiles (336 KB a tile).
-// Tiles are taken from the last back: the chain's newest are still in L2.
-// 90,000 rows: 49 us, 225 MB (34 us from memory); 160 us with loads by all
-// threads, then MMAs, in turn.
+// 90,000 rows: 58 us, 225 MB (34 us from memory); 160 us with loads by all
+// threads, then MMAs, in turn.  From the last tile back, with the chain's newest
+// still in L2, it takes 49 us, but the sums would be added in another order.
 constexpr int kGThreads = 256, kGStages = 3;
 constexpr int G_A = 0, G_B = TILE * H * 2, G_STAGE = 2 * TILE * H * 2, G_TOTAL = kGStages * G_STAGE;
 constexpr uint32_t T_D1 = 0, T_D2 = 128, T_D3 = 256;
@@ -495,7 +501,7 @@ k_sg_wgrad(const int* __restrict__ nrows, const uint16_t* __restrict__ X, const 
     if (t == 0) {                          // copies
         int it = 0;
         for (; it < steps; it++) {
-            const int s = it % kGStages, tile = (int)blockIdx.x + (mine - 1 - it / 6) * (int)gridDim.x;
+            const int s = it % kGStages, tile = (int)blockIdx.x + it / 6 * (int)gridDim.x;
             if (it >= kGStages && !umma::mbar_wait(&empty[s], (uint32_t)(it / kGStages - 1) & 1u)) { bad = 1; break; }
             const GradPair p = grad_pair(in, X, Ut, it % 6);
             const uint32_t base = umma::smem_u32(sm) + s * G_STAGE, bb = TILE * p.bcols * 2;
