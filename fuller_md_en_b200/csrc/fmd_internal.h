@@ -5,7 +5,6 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
-#include <map>
 #include <string>
 #include <vector>
 
@@ -71,24 +70,32 @@ struct fmd_ctx {
     // Device blocks released by systems of this context, by size: the next
     // system of the same size takes them instead of mapping fresh memory
     // (cudaMalloc of a few hundred MB costs milliseconds and varies with the
-    // process's allocation history).  At most kCacheMax bytes; given back when
-    // an allocation fails, and with the context.
-    static constexpr size_t kCacheMax = (size_t)16 << 30;
-    std::multimap<size_t, void*> mem_cache;
+    // process's allocation history).  At most kCacheMax bytes, the longest
+    // unused given back first; all of them when an allocation fails, and with
+    // the context.
+    static constexpr size_t kCacheMax = (size_t)64 << 30;
+    struct Cached {
+        size_t bytes;
+        void* p;
+    };
+    std::vector<Cached> mem_cache;           // by time of release
     size_t cached = 0;
-    void drop_cache() {
-        for (auto& b : mem_cache) cudaFree(b.second);
-        mem_cache.clear();
-        cached = 0;
+    void drop_cache(size_t keep = 0) {
+        size_t n = 0;
+        for (; n < mem_cache.size() && cached > keep; n++) {
+            cudaFree(mem_cache[n].p);
+            cached -= mem_cache[n].bytes;
+        }
+        mem_cache.erase(mem_cache.begin(), mem_cache.begin() + n);
     }
     cudaError_t dev_alloc(void** p, size_t bytes) {
-        auto it = mem_cache.find(bytes);
-        if (it != mem_cache.end()) {
-            *p = it->second;
-            mem_cache.erase(it);
-            cached -= bytes;
-            return cudaSuccess;
-        }
+        for (size_t k = mem_cache.size(); k-- > 0;)
+            if (mem_cache[k].bytes == bytes) {
+                *p = mem_cache[k].p;
+                cached -= bytes;
+                mem_cache.erase(mem_cache.begin() + k);
+                return cudaSuccess;
+            }
         cudaError_t e = cudaMalloc(p, bytes);
         if (e == cudaErrorMemoryAllocation && !mem_cache.empty()) {
             cudaGetLastError();
@@ -100,11 +107,12 @@ struct fmd_ctx {
     // The caller has synchronised every stream that used the block.
     void dev_release(void* p, size_t bytes) {
         if (!p) return;
-        if (bytes > kCacheMax - std::min(cached, kCacheMax)) {
+        if (bytes > kCacheMax) {
             cudaFree(p);
             return;
         }
-        mem_cache.emplace(bytes, p);
+        drop_cache(kCacheMax - bytes);
+        mem_cache.push_back({bytes, p});
         cached += bytes;
     }
 

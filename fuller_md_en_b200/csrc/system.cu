@@ -171,10 +171,11 @@ int System::alloc_prune(double rc_lj) {
     const int n = arr.n;
     LJPrune q;
     if (alloc(&q.cnt, n, (const int*)nullptr) || alloc(&q.list, (size_t)n * arr.in_cap, (const int*)nullptr) ||
-        alloc(&q.sb, 3 * (size_t)n, (const double*)nullptr) || alloc(&q.hb, 9, (const double*)nullptr) ||
-        alloc(&q.words, 2, (const unsigned long long*)nullptr) ||
-        alloc(&q.stats, 2, (const unsigned long long*)nullptr))
+        alloc(&q.sb, 3 * (size_t)n, (const double*)nullptr) ||
+        alloc(&q.words, 4 + 9, (const unsigned long long*)nullptr))
         return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
+    q.stats = q.words + 2;
+    q.hb = reinterpret_cast<double*>(q.words + 4);
     q.n = n;
     q.stride = arr.in_cap;
     q.rc = rc_lj;
@@ -215,10 +216,12 @@ int System::alloc_clus(const double* pos_h) {
             x[3 * a + c] = L > 0.0 ? d - L * std::rint(d / L) : d;
         }
     const std::vector<int> perm = lj_clus_assign(x.data(), q.S);
-    int* dp;
-    if (alloc(&dp, perm.size(), (const int*)nullptr) || alloc(&q.cnt, q.nclus, (const int4*)nullptr) ||
-        alloc(&q.upos, 3 * (size_t)arr.n, (const double*)nullptr))
+    // one block: rows' ends, followed positions, clusters
+    const size_t perm4 = (perm.size() + 3) / 4, upos4 = (3 * (size_t)arr.n + 1) / 2;
+    if (alloc(&q.cnt, q.nclus + upos4 + perm4, (const int4*)nullptr))
         return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
+    q.upos = reinterpret_cast<double*>(q.cnt + q.nclus);
+    int* dp = reinterpret_cast<int*>(q.cnt + q.nclus + upos4);
     if (cudaMemcpyAsync(dp, perm.data(), sizeof(int) * perm.size(), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
         return ctx->fail(FMD_ERR_CUDA, "cluster table copy failed");
     q.perm = dp;
