@@ -237,11 +237,15 @@ int System::alloc_clus(const double* pos_h) {
 // The step's LJ term walks cluster rows when the tables exist, pruning is on,
 // no launch shape of the row gather is pinned and the initial cell takes them
 // (lj_clus_mode; a cell that stops doing so walks the full rows).
+// The margin keeps out small cells that may shrink to the limit; those are also
+// the ones (2 x 2 x 2 BCC) whose crystal comes apart within some thousand steps,
+// and in a gas of 1e18 K, which needs new rows on every evaluation, the row
+// gather takes 12 us where building cluster rows takes 35.
 void System::set_clus(bool allowed) {
     const bool diag = h0[1] == 0.0 && h0[2] == 0.0 && h0[3] == 0.0 && h0[5] == 0.0 && h0[6] == 0.0 && h0[7] == 0.0;
     const double edge = std::min(h0[0], std::min(h0[4], h0[8]));
     arr.clus.on = allowed && arr.clus.perm && prune.delta > 0.0 && diag &&
-                  edge > 1.02 * (2.0 * (prune.rc + prune.delta) + 0.1);
+                  edge > 1.1 * (2.0 * (prune.rc + prune.delta) + 0.1);
 }
 
 // Cell edges beyond which a rebuild leaves the full rows unbuilt (0: it builds
