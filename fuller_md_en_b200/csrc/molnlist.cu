@@ -29,6 +29,7 @@
 #include "kernels.h"
 #include "ljprune.h"
 #include "molnlist.h"
+#include "molquad.h"
 
 namespace fmd {
 namespace {
@@ -480,8 +481,8 @@ __device__ __forceinline__ void mol_half_quad_body(const double* __restrict__ po
         float4 q[2], qn[2];
         auto load = [&](int t) {
             const int j0 = t < ns ? __float_as_int(sh.part[w][t].w) : i0;
-            qn[0] = pos32[j0 + (low ? lane : 0)];
-            qn[1] = pos32[j0 + (high ? lane + 32 : 0)];
+            qn[0] = pos32[quad_atom(t, ns, j0, i0, S, lane, 0)];
+            qn[1] = pos32[quad_atom(t, ns, j0, i0, S, lane, 1)];
         };
         load(0);
         for (int t = 0; t < ns; t++) {
