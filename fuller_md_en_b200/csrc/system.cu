@@ -160,8 +160,9 @@ int System::alloc_rebo() {
     return FMD_OK;
 }
 
-// Partial records of the REBO term (the learned one apart).
+// Partial records of the system's REBO term.
 int System::rebo_records() const {
+    if (arr.sg) return sg::kRowBlocks;
     if (arr.rebo2_flags & FMD_REBO2_BOND_ORDER) return rebo2_blocks(arr.n);
     return arr.rebo_mol.M ? rebo_mol_blocks(arr.rebo_mol) : rebo_slot_blocks(arr.n);
 }
@@ -1428,7 +1429,6 @@ int fmd::System::use_surrogate(fmd_sg* model, int judge_every, double rmse_max) 
     drop_graphs();                       // captured graphs hold the old REBO term
     if (!model) {
         arr.sg = nullptr;
-        arr.rebo_blocks = rebo_records();
     } else {
         if (arr.rebo2_flags & FMD_REBO2_BOND_ORDER)
             return ctx->fail(FMD_ERR_ARG, "fmd_system_use_surrogate: the system uses the REBO-II bond order");
@@ -1447,7 +1447,6 @@ int fmd::System::use_surrogate(fmd_sg* model, int judge_every, double rmse_max) 
         sg->judge_every = judge_every;
         sg->rmse_max = rmse_max;
         arr.sg = sg.get();
-        arr.rebo_blocks = sg::kRowBlocks;
         // part_f1 holds max(kForceBlocks, n) records; the learned term writes kRowBlocks.
         if (std::max(kForceBlocks, arr.n) < sg::kRowBlocks) {
             double* p1;
@@ -1456,6 +1455,7 @@ int fmd::System::use_surrogate(fmd_sg* model, int judge_every, double rmse_max) 
             arr.part_f1 = p1;
         }
     }
+    arr.rebo_blocks = rebo_records();
     // fresh judge record: the learned term is active again
     SysScal z;
     std::memset(&z, 0, sizeof(z));
