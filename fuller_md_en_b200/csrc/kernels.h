@@ -216,11 +216,14 @@ struct LJClus {
     // the molecule builder's tables and candidate bitmaps (molnlist.h)
     const int* npart = nullptr; const int* part = nullptr; const int* rev = nullptr;
     const unsigned* bm = nullptr;
-    const int* flag = nullptr;  // [0]: the last build was the molecule builder's
+    int* flag = nullptr;        // MolLists::flag: [0] the last build was the molecule builder's, [2] it left the full rows unbuilt
+    // the half rows, and the full rows (of full_cap entries), which the gather
+    // builds itself when it needs them unbuilt
+    const int* half_cnt = nullptr; const int* half_list = nullptr; int half_cap = 0;
+    int* full_cnt = nullptr; int* full_list = nullptr; int full_cap = 0;
     int4* cnt = nullptr;        // [nclus] {entries that count energy, all entries, images of its atoms}
     int* rows = nullptr;        // [nclus * stride]
     int stride = 0;
-    int in_lim = 0;             // entries from lower molecules an atom's full row holds
     double* upos = nullptr;     // [3 n] positions followed without wrapping since the last prune
     DevErr* err = nullptr;
 };
@@ -229,9 +232,9 @@ struct LJClus {
 // cannot be built (LJClus).  F, Facc, part as lj_gather_launch.  mode < 0:
 // decide (lj_clus_mode); 2: walk the rows of the last prune as they are.
 int lj_clus_blocks(int ff, int precision);
-cudaError_t lj_clus_launch(int ff, const LJClus& c, const double* pos, const double* hh, const int* in_cnt,
-                           const int* in_list, int in_cap, int na, double* F, double* Facc, double* part,
-                           cudaStream_t st, int precision, const LJPruneOut& po, int nrec, int mode = -1);
+cudaError_t lj_clus_launch(int ff, const LJClus& c, const double* pos, const double* hh, int na, double* F,
+                           double* Facc, double* part, cudaStream_t st, int precision, const LJPruneOut& po, int nrec,
+                           int mode = -1);
 cudaError_t lj_gather_launch(int ff, const double* pos, const double* hh, const int* cnt,
                              const int* list, int cap, const int* in_cnt, const int* in_list,
                              int in_cap, int na, double* F, double* Facc, double* part,

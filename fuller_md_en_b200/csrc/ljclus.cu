@@ -353,7 +353,7 @@ __device__ __forceinline__ void build_row(const LJClus& c, int k, const double* 
             po.cnt[i] = (int)((per[g / 2] >> (16 * (g & 1))) & 0xffffu);
             // more than a full row holds: an error, as where the full rows are built
             const int in = (int)((inc[g / 2] >> (16 * (g & 1))) & 0xffffu);
-            if (in > c.in_lim && atomicCAS(&c.err->code, FMD_OK, FMD_ERR_CAPACITY) == FMD_OK) {
+            if (in > c.full_cap - c.half_cap && atomicCAS(&c.err->code, FMD_OK, FMD_ERR_CAPACITY) == FMD_OK) {
                 c.err->where = K_TRANSPOSE; c.err->index = i; c.err->value = in;
             }
             po.sb[3 * i] = hi[0] * px; po.sb[3 * i + 1] = hi[4] * py; po.sb[3 * i + 2] = hi[8] * pz;
@@ -493,13 +493,43 @@ __device__ __forceinline__ void clus_reduce(ClusSum& s, int lane, double& fx, do
     }
 }
 
+// Atom i's full row, by a warp, from the candidate bitmaps: the row that
+// k_mol_incoming (molnlist.cu) builds.
+__device__ __noinline__ void build_full_row(const LJClus& c, int i, int lane) {
+    const int B = i / c.S, jb = i - B * c.S, lim = c.full_cap - c.half_cap;
+    const unsigned below = (1u << lane) - 1u;
+    int* row = c.full_list + (size_t)i * c.full_cap;
+    const int* pa = c.part + (size_t)B * c.pmax;
+    const int* rv = c.rev + (size_t)B * c.pmax;
+    const int np = c.npart[B];
+    int n = 0;
+    for (int q = 0; q < np && pa[q] < B; q++) {            // ascending: the lower partners come first
+        const int A = pa[q];
+        const unsigned* bw = c.bm + ((size_t)A * 2 * c.pmax + 2 * rv[q] + (jb >> 5)) * c.S;
+        for (int a0 = 0; a0 < c.S; a0 += 32) {
+            const bool in = a0 + lane < c.S && (bw[a0 + lane] >> (jb & 31) & 1u);
+            const unsigned m = __ballot_sync(kFull, in);
+            const int k = n + __popc(m & below);
+            if (in && k < lim) row[k] = A * c.S + a0 + lane;
+            n += __popc(m);
+        }
+    }
+    if (lane == 0 && n > lim && atomicCAS(&c.err->code, FMD_OK, FMD_ERR_CAPACITY) == FMD_OK) {
+        c.err->where = K_TRANSPOSE; c.err->index = i; c.err->value = n;
+    }
+    n = min(n, lim);
+    const int own = c.half_cnt[i];
+    for (int k = lane; k < own; k += 32) row[n + k] = c.half_list[(size_t)i * c.half_cap + k];
+    if (lane == 0) c.full_cnt[i] = n + own;
+    __syncwarp();                                          // the row, before the warp's lanes read it
+}
+
 // Atom i over its full row (when no cluster rows can be built): F, and {E, W} added to the warp's record.  Apart from the walk, so that its
 // registers are not the walk's.
 template <bool FV, bool F32>
-__device__ __noinline__ void full_row(const double* __restrict__ pos, const double* hh,
-                                      const int* __restrict__ in_cnt, const int* __restrict__ in_list, int in_cap,
-                                      int i, double* __restrict__ F, double* __restrict__ Facc, LJP p,
-                                      double* extra, int lane) {
+__device__ __noinline__ void full_row(const double* __restrict__ pos, const double* hh, const int* in_cnt,
+                                      const int* in_list, int in_cap, int i, double* __restrict__ F,
+                                      double* __restrict__ Facc, LJP p, double* extra, int lane) {
     const double* h = hh;
     const double* hi = hh + 9;
     const bool diag = h[1] == 0.0 && h[2] == 0.0 && h[3] == 0.0 && h[5] == 0.0 && h[6] == 0.0 && h[7] == 0.0 &&
@@ -539,11 +569,9 @@ __device__ __noinline__ void full_row(const double* __restrict__ pos, const doub
 // schedulers).
 template <bool FV, bool F32>
 __device__ __forceinline__ void lj_clus_body(const LJClus& c, const double* __restrict__ pos,
-                                             const double* __restrict__ hh, const int* __restrict__ in_cnt,
-                                             const int* __restrict__ in_list, int in_cap, int na,
-                                             double* __restrict__ F, double* __restrict__ Facc, const LJP& p,
-                                             double* __restrict__ part, const LJPruneOut& po, int mode, int blk,
-                                             int nblk, ClusShared& sh) {
+                                             const double* __restrict__ hh, int na, double* __restrict__ F,
+                                             double* __restrict__ Facc, const LJP& p, double* __restrict__ part,
+                                             const LJPruneOut& po, int mode, int blk, int nblk, ClusShared& sh) {
     constexpr int kClusWarps = kWarps<F32>, kClusThreads = 32 * kClusWarps;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x < 18) sh.hh[threadIdx.x] = hh[threadIdx.x];
@@ -565,8 +593,11 @@ __device__ __forceinline__ void lj_clus_body(const LJClus& c, const double* __re
     for (int k = 0; k < 6; k++) s.w[k] = 0.0;
     if (mode == CLUS_FULL) {
         const int i0 = (int)((long long)blk * na / nblk), i1 = (int)((long long)(blk + 1) * na / nblk);
-        for (int i = i0 + w; i < i1; i += kClusWarps)
-            full_row<FV, F32>(pos, sh.hh, in_cnt, in_list, in_cap, i, F, Facc, p, sh.extra[w], lane);
+        const bool build = c.flag[2] != 0;     // the last list build left them out (the step's reduction notes that they are there)
+        for (int i = i0 + w; i < i1; i += kClusWarps) {
+            if (build) build_full_row(c, i, lane);
+            full_row<FV, F32>(pos, sh.hh, c.full_cnt, c.full_list, c.full_cap, i, F, Facc, p, sh.extra[w], lane);
+        }
     } else {
         __syncthreads();                       // image offsets, clusters
         if (mode == CLUS_PRUNE)
@@ -658,13 +689,11 @@ __device__ __forceinline__ void lj_clus_body(const LJClus& c, const double* __re
 
 template <bool FV, bool F32>
 __global__ void __launch_bounds__(32 * kWarps<F32>, kBlocks<F32>)
-k_lj_clus(LJClus c, const double* __restrict__ pos, const double* __restrict__ hh, const int* __restrict__ in_cnt,
-          const int* __restrict__ in_list, int in_cap, int na, double* __restrict__ F, double* __restrict__ Facc,
-          LJP p, double* __restrict__ part, LJPruneOut po, int nrec, int mode) {
+k_lj_clus(LJClus c, const double* __restrict__ pos, const double* __restrict__ hh, int na, double* __restrict__ F,
+          double* __restrict__ Facc, LJP p, double* __restrict__ part, LJPruneOut po, int nrec, int mode) {
     FMD_PDL_WAIT();
     __shared__ ClusShared sh;
-    lj_clus_body<FV, F32>(c, pos, hh, in_cnt, in_list, in_cap, na, F, Facc, p, part, po, mode, blockIdx.x, gridDim.x,
-                          sh);
+    lj_clus_body<FV, F32>(c, pos, hh, na, F, Facc, p, part, po, mode, blockIdx.x, gridDim.x, sh);
     if (threadIdx.x < kNV)
         for (int r = gridDim.x + blockIdx.x; r < nrec; r += gridDim.x) part[(size_t)r * kNV + threadIdx.x] = 0.0;
 }
@@ -686,8 +715,8 @@ k_b_lj_clus(const StepArrays* __restrict__ As, const int* __restrict__ off, int 
     po.hb = a.prune_hb;
     po.delta = a.prune_delta;
     po.rc = a.prune_rc;
-    lj_clus_body<false, F32>(a.clus, a.pos, a.S->h, a.in_cnt, a.in_list, a.in_cap, a.n, a.F, a.Facc, p, a.part_f2, po,
-                             -1, blockIdx.x - off[r], off[r + 1] - off[r], sh);
+    lj_clus_body<false, F32>(a.clus, a.pos, a.S->h, a.n, a.F, a.Facc, p, a.part_f2, po, -1, blockIdx.x - off[r],
+                             off[r + 1] - off[r], sh);
 }
 
 template <bool FV, bool F32>
@@ -710,15 +739,14 @@ int lj_clus_blocks(int ff, int precision) {
     return f32 ? clus_grid<false, true>() : clus_grid<false, false>();
 }
 
-cudaError_t lj_clus_launch(int ff, const LJClus& c, const double* pos, const double* hh, const int* in_cnt,
-                           const int* in_list, int in_cap, int na, double* F, double* Facc, double* part,
-                           cudaStream_t st, int precision, const LJPruneOut& po, int nrec, int mode) {
+cudaError_t lj_clus_launch(int ff, const LJClus& c, const double* pos, const double* hh, int na, double* F,
+                           double* Facc, double* part, cudaStream_t st, int precision, const LJPruneOut& po, int nrec,
+                           int mode) {
     const LJP p = lj_params_dev(ff);
     const bool f32 = precision == FMD_PREC_FP32_PAIR;
     const dim3 grid(lj_clus_blocks(ff, precision)), block(32 * (f32 ? kWarps<true> : kWarps<false>));
 #define FMD_CLUS(FV, F32)                                                                                            \
-    launch_pdl(k_lj_clus<FV, F32>, grid, block, 0, st, c, pos, hh, in_cnt, in_list, in_cap, na, F, Facc, p, part, po, \
-               nrec, mode)
+    launch_pdl(k_lj_clus<FV, F32>, grid, block, 0, st, c, pos, hh, na, F, Facc, p, part, po, nrec, mode)
     if (ff == FMD_FF_AIREBO) return f32 ? FMD_CLUS(true, true) : FMD_CLUS(true, false);
     return f32 ? FMD_CLUS(false, true) : FMD_CLUS(false, false);
 #undef FMD_CLUS

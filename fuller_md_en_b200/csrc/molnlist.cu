@@ -604,8 +604,11 @@ __global__ void k_mol_rev(int M, const int* __restrict__ npart, const int* __res
 // i < j whose kept row lists j, ascending, then j's own row -- the rows the
 // transpose (nlist_transpose) builds, without atomics or a sort.  The own rows
 // are copied with 8 loads in flight per lane.
-__device__ __forceinline__ bool rows_deferred(const double* hh, double lazy_edge) {
-    return lazy_edge > 0.0 && fmin(hh[0], fmin(hh[4], hh[8])) > lazy_edge;
+// Whether this build leaves the full rows out; one block notes it.
+__device__ __forceinline__ bool rows_deferred(const double* hh, double lazy_edge, int* flag, bool note) {
+    const bool d = flag[0] != 0 && lazy_edge > 0.0 && fmin(hh[0], fmin(hh[4], hh[8])) > lazy_edge;
+    if (note && threadIdx.x == 0) flag[2] = d ? 1 : 0;
+    return d;
 }
 constexpr int kInChunk = 32;
 constexpr int kInWarps = 8;
@@ -717,9 +720,9 @@ __global__ void __launch_bounds__(32 * kInWarps)
 k_mol_incoming(int M, int S, const int* __restrict__ npart, const int* __restrict__ part, int pmax,
                const int* __restrict__ rev, int W, const unsigned* __restrict__ bm, int cap,
                const int* __restrict__ cnt, const int* __restrict__ list, int* __restrict__ in_cnt,
-               int* __restrict__ in_list, int in_cap, DevErr* err, const int* __restrict__ flag,
-               const double* __restrict__ hh, double lazy_edge) {
-    if (rows_deferred(hh, lazy_edge)) return;
+               int* __restrict__ in_list, int in_cap, DevErr* err, int* flag, const double* __restrict__ hh,
+               double lazy_edge) {
+    if (rows_deferred(hh, lazy_edge, flag, blockIdx.x == 0)) return;
     mol_incoming_body(M, S, npart, part, pmax, rev, W, bm, cap, cnt, list, in_cnt, in_list, in_cap, err, flag,
                       blockIdx.x, gridDim.x);
 }
@@ -796,7 +799,7 @@ __global__ void __launch_bounds__(32 * kInWarps)
 k_b_mol_incoming(const MolRep* __restrict__ reps, const int* __restrict__ off, int R) {
     const int r = rep_of(off, R, blockIdx.x);
     const MolRep& q = reps[r];
-    if (rows_deferred(q.hh, q.lazy_edge)) return;
+    if (rows_deferred(q.hh, q.lazy_edge, q.m.flag, (int)blockIdx.x == off[r])) return;
     mol_incoming_body(q.m.M, q.m.usize, q.m.npart, q.m.part, q.m.pmax, q.m.rev, q.m.words, q.m.bm, q.cap, q.cnt,
                       q.list, q.in_cnt, q.in_list, q.in_cap, q.err, q.m.flag, blockIdx.x - off[r],
                       off[r + 1] - off[r]);
@@ -880,10 +883,10 @@ cudaError_t mol_lists_alloc(MolLists& m, int n, const int* mol_id_host, const De
     }
     A((void**)&m.npart, sizeof(int) * M);
     A((void**)&m.part, sizeof(int) * (size_t)M * m.pmax);
-    A((void**)&m.flag, sizeof(int) * 2);
+    A((void**)&m.flag, sizeof(int) * 3);
     if (e == cudaSuccess) e = cudaMemcpy(m.off, off.data(), sizeof(int) * (M + 1), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(m.amol, amol.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(m.flag, 0, sizeof(int) * 2);
+    if (e == cudaSuccess) e = cudaMemset(m.flag, 0, sizeof(int) * 3);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);     // before any other stream reads them
     if (e != cudaSuccess) {
         mol_lists_free(m);
@@ -948,8 +951,7 @@ cudaError_t mol_rows_incoming(const MolLists& m, int cap, const int* cnt, const 
     if (!m.masks) return cudaErrorInvalidValue;
     const int blocks = 2 * m.M < kRowBlocksMol ? 2 * m.M : kRowBlocksMol;
     k_mol_incoming<<<blocks, 32 * kInWarps, 0, st>>>(m.M, m.usize, m.npart, m.part, m.pmax, m.rev, m.words, m.bm,
-                                                     cap, cnt, list, in_cnt, in_list, in_cap, err, m.flag, hh,
-                                                     hh ? lazy_edge : 0.0);
+                                                     cap, cnt, list, in_cnt, in_list, in_cap, err, m.flag, hh, lazy_edge);
     return cudaGetLastError();
 }
 

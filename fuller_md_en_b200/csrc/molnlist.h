@@ -30,7 +30,7 @@ struct MolLists {
     float4* pos32 = nullptr;  // [n] positions of the build rounded to FP32 (w unused), for the prefilter
     int* npart = nullptr;     // [M] partner count
     int* part = nullptr;      // [M * pmax] partners, ascending
-    int* flag = nullptr;      // [2] {molecule path valid, partner overflow}
+    int* flag = nullptr;      // [3] {molecule path valid, partner overflow, full rows left unbuilt}
 };
 
 // Host set-up from the atoms' molecule ids; m.ok stays false (the cell-grid
@@ -50,7 +50,9 @@ cudaError_t mol_rows_half(const MolLists& m, const double* pos, const double* hh
 // unless flag[0] is set.
 // hh, lazy_edge > 0: nothing is built while every edge of the (diagonal) cell
 // exceeds lazy_edge -- the system's gather walks cluster rows and the full
-// rows are built when somebody asks for them (System::ensure_full_rows).
+// rows are built when somebody asks for them (System::ensure_full_rows) or
+// when a cell that no longer takes cluster rows needs them (ljclus.cu).
+// flag[2] says whether the last build left them out.
 cudaError_t mol_rows_incoming(const MolLists& m, int cap, const int* cnt, const int* list, int* in_cnt,
                               int* in_list, int in_cap, DevErr* err, cudaStream_t st, const double* hh = nullptr,
                               double lazy_edge = 0.0);

@@ -487,10 +487,14 @@ __device__ void lj_prune_commit(const StepArrays& a, const double* hh) {
         atomicAdd(&a.prune_stats[0], 1ull);
         return;
     }
-    const bool pruned = a.clus.on ? lj_clus_mode(a.clus, a.prune_umax, hh, a.prune_hb, a.prune_delta, a.prune_rc) ==
-                                        CLUS_PRUNE
-                                  : lj_prune_needed(a.prune_umax, hh, a.prune_hb, a.prune_delta, a.prune_rc,
-                                                    kRowsAtoms);
+    bool pruned;
+    if (a.clus.on) {
+        const int mode = lj_clus_mode(a.clus, a.prune_umax, hh, a.prune_hb, a.prune_delta, a.prune_rc);
+        if (mode == CLUS_FULL) a.clus.flag[2] = 0;         // the gather has built the full rows
+        pruned = mode == CLUS_PRUNE;
+    } else {
+        pruned = lj_prune_needed(a.prune_umax, hh, a.prune_hb, a.prune_delta, a.prune_rc, kRowsAtoms);
+    }
     if (pruned) {
         a.prune_umax[0] = 0ull;
         a.prune_umax[1] = lj_rows_tag(a.clus.on ? kRowsClusters : kRowsAtoms, a.prune_delta);
@@ -728,8 +732,8 @@ cudaError_t enqueue_lj(const StepArrays& a, int ff, cudaStream_t st) {
         return lj_gather_launch(ff, a.pos, hh, a.cnt_a, a.list_a, a.cap_a, a.in_cnt, a.in_list, a.in_cap, a.n, a.F,
                                 a.Facc, a.part_f2, st, a.precision, a.lj_shape, a.err, LJPruneOut{}, a.lj_blocks);
     if (a.clus.on)
-        return lj_clus_launch(ff, a.clus, a.pos, hh, a.in_cnt, a.in_list, a.in_cap, a.n, a.F, a.Facc, a.part_f2, st,
-                              a.precision, lj_prune_out(*a.prune), a.lj_blocks);
+        return lj_clus_launch(ff, a.clus, a.pos, hh, a.n, a.F, a.Facc, a.part_f2, st, a.precision,
+                              lj_prune_out(*a.prune), a.lj_blocks);
     // one launch: each block decides whether this evaluation prunes (full
     // rows, pruned rows written) or walks the pruned rows; the step's
     // reduction then restarts the displacement bound (lj_prune_commit)

@@ -228,7 +228,8 @@ int System::alloc_clus(const double* pos_h) {
     q.perm = dp;
     q.npart = mol.npart; q.part = mol.part; q.rev = mol.rev; q.bm = mol.bm; q.flag = mol.flag;
     q.err = ctx->d_err;
-    q.in_lim = arr.in_cap - arr.cap_a;
+    q.half_cnt = arr.cnt_a; q.half_list = arr.list_a; q.half_cap = arr.cap_a;
+    q.full_cnt = const_cast<int*>(arr.in_cnt); q.full_list = const_cast<int*>(arr.in_list); q.full_cap = arr.in_cap;
     q.rows = prune.list;
     q.stride = (int)std::min<size_t>((size_t)kClusG * arr.in_cap, (size_t)arr.n * arr.in_cap / q.nclus);
     arr.clus = q;
@@ -252,6 +253,8 @@ void System::set_clus(bool allowed) {
 // Cell edges beyond which a rebuild leaves the full rows unbuilt (0: it builds
 // them): those the cluster gather takes, with a margin above what the barostat
 // (edge rates clamped at 0.005 A/fs) can shorten them by before the next one.
+// Where that does not hold (a cell that shears, steps that go on without a
+// rebuild), the gather builds the rows that it needs.
 double System::lazy_edge() const {
     if (!arr.clus.on) return 0.0;
     return 2.0 * (prune.rc + prune.delta) + 0.2 + 0.01 * std::fabs(sp.dt) * p.nlup;
@@ -1205,8 +1208,8 @@ extern "C" int fmd_system_kernel_ms(fmd_system* s, int stage, int reps, double* 
                 if (!a.prune) return cudaErrorInvalidValue;
                 if (a.clus.on)
                     return lj_clus_launch(a.kind == FMD_SYS_AIREBO ? FMD_FF_AIREBO : FMD_FF_MM, a.clus, a.pos, hh,
-                                          a.in_cnt, a.in_list, a.in_cap, a.n, a.Facc, a.Facc, a.part_f2, st,
-                                          a.precision, lj_prune_out(*a.prune), 0, 2);
+                                          a.n, a.Facc, a.Facc, a.part_f2, st, a.precision, lj_prune_out(*a.prune), 0,
+                                          2);
                 return lj_gather_launch(a.kind == FMD_SYS_AIREBO ? FMD_FF_AIREBO : FMD_FF_MM, a.pos, hh, a.cnt_a,
                                         a.list_a, a.cap_a, a.prune->cnt, a.prune->list, a.in_cap, a.n, a.Facc,
                                         a.Facc, a.part_f2, st, a.precision, a.lj_shape_p, a.err);
