@@ -105,6 +105,7 @@ struct fmd_batch {
             q.in_list = const_cast<int*>(s->arr.in_list);
             q.err = ctx->d_err;
             q.prune_words = s->prune.ok ? s->prune.words : nullptr;
+            q.stats = bd.lj_clus ? s->prune.stats : nullptr;
             q.lazy_edge = bd.lj_clus ? s->lazy_edge() : 0.0;
             const int M = s->mol.M;
             const int share = (int)std::max(1LL, (kRowBlocks * (long long)s->arr.n + ntot / 2) / ntot);

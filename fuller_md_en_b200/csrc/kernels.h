@@ -216,7 +216,7 @@ struct LJClus {
     // the molecule builder's tables and candidate bitmaps (molnlist.h)
     const int* npart = nullptr; const int* part = nullptr; const int* rev = nullptr;
     const unsigned* bm = nullptr;
-    int* flag = nullptr;        // MolLists::flag: [0] the last build was the molecule builder's, [2] it left the full rows unbuilt
+    int* flag = nullptr;        // MolLists::flag
     // the half rows, and the full rows (of full_cap entries), which the gather
     // builds itself when it needs them unbuilt
     const int* half_cnt = nullptr; const int* half_list = nullptr; int half_cap = 0;
@@ -227,11 +227,12 @@ struct LJClus {
     double* upos = nullptr;     // [3 n] positions followed without wrapping since the last prune
     DevErr* err = nullptr;
 };
-// The step's LJ term over cluster rows: each evaluation builds them when a
-// prune is due (lj_prune_needed) and walks them, or the full rows when they
-// cannot be built (LJClus).  F, Facc, part as lj_gather_launch.  mode < 0:
-// decide (lj_clus_mode); 2: walk the rows of the last prune as they are.
+// The step's LJ term over cluster rows, or over pruned rows of atoms where
+// those cannot be had or do not pay: each evaluation builds them when a prune
+// is due (lj_prune_needed) and walks them.  F, Facc, part as lj_gather_launch.
+// mode < 0: decide (lj_clus_mode), else as told.
 int lj_clus_blocks(int ff, int precision);
+int lj_clus_threads(int precision);
 cudaError_t lj_clus_launch(int ff, const LJClus& c, const double* pos, const double* hh, int na, double* F,
                            double* Facc, double* part, cudaStream_t st, int precision, const LJPruneOut& po, int nrec,
                            int mode = -1);

@@ -36,6 +36,15 @@
 // rc + delta now are kept.  When they may be used and must be rebuilt is the
 // pruned rows' rule (ljprune.cu).
 //
+// Rows of atoms.  Where cluster rows cannot be had (a build by cells, a cell that
+// is not diagonal or too narrow) or do not pay (atoms so fast that most
+// evaluations build rows: molnlist.cu decides at each list build), the same
+// kernel does what the row gather does, an atom a warp over full and pruned
+// rows (atom_rows), with the pair terms of a chunk free of branches: with 12
+// warps an SM the chunk's independent chains stand in for the row gather's
+// warps.  30,000 atoms, pruning / walking: 126 / 66 us (the row gather 122 /
+// 67; with its branches here 155 / 82), FP32 pairs 132 / 72 (200 / 109).
+//
 // Virial: sum over pairs of fm d (x) d with d = d0 - x_g, d0 the partner
 // from the cluster's first atom and x_g atom g from it, is
 // sum d0 (x) (sum_g fm d) - sum_g x_g (x) (sum fm d): per entry one product of
@@ -43,6 +52,7 @@
 #include <algorithm>
 #include <cmath>
 #include <limits>
+#include <type_traits>
 #include <vector>
 
 #include "ljclus.cuh"
@@ -61,6 +71,7 @@ namespace {
 template <bool F32> constexpr int kWarps = F32 ? 8 : 12;
 template <bool F32> constexpr int kBlocks = F32 ? 2 : 1;
 constexpr int kMaxWarps = 12;
+constexpr int kAtomUnroll = 4;             // entries per lane in flight of rows of atoms
 constexpr int kClusUnroll = 2;             // slices per trip: saves the feed's register moves (142 -> 138 us)
 constexpr int kMaskBit = 22, kCodeBit = 27;
 constexpr unsigned kAtomBits = (1u << kMaskBit) - 1u;
@@ -362,11 +373,44 @@ __device__ __forceinline__ void build_row(const LJClus& c, int k, const double* 
     }
 }
 
-// Pair sums of a lane: fm d per atom of the cluster, and on the counting side
-// the virial's first part, the energy and the number of pairs.
+// A pair's force over its distance, zero where the pair is out (in), without
+// the factor 24 eps sigma^6 in FP64.  COUNT: its energy (without 4 eps sigma^6
+// and the shift in FP64) and number, with SOME only where count says so.  No
+// branches, so that the pairs of a lane are independent chains.
 struct ClusConst {
     double s6, two_s6;                         // sigma^6, twice
 };
+template <bool F32, bool COUNT, bool SOME>
+__device__ __forceinline__ double pair_term(double r2, bool in, bool count, const LJP& p, const LJF& pf,
+                                            const ClusConst& cc, double& e, int& np) {
+    // r^2 < 1/4 by its high word: exact, and not on the FP64 pipe
+    const int rh = __double2hiint(r2);
+    const bool close = rh < 0x3fd00000;
+    r2 = __hiloint2double(close ? 0x3fd00000 : rh, close ? 0 : __double2loint(r2));
+    if (F32) {
+        // the FP32 pair algebra of lj_pair, operation for operation
+        const float ri2 = rcp_f32((float)r2);
+        const float s2 = fmaf(pf.sig2, ri2, pf.sig2_lo * ri2), s6 = s2 * s2 * s2, s12 = s6 * s6;
+        if (COUNT && (SOME ? count : in)) e += (double)(pf.c4 * (s12 - s6)) - p.vshift;
+        return in ? (double)(pf.c24 * (2.f * s12 - s6) * ri2) : 0.0;
+    }
+    // 1/r^2 as in lj_pair, zero where the pair is out (by the approximation's
+    // high word)
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+    y = __hiloint2double(in ? __double2hiint(y) : 0, 0);
+    const double e0 = fma(-r2, y, 1.0), e1 = fma(e0, e0, e0), i2 = fma(y, e1, y);
+    const double i6 = i2 * i2 * i2;
+    if (COUNT) {
+        const double c6 = SOME ? __hiloint2double(count ? __double2hiint(i6) : 0, count ? __double2loint(i6) : 0) : i6;
+        e = fma(c6, fma(cc.s6, i6, -1.0), e);
+        np += SOME ? count : in;
+    }
+    return (i6 * i2) * fma(cc.two_s6, i6, -1.0);
+}
+
+// Pair sums of a lane: fm d per atom of the cluster, and on the counting side
+// the virial's first part, the energy and the number of pairs.
 struct ClusSum {
     double fx[kClusG], fy[kClusG], fz[kClusG];
     double w[6];                               // xx xy xz yy yz zz
@@ -408,34 +452,9 @@ __device__ __forceinline__ void clus_slices(const double* __restrict__ pos, int 
 #pragma unroll
         for (int g = 0; g < kClusG; g++) {
             const double dx = g ? d0x - q.x[g] : d0x, dy = g ? d0y - q.y[g] : d0y, dz = g ? d0z - q.z[g] : d0z;
-            double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+            const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
             const bool in = ((ec >> (kMaskBit + g)) & 1u) && !(r2 > p.rc2);
-            // r^2 < 1/4 by its high word: exact, and not on the FP64 pipe
-            const int rh = __double2hiint(r2);
-            const bool close = rh < 0x3fd00000;
-            r2 = __hiloint2double(close ? 0x3fd00000 : rh, close ? 0 : __double2loint(r2));
-            double fm;
-            if (F32) {
-                // the FP32 pair algebra of lj_pair, operation for operation
-                const float ri2 = rcp_f32((float)r2);
-                const float s2 = fmaf(pf.sig2, ri2, pf.sig2_lo * ri2), s6 = s2 * s2 * s2, s12 = s6 * s6;
-                fm = in ? (double)(pf.c24 * (2.f * s12 - s6) * ri2) : 0.0;
-                if (OWN && in) s.e += (double)(pf.c4 * (s12 - s6)) - p.vshift;
-            } else {
-                // 1/r^2 as in lj_pair, zero where the pair is out (by the
-                // approximation's high word); fm and the energy without their
-                // factors 24 eps sigma^6 and 4 eps sigma^6
-                double y;
-                asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
-                y = __hiloint2double(in ? __double2hiint(y) : 0, 0);
-                const double e0 = fma(-r2, y, 1.0), e1 = fma(e0, e0, e0), i2 = fma(y, e1, y);
-                const double i6 = i2 * i2 * i2;
-                fm = (i6 * i2) * fma(cc.two_s6, i6, -1.0);
-                if (OWN) {
-                    s.e = fma(i6, fma(cc.s6, i6, -1.0), s.e);
-                    s.np += in;
-                }
-            }
+            const double fm = pair_term<F32, OWN, false>(r2, in, in, p, pf, cc, s.e, s.np);
             s.fx[g] = fma(fm, dx, s.fx[g]);
             s.fy[g] = fma(fm, dy, s.fy[g]);
             s.fz[g] = fma(fm, dz, s.fz[g]);
@@ -524,41 +543,113 @@ __device__ __noinline__ void build_full_row(const LJClus& c, int i, int lane) {
     __syncwarp();                                          // the row, before the warp's lanes read it
 }
 
-// Atom i over its full row (when no cluster rows can be built): F, and {E, W} added to the warp's record.  Apart from the walk, so that its
-// registers are not the walk's.
+// Atoms i0 + w, i0 + w + (warps), ... below i1 over rows of their own, as the
+// row gather (airebo.cu): over the full rows, which it builds first where the
+// list build left them out, writing the pruned ones (prune), or over those of
+// the last prune.  F, and {E, W} added to the warp's record.  Apart from the
+// cluster walk, so that its registers are not the walk's.
 template <bool FV, bool F32>
-__device__ __noinline__ void full_row(const double* __restrict__ pos, const double* hh, const int* in_cnt,
-                                      const int* in_list, int in_cap, int i, double* __restrict__ F,
-                                      double* __restrict__ Facc, LJP p, double* extra, int lane) {
+__device__ __noinline__ void atom_rows(const LJClus& c, const double* __restrict__ pos, const double* hh, int i0,
+                                       int i1, int w, double* __restrict__ F, double* __restrict__ Facc, LJP p,
+                                       const LJPruneOut& rows, bool prune, double* extra, int lane) {
     const double* h = hh;
     const double* hi = hh + 9;
     const bool diag = h[1] == 0.0 && h[2] == 0.0 && h[3] == 0.0 && h[5] == 0.0 && h[6] == 0.0 && h[7] == 0.0 &&
                       hi[1] == 0.0 && hi[2] == 0.0 && hi[3] == 0.0 && hi[5] == 0.0 && hi[6] == 0.0 && hi[7] == 0.0;
     const bool wide = diag && 0.25 * fmin(h[0] * h[0], fmin(h[4] * h[4], h[8] * h[8])) > p.rc2 * (1.0 + 1e-9);
     const LJF pf{(float)p.sig2, (float)(p.sig2 - (double)(float)p.sig2), (float)p.c4, (float)p.c24};
-    double acc[kNV];
+    const ClusConst cc{p.sig2 * p.sig2 * p.sig2, 2.0 * (p.sig2 * p.sig2 * p.sig2)};
+    const double fs = F32 ? 1.0 : p.c24 * cc.s6;
+    double acc[kNV], e = 0.0, vir[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    int np = 0;
 #pragma unroll
     for (int k = 0; k < kNV; k++) acc[k] = 0.0;
-    constexpr int U = 4;
-    const double px = pos[3 * i], py = pos[3 * i + 1], pz = pos[3 * i + 2];
-    const LJAcc fa = lj_acc_load(Facc, i, lane);
-    double fx = 0.0, fy = 0.0, fz = 0.0;
-    const int tot = min(in_cnt[i], in_cap);
-    const int* row = in_list + (size_t)i * in_cap;
-    int pc = 0;
-    for (int b0 = 0; b0 < tot; b0 += 32 * U) {
-        int jc[U];
-        double cx[U], cy[U], cz[U];
-        lj_fetch<U>(pos, row, tot, b0 + lane, i, jc, cx, cy, cz);
-        lj_chunk<FV, F32, U>(jc, cx, cy, cz, i, px, py, pz, h, hi, diag, wide, p, pf, fx, fy, fz, acc, LJPruneOut{},
-                             nullptr, pc, lane);
+    constexpr int U = kAtomUnroll;
+    LJPruneOut po = rows;
+    po.list = c.rows;
+    const int* cnt = prune ? c.full_cnt : po.cnt;
+    const int* list = prune ? c.full_list : c.rows;
+    if (!prune) po.cnt = nullptr;
+    const bool build = prune && c.flag[2] != 0;
+    for (int i = i0 + w; i < i1; i += kWarps<F32>) {
+        if (build) build_full_row(c, i, lane);
+        const double px = pos[3 * i], py = pos[3 * i + 1], pz = pos[3 * i + 2];
+        const LJAcc fa = lj_acc_load(Facc, i, lane);
+        double fx = 0.0, fy = 0.0, fz = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
+        const int tot = min(cnt[i], c.full_cap);
+        const int* row = list + (size_t)i * c.full_cap;
+        int* prow = c.rows + (size_t)i * c.full_cap;
+        int pc = 0;
+        int jj[U];                                         // indices one chunk ahead
+#pragma unroll
+        for (int u = 0; u < U; u++) jj[u] = lane + 32 * u < tot ? row[lane + 32 * u] : -1;
+        for (int b0 = 0; b0 < tot; b0 += 32 * U) {
+            int jc[U];
+            double cx[U], cy[U], cz[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int j = jj[u] < 0 ? i : jj[u];
+                jc[u] = jj[u];
+                cx[u] = pos[3 * j]; cy[u] = pos[3 * j + 1]; cz[u] = pos[3 * j + 2];
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int k = b0 + 32 * (U + u) + lane;
+                jj[u] = k < tot ? row[k] : -1;
+            }
+            if (!wide) {
+                lj_chunk<FV, F32, U>(jc, cx, cy, cz, i, px, py, pz, h, hi, diag, wide, p, pf, fx, fy, fz, acc, po, prow,
+                                     pc, lane);
+                continue;
+            }
+            bool keep[U];
+            auto chunk = [&](auto count_tag) {
+                constexpr bool COUNT = decltype(count_tag)::value;
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const double dx = mimg1_rint(__dsub_rn(cx[u], px), h[0], hi[0]),
+                                 dy = mimg1_rint(__dsub_rn(cy[u], py), h[4], hi[4]),
+                                 dz = mimg1_rint(__dsub_rn(cz[u], pz), h[8], hi[8]);
+                    const double r2 = norm2_rn(dx, dy, dz);
+                    const bool in = jc[u] >= 0 && !(r2 > p.rc2), own = jc[u] > i;
+                    keep[u] = jc[u] >= 0 && r2 <= po.r2;
+                    const double fm = pair_term<F32, COUNT, true>(r2, in, in && own, p, pf, cc, e, np);
+                    const double gx = fm * dx, gy = fm * dy, gz = fm * dz;
+                    sx += gx; sy += gy; sz += gz;
+                    if (COUNT) {
+                        const double ox = own ? gx : 0.0, oy = own ? gy : 0.0, oz = own ? gz : 0.0;
+                        vir[0] = fma(dx, ox, vir[0]);
+                        if (FV) { vir[1] = fma(dx, oy, vir[1]); vir[2] = fma(dx, oz, vir[2]); }
+                        vir[3] = fma(dy, oy, vir[3]);
+                        if (FV) vir[4] = fma(dy, oz, vir[4]);
+                        vir[5] = fma(dz, oz, vir[5]);
+                    }
+                }
+            };
+            bool own = false;
+#pragma unroll
+            for (int u = 0; u < U; u++) own = own || jc[u] > i;
+            if (__any_sync(kFull, own)) chunk(std::true_type{});
+            else chunk(std::false_type{});
+            if (po.cnt) {
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const unsigned m = __ballot_sync(kFull, keep[u]);
+                    if (keep[u]) prow[pc + __popc(m & ((1u << lane) - 1u))] = jc[u];
+                    pc += __popc(m);
+                }
+            }
+        }
+        lj_atom_done(i, fx - fs * sx, fy - fs * sy, fz - fs * sz, px, py, pz, hi, F, Facc, po, pc, lane, fa);
     }
-    lj_atom_done(i, fx, fy, fz, px, py, pz, hi, F, Facc, LJPruneOut{}, 0, lane, fa);
+    acc[0] += F32 ? e : p.c4 * cc.s6 * e - p.vshift * np;
+    acc[1] += fs * vir[0]; acc[5] += fs * vir[3]; acc[9] += fs * vir[5];
+    acc[2] += fs * vir[1]; acc[3] += fs * vir[2]; acc[6] += fs * vir[4];
     lj_virial_mirror<FV>(acc);
 #pragma unroll
     for (int k = 0; k < kNV; k++) {
         const double t = warp_sum(acc[k]);
-        if (lane == 0) extra[k] += t;
+        if (lane == 0) extra[k] = t;
     }
 }
 
@@ -591,13 +682,9 @@ __device__ __forceinline__ void lj_clus_body(const LJClus& c, const double* __re
     s.np = 0;
 #pragma unroll
     for (int k = 0; k < 6; k++) s.w[k] = 0.0;
-    if (mode == CLUS_FULL) {
+    if (lj_clus_kind(mode) == kRowsAtoms) {
         const int i0 = (int)((long long)blk * na / nblk), i1 = (int)((long long)(blk + 1) * na / nblk);
-        const bool build = c.flag[2] != 0;     // the last list build left them out (the step's reduction notes that they are there)
-        for (int i = i0 + w; i < i1; i += kClusWarps) {
-            if (build) build_full_row(c, i, lane);
-            full_row<FV, F32>(pos, sh.hh, c.full_cnt, c.full_list, c.full_cap, i, F, Facc, p, sh.extra[w], lane);
-        }
+        atom_rows<FV, F32>(c, pos, sh.hh, i0, i1, w, F, Facc, p, po, lj_clus_prunes(mode), sh.extra[w], lane);
     } else {
         __syncthreads();                       // image offsets, clusters
         if (mode == CLUS_PRUNE)
@@ -689,8 +776,9 @@ __device__ __forceinline__ void lj_clus_body(const LJClus& c, const double* __re
 
 template <bool FV, bool F32>
 __global__ void __launch_bounds__(32 * kWarps<F32>, kBlocks<F32>)
-k_lj_clus(LJClus c, const double* __restrict__ pos, const double* __restrict__ hh, int na, double* __restrict__ F,
-          double* __restrict__ Facc, LJP p, double* __restrict__ part, LJPruneOut po, int nrec, int mode) {
+k_lj_clus(const __grid_constant__ LJClus c, const double* __restrict__ pos, const double* __restrict__ hh, int na,
+          double* __restrict__ F, double* __restrict__ Facc, LJP p, double* __restrict__ part,
+          const __grid_constant__ LJPruneOut po, int nrec, int mode) {
     FMD_PDL_WAIT();
     __shared__ ClusShared sh;
     lj_clus_body<FV, F32>(c, pos, hh, na, F, Facc, p, part, po, mode, blockIdx.x, gridDim.x, sh);
@@ -733,6 +821,8 @@ int clus_grid() {
 
 }  // namespace
 
+int lj_clus_threads(int precision) { return 32 * (precision == FMD_PREC_FP32_PAIR ? kWarps<true> : kWarps<false>); }
+
 int lj_clus_blocks(int ff, int precision) {
     const bool f32 = precision == FMD_PREC_FP32_PAIR;
     if (ff == FMD_FF_AIREBO) return f32 ? clus_grid<true, true>() : clus_grid<true, false>();
@@ -744,7 +834,7 @@ cudaError_t lj_clus_launch(int ff, const LJClus& c, const double* pos, const dou
                            int mode) {
     const LJP p = lj_params_dev(ff);
     const bool f32 = precision == FMD_PREC_FP32_PAIR;
-    const dim3 grid(lj_clus_blocks(ff, precision)), block(32 * (f32 ? kWarps<true> : kWarps<false>));
+    const dim3 grid(lj_clus_blocks(ff, precision)), block(lj_clus_threads(precision));
 #define FMD_CLUS(FV, F32)                                                                                            \
     launch_pdl(k_lj_clus<FV, F32>, grid, block, 0, st, c, pos, hh, na, F, Facc, p, part, po, nrec, mode)
     if (ff == FMD_FF_AIREBO) return f32 ? FMD_CLUS(true, true) : FMD_CLUS(true, false);

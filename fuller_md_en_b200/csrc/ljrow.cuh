@@ -1,7 +1,6 @@
 // ljrow.cuh -- one atom's row of the LJ gather: entries fetched by the lanes of
 // a warp, the pair terms of a chunk, and the end of the row.  Used by the row
-// gathers (airebo.cu) and by the cluster gather where it cannot build its
-// rows (ljclus.cu).
+// gathers (airebo.cu) and by the cluster gather's rows of atoms (ljclus.cu).
 #pragma once
 #include "geom.cuh"
 #include "kernels.h"

@@ -153,8 +153,30 @@ __global__ void k_mol_pairs(const double* __restrict__ hh, int M, const double* 
     mol_pairs_body(hh, M, cen, rad, rc, pmax, npart, part, flag, blockIdx.x);
 }
 
-__global__ void k_mol_decide(const double* __restrict__ hh, int* __restrict__ flag) {
-    if (threadIdx.x == 0) flag[0] = (diag_cell(hh, hh + 9) && flag[1] == 0) ? 1 : 0;
+// Whether the LJ gather walks rows of atoms until the next build: when more
+// than a quarter of the evaluations since the last build pruned because atoms
+// had moved (the first one after a build prunes anyway).  us per evaluation
+// over cluster rows, walk / prune, and over rows of atoms, with the full rows a
+// build then makes (FP64, molecules heating up): 1,920 atoms 8 / 32 and 12 /
+// 16 + 20 a build, 30,000 atoms 40 / 185 and 66 / 126 + 65, 122,880 atoms 160 /
+// 720 and 300 / 485 + 243; with a build every 20 steps these meet at 3, 6 and 7
+// such prunes between two builds.
+__device__ __forceinline__ void rows_decide(unsigned long long* stats, int* flag) {
+    if (!stats) {
+        flag[3] = 0;
+        return;
+    }
+    const unsigned long long n = stats[0] - stats[2], p = stats[1] - stats[3];
+    if (n == 0) return;                    // no evaluation since the last build
+    flag[3] = 4 * (p - (p > 0)) > n ? 1 : 0;
+    stats[2] = stats[0];
+    stats[3] = stats[1];
+}
+
+__global__ void k_mol_decide(const double* __restrict__ hh, int* __restrict__ flag, unsigned long long* stats) {
+    if (threadIdx.x != 0) return;
+    flag[0] = (diag_cell(hh, hh + 9) && flag[1] == 0) ? 1 : 0;
+    rows_decide(stats, flag);
 }
 
 // FP32 screen of the reference's test r^2 < rc2 (diagonal cell): positions
@@ -606,7 +628,7 @@ __global__ void k_mol_rev(int M, const int* __restrict__ npart, const int* __res
 // are copied with 8 loads in flight per lane.
 // Whether this build leaves the full rows out; one block notes it.
 __device__ __forceinline__ bool rows_deferred(const double* hh, double lazy_edge, int* flag, bool note) {
-    const bool d = flag[0] != 0 && lazy_edge > 0.0 && fmin(hh[0], fmin(hh[4], hh[8])) > lazy_edge;
+    const bool d = flag[0] != 0 && flag[3] == 0 && lazy_edge > 0.0 && fmin(hh[0], fmin(hh[4], hh[8])) > lazy_edge;
     if (note && threadIdx.x == 0) flag[2] = d ? 1 : 0;
     return d;
 }
@@ -767,6 +789,7 @@ __global__ void k_b_mol_decide(const MolRep* __restrict__ reps, int R) {
         const double* hh = reps[r].hh;
         int* flag = reps[r].m.flag;
         flag[0] = (diag_cell(hh, hh + 9) && flag[1] == 0) ? 1 : 0;
+        rows_decide(reps[r].stats, flag);
     }
 }
 
@@ -883,10 +906,10 @@ cudaError_t mol_lists_alloc(MolLists& m, int n, const int* mol_id_host, const De
     }
     A((void**)&m.npart, sizeof(int) * M);
     A((void**)&m.part, sizeof(int) * (size_t)M * m.pmax);
-    A((void**)&m.flag, sizeof(int) * 3);
+    A((void**)&m.flag, sizeof(int) * 4);
     if (e == cudaSuccess) e = cudaMemcpy(m.off, off.data(), sizeof(int) * (M + 1), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(m.amol, amol.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(m.flag, 0, sizeof(int) * 3);
+    if (e == cudaSuccess) e = cudaMemset(m.flag, 0, sizeof(int) * 4);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);     // before any other stream reads them
     if (e != cudaSuccess) {
         mol_lists_free(m);
@@ -908,11 +931,12 @@ void mol_lists_free(MolLists& m) {
     m = MolLists();
 }
 
-cudaError_t mol_partners(MolLists& m, const double* pos, const double* hh, double rc, cudaStream_t st) {
+cudaError_t mol_partners(MolLists& m, const double* pos, const double* hh, double rc, cudaStream_t st,
+                         unsigned long long* stats) {
     const int wblocks = (m.M * 32 + 255) / 256;
     k_mol_centre<<<wblocks, 256, 0, st>>>(pos, hh, m.off, m.M, m.cen, m.rad, m.pos32, m.flag);
     k_mol_pairs<<<wblocks, 256, 0, st>>>(hh, m.M, m.cen, m.rad, rc, m.pmax, m.npart, m.part, m.flag);
-    k_mol_decide<<<1, 32, 0, st>>>(hh, m.flag);
+    k_mol_decide<<<1, 32, 0, st>>>(hh, m.flag, stats);
     if (m.masks) k_mol_rev<<<wblocks, 256, 0, st>>>(m.M, m.npart, m.part, m.pmax, m.rev, m.flag);
     return cudaGetLastError();
 }

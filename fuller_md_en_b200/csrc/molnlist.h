@@ -30,7 +30,8 @@ struct MolLists {
     float4* pos32 = nullptr;  // [n] positions of the build rounded to FP32 (w unused), for the prefilter
     int* npart = nullptr;     // [M] partner count
     int* part = nullptr;      // [M * pmax] partners, ascending
-    int* flag = nullptr;      // [3] {molecule path valid, partner overflow, full rows left unbuilt}
+    int* flag = nullptr;      // [4] {molecule path valid, partner overflow, full rows left unbuilt,
+                              //      LJ rows of atoms until the next build}
 };
 
 // Host set-up from the atoms' molecule ids; m.ok stays false (the cell-grid
@@ -38,7 +39,9 @@ struct MolLists {
 cudaError_t mol_lists_alloc(MolLists& m, int n, const int* mol_id_host, const DevAlloc& da = DevAlloc{});
 void mol_lists_free(MolLists& m);
 // Centres, radii and partner molecules for list radius rc; sets flag[0].
-cudaError_t mol_partners(MolLists& m, const double* pos, const double* hh, double rc, cudaStream_t st);
+// stats (LJPrune::stats, or null): flag[3] from the prunes since the last build.
+cudaError_t mol_partners(MolLists& m, const double* pos, const double* hh, double rc, cudaStream_t st,
+                         unsigned long long* stats = nullptr);
 // Intramolecular rows (always valid for contiguous molecules).
 cudaError_t mol_rows_intra(const MolLists& m, const double* pos, const double* hh, double rc2, int cap, int* cnt,
                            int* list, int* dropped, cudaStream_t st);
@@ -49,7 +52,7 @@ cudaError_t mol_rows_half(const MolLists& m, const double* pos, const double* hh
 // the candidate bitmaps of the last mol_rows_half (m.masks only); no-op
 // unless flag[0] is set.
 // hh, lazy_edge > 0: nothing is built while every edge of the (diagonal) cell
-// exceeds lazy_edge -- the system's gather walks cluster rows and the full
+// exceeds lazy_edge and flag[3] is clear -- the system's gather walks cluster rows and the full
 // rows are built when somebody asks for them (System::ensure_full_rows) or
 // when a cell that no longer takes cluster rows needs them (ljclus.cu).
 // flag[2] says whether the last build left them out.
@@ -72,6 +75,7 @@ struct MolRep {
     int* in_list = nullptr;
     double lazy_edge = 0.0;               // as mol_rows_incoming
     DevErr* err = nullptr;
+    unsigned long long* stats = nullptr;  // as mol_partners
     unsigned long long* prune_words = nullptr;   // the replica's pruned-row bound (marked stale), or null
 };
 // Device table of the replicas and the block offsets (R + 1 each) of the

@@ -487,21 +487,19 @@ __device__ void lj_prune_commit(const StepArrays& a, const double* hh) {
         atomicAdd(&a.prune_stats[0], 1ull);
         return;
     }
-    bool pruned;
-    if (a.clus.on) {
-        const int mode = lj_clus_mode(a.clus, a.prune_umax, hh, a.prune_hb, a.prune_delta, a.prune_rc);
-        if (mode == CLUS_FULL) a.clus.flag[2] = 0;         // the gather has built the full rows
-        pruned = mode == CLUS_PRUNE;
-    } else {
-        pruned = lj_prune_needed(a.prune_umax, hh, a.prune_hb, a.prune_delta, a.prune_rc, kRowsAtoms);
-    }
-    if (pruned) {
+    const int mode = a.clus.on ? lj_clus_mode(a.clus, a.prune_umax, hh, a.prune_hb, a.prune_delta, a.prune_rc)
+                     : lj_prune_needed(a.prune_umax, hh, a.prune_hb, a.prune_delta, a.prune_rc, kRowsAtoms)
+                         ? ATOMS_PRUNE
+                         : ATOMS_WALK;
+    if (a.clus.on && mode == ATOMS_PRUNE) a.clus.flag[2] = 0;          // the gather has built the full rows
+    if (lj_clus_prunes(mode)) {
         a.prune_umax[0] = 0ull;
-        a.prune_umax[1] = lj_rows_tag(a.clus.on ? kRowsClusters : kRowsAtoms, a.prune_delta);
+        a.prune_umax[1] = lj_rows_tag(lj_clus_kind(mode), a.prune_delta);
         for (int q = 0; q < 9; q++) a.prune_hb[q] = hh[q];
         atomicAdd(&a.prune_stats[1], 1ull);
     }
     atomicAdd(&a.prune_stats[0], 1ull);
+    atomicAdd(&a.prune_stats[4 + mode], 1ull);
 }
 
 // The scalar end of a step on the copy S, by the block's threads: thread 0 the

@@ -12,8 +12,8 @@
 #include <map>
 #include <memory>
 #include <tuple>
+#include "ljclus.cuh"
 #include "ljclus.h"
-#include "ljprune.cuh"
 #include "mmmol.h"
 #include "rebomol.h"
 #include "step.h"
@@ -173,10 +173,10 @@ int System::alloc_prune(double rc_lj) {
     LJPrune q;
     if (alloc(&q.cnt, n, (const int*)nullptr) || alloc(&q.list, (size_t)n * arr.in_cap, (const int*)nullptr) ||
         alloc(&q.sb, 3 * (size_t)n, (const double*)nullptr) ||
-        alloc(&q.words, 4 + 9, (const unsigned long long*)nullptr))
+        alloc(&q.words, 2 + 8 + 9, (const unsigned long long*)nullptr))
         return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
     q.stats = q.words + 2;
-    q.hb = reinterpret_cast<double*>(q.words + 4);
+    q.hb = reinterpret_cast<double*>(q.words + 10);
     q.n = n;
     q.stride = arr.in_cap;
     q.rc = rc_lj;
@@ -236,29 +236,28 @@ int System::alloc_clus(const double* pos_h) {
     return FMD_OK;
 }
 
-// The step's LJ term walks cluster rows when the tables exist, pruning is on,
-// no launch shape of the row gather is pinned and the initial cell takes them
-// (lj_clus_mode; a cell that stops doing so walks the full rows).
-// The margin keeps out small cells that may shrink to the limit; those are also
-// the ones (2 x 2 x 2 BCC) whose crystal comes apart within some thousand steps,
-// and in a gas of 1e18 K, which needs new rows on every evaluation, the row
-// gather takes 12 us where building cluster rows takes 35.
-void System::set_clus(bool allowed) {
-    const bool diag = h0[1] == 0.0 && h0[2] == 0.0 && h0[3] == 0.0 && h0[5] == 0.0 && h0[6] == 0.0 && h0[7] == 0.0;
-    const double edge = std::min(h0[0], std::min(h0[4], h0[8]));
-    arr.clus.on = allowed && arr.clus.perm && prune.delta > 0.0 && diag &&
-                  edge > 1.1 * (2.0 * (prune.rc + prune.delta) + 0.1);
+// The step's LJ term is the cluster gather when the tables exist, pruning is on,
+// no launch shape of the row gather is pinned and the cell h takes cluster rows
+// with the margin of wide_edge (lj_clus_mode; a cell that stops doing so, or whose
+// atoms move so fast that cluster rows do not pay, gets rows of atoms).
+void System::set_clus(bool allowed, const double* h) {
+    const bool diag = h[1] == 0.0 && h[2] == 0.0 && h[3] == 0.0 && h[5] == 0.0 && h[6] == 0.0 && h[7] == 0.0;
+    const double edge = std::min(h[0], std::min(h[4], h[8]));
+    arr.clus.on = allowed && arr.clus.perm && prune.delta > 0.0 && diag && edge > wide_edge();
+}
+
+// The edge above which a cell takes cluster rows until the next list build: the
+// gather's limit (lj_clus_mode) and what the barostat (edge rates clamped at
+// 0.005 A/fs) can shorten an edge by until then.
+double System::wide_edge() const {
+    return 2.0 * (prune.rc + prune.delta) + 0.2 + 0.01 * std::fabs(sp.dt) * p.nlup;
 }
 
 // Cell edges beyond which a rebuild leaves the full rows unbuilt (0: it builds
-// them): those the cluster gather takes, with a margin above what the barostat
-// (edge rates clamped at 0.005 A/fs) can shorten them by before the next one.
-// Where that does not hold (a cell that shears, steps that go on without a
-// rebuild), the gather builds the rows that it needs.
-double System::lazy_edge() const {
-    if (!arr.clus.on) return 0.0;
-    return 2.0 * (prune.rc + prune.delta) + 0.2 + 0.01 * std::fabs(sp.dt) * p.nlup;
-}
+// them).  Where the cell stops taking cluster rows before the next one after
+// all (it shears, or steps go on without a rebuild), the gather builds the
+// rows that it needs.
+double System::lazy_edge() const { return arr.clus.on ? wide_edge() : 0.0; }
 
 // The full rows of the last build, when the gather left them unbuilt.
 cudaError_t System::ensure_full_rows(cudaStream_t st) {
@@ -306,7 +305,7 @@ cudaError_t System::enqueue_rebuild(cudaStream_t st, bool lazy) {
     // none of its kernels.
     const int* gate = nullptr;
     if (mol.ok) {
-        if ((e = mol_partners(mol, arr.pos, hh, rc_a, st)) != cudaSuccess) return e;
+        if ((e = mol_partners(mol, arr.pos, hh, rc_a, st, arr.clus.on ? prune.stats : nullptr)) != cudaSuccess) return e;
         gate = mol.flag;
     }
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -476,7 +475,7 @@ LJShape System::pick_lj_shape(bool pruned, int& rc) {
 void System::set_lj_blocks() {
     const int ff = arr.kind == FMD_SYS_AIREBO ? FMD_FF_AIREBO : FMD_FF_MM;
     if (arr.clus.on) {
-        arr.lj_shape_p = LJShape{256, 4, 0, 1};       // reported: 256 threads, 4 atoms in flight, contiguous runs
+        arr.lj_shape_p = LJShape{lj_clus_threads(arr.precision), kClusG, 0, 1};   // reported: kClusG atoms a row, contiguous runs
         arr.lj_blocks = lj_clus_blocks(ff, arr.precision);
         return;
     }
@@ -548,8 +547,12 @@ int System::tune_lj() {
 int System::retune_lj() {
     if (lj_pinned) return FMD_OK;
     const bool was = arr.clus.on;
-    if (ensure_full_rows(ctx->stream) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "full rows failed");
-    set_clus(true);
+    double h[9];
+    if (ensure_full_rows(ctx->stream) != cudaSuccess ||
+        cudaMemcpyAsync(h, arr.S->h, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
+        cudaStreamSynchronize(ctx->stream) != cudaSuccess)
+        return ctx->fail(FMD_ERR_CUDA, "full rows failed");
+    set_clus(true, h);
     if (arr.clus.on == was) return FMD_OK;
     if (arr.clus.on) {
         set_lj_blocks();
@@ -596,7 +599,7 @@ int System::init() {
     // Pre-loop order of the reference: lists from the unwrapped positions,
     // then apply_pbc, then the first forces (LJ:813-828, AI:830-853).
     if (std::getenv("FMD_LJ_SHAPE")) lj_pinned = true;
-    set_clus(!lj_pinned);
+    set_clus(!lj_pinned, h0);
     if (enqueue_rebuild(st) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "list build launch failed");
     full_rows_stale = arr.clus.on;
     if (apply_pbc_launch(arr.pos, arr.n, arr.S->h, st) != cudaSuccess) return ctx->fail(FMD_ERR_CUDA, "apply_pbc failed");
@@ -1179,6 +1182,7 @@ extern "C" int fmd_system_kernel_ms(fmd_system* s, int stage, int reps, double* 
     cudaStream_t st = y.ctx->stream;
     const StepArrays& a = y.arr;
     const double* hh = a.S->h;
+    int walk = CLUS_WALK;                // stage 4
     auto launch = [&]() -> cudaError_t {
         switch (stage) {
             case 0:
@@ -1209,7 +1213,7 @@ extern "C" int fmd_system_kernel_ms(fmd_system* s, int stage, int reps, double* 
                 if (a.clus.on)
                     return lj_clus_launch(a.kind == FMD_SYS_AIREBO ? FMD_FF_AIREBO : FMD_FF_MM, a.clus, a.pos, hh,
                                           a.n, a.Facc, a.Facc, a.part_f2, st, a.precision, lj_prune_out(*a.prune), 0,
-                                          2);
+                                          walk);
                 return lj_gather_launch(a.kind == FMD_SYS_AIREBO ? FMD_FF_AIREBO : FMD_FF_MM, a.pos, hh, a.cnt_a,
                                         a.list_a, a.cap_a, a.prune->cnt, a.prune->list, a.in_cap, a.n, a.Facc,
                                         a.Facc, a.part_f2, st, a.precision, a.lj_shape_p, a.err);
@@ -1222,13 +1226,19 @@ extern "C" int fmd_system_kernel_ms(fmd_system* s, int stage, int reps, double* 
                 return enqueue_forces(a, st);
         }
     };
-    // stage 4 walks the rows as they are: of this system's gather
+    // stage 4 walks the rows as they are: of this system's gather, which builds
+    // its own first where the memory holds others
     if (stage == 4 && a.prune) {
-        unsigned long long kind = 0;
-        if (cudaMemcpyAsync(&kind, a.prune_umax + 1, sizeof(kind), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess)
-            return y.ctx->fail(FMD_ERR_CUDA, "kernel timing: read failed");
-        if (kind != fmd::lj_rows_tag(a.clus.on ? fmd::kRowsClusters : fmd::kRowsAtoms, a.prune_delta)) {
+        for (int pass = 0; pass < 2; pass++) {
+            unsigned long long kind = 0;
+            if (cudaMemcpyAsync(&kind, a.prune_umax + 1, sizeof(kind), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                cudaStreamSynchronize(st) != cudaSuccess)
+                return y.ctx->fail(FMD_ERR_CUDA, "kernel timing: read failed");
+            const bool clusters = kind == fmd::lj_rows_tag(fmd::kRowsClusters, a.prune_delta);
+            walk = clusters ? CLUS_WALK : ATOMS_WALK;
+            if (a.clus.on ? clusters || kind == fmd::lj_rows_tag(fmd::kRowsAtoms, a.prune_delta)
+                          : kind == fmd::lj_rows_tag(fmd::kRowsAtoms, a.prune_delta))
+                break;
             enqueue_forces(a, st);
             enqueue_force_reduce(a, st);
         }
@@ -1288,7 +1298,7 @@ extern "C" int fmd_system_set_lj_shape(fmd_system* s, int threads, int unroll, i
     if (y.initialized && y.ensure_full_rows(y.ctx->stream) != cudaSuccess)
         return y.ctx->fail(FMD_ERR_CUDA, "full rows failed");
     y.lj_pinned = true;
-    y.set_clus(false);                   // the pinned row gather; the memory it shares with the cluster rows is stale
+    y.arr.clus.on = 0;                   // the pinned row gather; the memory it shares with the cluster rows is stale
     if (y.prune.ok && lj_prune_mark(y.prune, y.ctx->stream) != cudaSuccess)
         return y.ctx->fail(FMD_ERR_CUDA, "prune mark failed");
     y.arr.lj_shape = sh;
@@ -1346,6 +1356,17 @@ extern "C" int fmd_system_lj_prune(fmd_system* s, double* delta, long long* eval
     }
     if (evaluations) *evaluations = (long long)st[0];
     if (prunes) *prunes = (long long)st[1];
+    return FMD_OK;
+}
+
+extern "C" int fmd_system_lj_gathers(fmd_system* s, long long counts[4]) {
+    if (!s || !s->sys || !counts) return FMD_ERR_ARG;
+    fmd::System& y = *s->sys;
+    unsigned long long n[4] = {0ull, 0ull, 0ull, 0ull};
+    if (y.prune.ok && (cudaStreamSynchronize(y.ctx->stream) != cudaSuccess ||
+                       cudaMemcpy(n, y.prune.stats + 4, sizeof(n), cudaMemcpyDeviceToHost) != cudaSuccess))
+        return y.ctx->fail(FMD_ERR_CUDA, "fmd_system_lj_gathers: read failed");
+    for (int k = 0; k < 4; k++) counts[k] = (long long)n[k];
     return FMD_OK;
 }
 

@@ -50,7 +50,8 @@ struct System {
     int alloc_clus(const double* pos);
     double lazy_edge() const;
     cudaError_t ensure_full_rows(cudaStream_t st);
-    void set_clus(bool allowed);
+    void set_clus(bool allowed, const double* h);
+    double wide_edge() const;
     int retune_lj();
     int upload_topology(const fmd_mm_topology* t, const int* mol_id);
     int upload_template(const fmd_mm_topology* t, int copies, int nmol, int natom);

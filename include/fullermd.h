@@ -383,6 +383,12 @@ int fmd_system_lj_shape_pruned(fmd_system *s, int *threads, int *unroll, int *fe
  * evaluations and of prunes among them since set-up. */
 int fmd_system_set_lj_prune(fmd_system *s, double delta);
 int fmd_system_lj_prune(fmd_system *s, double *delta, long long *evaluations, long long *prunes);
+
+/* Force evaluations since set-up by the rows the LJ gather walked: counts[0]
+ * rows of single atoms, pruned in that evaluation, [1] as the last prune left
+ * them, [2], [3] likewise rows of clusters of atoms (equal contiguous molecules
+ * of 32-64 atoms in a wide diagonal cell whose atoms do not move too fast). */
+int fmd_system_lj_gathers(fmd_system *s, long long counts[4]);
 int fmd_system_set_lj_shape(fmd_system *s, int threads, int unroll, int feed);
 int fmd_system_step_kernels(fmd_system *s, int rebuild, int phase, int *nkernels);
 /* Rigid systems: the number of site pairs within the LJ cutoff in the
