@@ -1,5 +1,6 @@
-// rebo_row.cuh -- REBO bonds of one list row straight from positions, and the
-// functions that every REBO kernel shares (airebo.cu, rebomol.cu).
+// rebo_row.cuh -- REBO bonds of one list row straight from positions
+// (airebo.cu), and the functions that every REBO kernel shares (airebo.cu,
+// rebomol.cu).
 #pragma once
 #include "rebo_fn.cuh"
 
