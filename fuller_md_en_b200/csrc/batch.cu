@@ -44,7 +44,8 @@ struct Tune {
     double lj_ms = 0, f1_ms = 0;
 };
 
-using TuneKey = std::tuple<int, int, long long, bool>;
+// device, replicas, atoms, and which kernels: bonded terms by molecules, cluster gather, precision
+using TuneKey = std::tuple<int, int, long long, bool, bool, int>;
 std::map<TuneKey, Tune>& tune_cache() {
     static std::map<TuneKey, Tune> m;
     return m;
@@ -263,7 +264,7 @@ struct fmd_batch {
 
     int autotune() {
         const int dev = ctx->device;
-        const auto key = std::make_tuple(dev, R, natoms, bd.mol_smem > 0);
+        const TuneKey key{dev, R, natoms, bd.mol_smem > 0, bd.lj_clus != 0, bd.precision};
         auto it = tune_cache().find(key);
         if (it != tune_cache().end()) {
             tune = it->second;
@@ -277,7 +278,7 @@ struct fmd_batch {
         for (System* s : sys) can_stage = can_stage && s->arr.in_cap == sys[0]->arr.in_cap;
         // cluster rows have one launch shape
         if (bd.lj_clus) {
-            best.lj_threads = 256; best.lj_unroll = kClusG; best.lj_apb = kClusAtomsPerBlock; best.lj_staged = 0;
+            best.lj_threads = lj_clus_threads(bd.precision); best.lj_unroll = kClusG; best.lj_apb = kClusAtomsPerBlock; best.lj_staged = 0;
             int rc = set_offsets(best);
             if (rc) return rc;
             best.lj_ms = time_ms(3, [&]() { return batch_lj_clus_launch(dA, bd.off_lj, R, bd.nblk_lj, bd.precision, st); });
