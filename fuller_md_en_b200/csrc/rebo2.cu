@@ -498,10 +498,11 @@ k_rebo2_bonds(const double* __restrict__ pos, const double* __restrict__ hh, con
 // The LJ pairs closer than 2^(1/6) sigma (where the switch acts), compacted
 // from the half rows: a warp per atom, kScanU slices of 32 entries in flight.
 // The distance is FP32 (its square off by less than 0.006 A^2 where it is used:
-// cell edges below 2048 A, half the narrowest beyond the radius by 1 A) with a
-// margin: the switch is zero for the few pairs that the margin adds.  30,000
-// atoms: 42 us; 79 us with a thread per slot of the table (occupied or
-// not), a 64-bit division to find its atom and the FP64 image of every entry.
+// cell edges below 2048 A, half the narrowest beyond the radius by 1 A); the
+// FP64 test decides within 0.01 A^2 of the radius, so the list holds no pair
+// more than the room for it was counted for.  30,000 atoms: 42 us; 79 us with a
+// thread per slot of the table (occupied or not), a 64-bit division to find its
+// atom and the FP64 image of every entry.
 constexpr int kScanU = 4;
 
 __global__ void __launch_bounds__(256)
@@ -520,7 +521,7 @@ k_lj_switch_scan(const double* __restrict__ pos, const double* __restrict__ hh, 
     const bool screen = diag && 0.5 * fmin(fabs(h[0]), fmin(fabs(h[4]), fabs(h[8]))) > sqrt(rmax2) + 1.0 &&
                         fmax(fabs(h[0]), fmax(fabs(h[4]), fabs(h[8]))) < 2048.0;
     const float L[3] = {(float)h[0], (float)h[4], (float)h[8]}, Li[3] = {(float)hi[0], (float)hi[4], (float)hi[8]};
-    const float far2 = (float)rmax2 + 0.01f;
+    const float near2 = (float)rmax2 - 0.01f, far2 = (float)rmax2 + 0.01f;
     const int lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
     for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < na; i += nw) {
         const int c = min(cnt_a[i], cap_a);
@@ -544,8 +545,9 @@ k_lj_switch_scan(const double* __restrict__ pos, const double* __restrict__ hh, 
                 dx = fmaf(-L[0], rintf(dx * Li[0]), dx);
                 dy = fmaf(-L[1], rintf(dy * Li[1]), dy);
                 dz = fmaf(-L[2], rintf(dz * Li[2]), dz);
-                bool take = j[u] >= 0 && !(screen && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > far2);
-                if (!screen && take) {
+                const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                bool take = j[u] >= 0 && !(screen && r2 > far2);
+                if (take && !(screen && r2 < near2)) {
                     double ex, ey, ez;
                     bond_vec(pos, i, j[u], h, hi, ex, ey, ez);
                     take = ex * ex + ey * ey + ez * ez < rmax2;
