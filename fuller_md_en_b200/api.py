@@ -570,10 +570,10 @@ class System:
     def lj_gathers(self) -> dict:
         """Force evaluations since set-up by the rows the LJ gather walked:
         of single atoms or of clusters, built in that evaluation or walked as
-        the last prune left them (fmd_system_lj_gathers)."""
-        n = (ctypes.c_longlong * 4)()
+        the last prune left them, or the full rows (fmd_system_lj_gathers)."""
+        n = (ctypes.c_longlong * 5)()
         self.ctx.check(self.ctx.lib.fmd_system_lj_gathers(self.h, n), "fmd_system_lj_gathers")
-        return dict(zip(("atoms_built", "atoms_walked", "clusters_built", "clusters_walked"), n))
+        return dict(zip(("atoms_built", "atoms_walked", "clusters_built", "clusters_walked", "full"), n))
 
     def use_surrogate(self, model, judge_every: int = 100, rmse_max: float = 0.025) -> None:
         """Learned REBO term from `model` (a surrogate.Surrogate, or None for

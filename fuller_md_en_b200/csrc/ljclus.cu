@@ -43,7 +43,10 @@
 // rows (atom_rows), with the pair terms of a chunk free of branches: with 12
 // warps an SM the chunk's independent chains stand in for the row gather's
 // warps.  30,000 atoms, pruning / walking: 126 / 66 us (the row gather 122 /
-// 67; with its branches here 155 / 82), FP32 pairs 132 / 72 (200 / 109).
+// 67; with its branches here 155 / 82), FP32 pairs 132 / 72 (200 / 109).  Where
+// nearly every evaluation prunes, the full rows are walked without writing
+// pruned ones, and the block's last atoms then split their rows over its warps:
+// 1,920 atoms 13.5 us instead of 16.7.
 //
 // Virial: sum over pairs of fm d (x) d with d = d0 - x_g, d0 the partner
 // from the cluster's first atom and x_g atom g from it, is
@@ -86,7 +89,7 @@ struct ClusShared {
     double shift[32][4];                       // image offsets of each code; from 27: far away
     int perm[64 + kClusG];                     // LJClus::perm (molecules of up to 64 atoms)
     double part[kMaxWarps][3 * kClusG];       // force sums of a row split over warps
-    double extra[kMaxWarps][kNV];              // {E, W} of full rows
+    double extra[kMaxWarps][kNV];              // {E, W} of rows of atoms
     unsigned cand[kMaxWarps][kCandMax];        // candidates of the row being built
 };
 
@@ -543,15 +546,18 @@ __device__ __noinline__ void build_full_row(const LJClus& c, int i, int lane) {
     __syncwarp();                                          // the row, before the warp's lanes read it
 }
 
-// Atoms i0 + w, i0 + w + (warps), ... below i1 over rows of their own, as the
-// row gather (airebo.cu): over the full rows, which it builds first where the
-// list build left them out, writing the pruned ones (prune), or over those of
-// the last prune.  F, and {E, W} added to the warp's record.  Apart from the
-// cluster walk, so that its registers are not the walk's.
+// The block's atoms i0 .. i1 - 1 over rows of their own, as the row gather
+// (airebo.cu): over the full rows, which it builds first where the list build
+// left them out, writing the pruned ones (ATOMS_PRUNE) or not (ATOMS_FULL), or
+// over those of the last prune.  Rounds of one atom per warp, then the remaining
+// atoms with their rows split over the warps where no row is written.  F, and
+// {E, W} into the warp's record.  Apart from the cluster walk, so that its
+// registers are not the walk's.
 template <bool FV, bool F32>
 __device__ __noinline__ void atom_rows(const LJClus& c, const double* __restrict__ pos, const double* hh, int i0,
                                        int i1, int w, double* __restrict__ F, double* __restrict__ Facc, LJP p,
-                                       const LJPruneOut& rows, bool prune, double* extra, int lane) {
+                                       const LJPruneOut& rows, int mode, double (*part)[3 * kClusG], double* extra,
+                                       int lane) {
     const double* h = hh;
     const double* hi = hh + 9;
     const bool diag = h[1] == 0.0 && h[2] == 0.0 && h[3] == 0.0 && h[5] == 0.0 && h[6] == 0.0 && h[7] == 0.0 &&
@@ -567,23 +573,34 @@ __device__ __noinline__ void atom_rows(const LJClus& c, const double* __restrict
     constexpr int U = kAtomUnroll;
     LJPruneOut po = rows;
     po.list = c.rows;
-    const int* cnt = prune ? c.full_cnt : po.cnt;
-    const int* list = prune ? c.full_list : c.rows;
-    if (!prune) po.cnt = nullptr;
-    const bool build = prune && c.flag[2] != 0;
-    for (int i = i0 + w; i < i1; i += kWarps<F32>) {
-        if (build) build_full_row(c, i, lane);
+    const int* cnt = mode == ATOMS_WALK ? po.cnt : c.full_cnt;
+    const int* list = mode == ATOMS_WALK ? c.rows : c.full_list;
+    if (mode != ATOMS_PRUNE) po.cnt = nullptr;
+    const bool build = mode == ATOMS_PRUNE && c.flag[2] != 0;
+    constexpr int W = kWarps<F32>;
+    const int whole = (i1 - i0) / W * W, rest = i1 - i0 - whole;
+    const int split = mode != ATOMS_PRUNE && rest > 0 ? W / rest : 1;
+    for (int r = 0; r <= whole; r += W) {
+        const bool tail = r == whole;
+        if (tail && rest == 0) break;
+        const int sp = tail ? split : 1, kk = w / sp, first = w - kk * sp;
+        const bool mine = !tail || kk < rest;
+        const int i = mine ? i0 + r + kk : i0;
+        if (build && mine) build_full_row(c, i, lane);
         const double px = pos[3 * i], py = pos[3 * i + 1], pz = pos[3 * i + 2];
         const LJAcc fa = lj_acc_load(Facc, i, lane);
         double fx = 0.0, fy = 0.0, fz = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
-        const int tot = min(cnt[i], c.full_cap);
+        const int tot = mine ? min(cnt[i], c.full_cap) : 0;
         const int* row = list + (size_t)i * c.full_cap;
         int* prow = c.rows + (size_t)i * c.full_cap;
         int pc = 0;
         int jj[U];                                         // indices one chunk ahead
 #pragma unroll
-        for (int u = 0; u < U; u++) jj[u] = lane + 32 * u < tot ? row[lane + 32 * u] : -1;
-        for (int b0 = 0; b0 < tot; b0 += 32 * U) {
+        for (int u = 0; u < U; u++) {
+            const int k = 32 * (U * first + u) + lane;
+            jj[u] = k < tot ? row[k] : -1;
+        }
+        for (int b0 = 32 * U * first; b0 < tot; b0 += 32 * U * sp) {
             int jc[U];
             double cx[U], cy[U], cz[U];
 #pragma unroll
@@ -594,7 +611,7 @@ __device__ __noinline__ void atom_rows(const LJClus& c, const double* __restrict
             }
 #pragma unroll
             for (int u = 0; u < U; u++) {
-                const int k = b0 + 32 * (U + u) + lane;
+                const int k = b0 + 32 * (U * sp + u) + lane;
                 jj[u] = k < tot ? row[k] : -1;
             }
             if (!wide) {
@@ -640,7 +657,19 @@ __device__ __noinline__ void atom_rows(const LJClus& c, const double* __restrict
                 }
             }
         }
-        lj_atom_done(i, fx - fs * sx, fy - fs * sy, fz - fs * sz, px, py, pz, hi, F, Facc, po, pc, lane, fa);
+        fx -= fs * sx; fy -= fs * sy; fz -= fs * sz;
+        if (sp == 1) {
+            if (mine) lj_atom_done(i, fx, fy, fz, px, py, pz, hi, F, Facc, po, pc, lane, fa);
+            continue;
+        }
+        fx = warp_sum(fx); fy = warp_sum(fy); fz = warp_sum(fz);
+        if (lane == 0) { part[w][0] = fx; part[w][1] = fy; part[w][2] = fz; }
+        __syncthreads();                                   // once: the tail is the last round
+        if (mine && first == 0 && lane == 0) {
+            for (int t = 1; t < sp; t++) { fx += part[w + t][0]; fy += part[w + t][1]; fz += part[w + t][2]; }
+            F[3 * i] = fa.x + fx; F[3 * i + 1] = fa.y + fy; F[3 * i + 2] = fa.z + fz;
+            if (Facc != F) { Facc[3 * i] = 0.0; Facc[3 * i + 1] = 0.0; Facc[3 * i + 2] = 0.0; }
+        }
     }
     acc[0] += F32 ? e : p.c4 * cc.s6 * e - p.vshift * np;
     acc[1] += fs * vir[0]; acc[5] += fs * vir[3]; acc[9] += fs * vir[5];
@@ -684,7 +713,7 @@ __device__ __forceinline__ void lj_clus_body(const LJClus& c, const double* __re
     for (int k = 0; k < 6; k++) s.w[k] = 0.0;
     if (lj_clus_kind(mode) == kRowsAtoms) {
         const int i0 = (int)((long long)blk * na / nblk), i1 = (int)((long long)(blk + 1) * na / nblk);
-        atom_rows<FV, F32>(c, pos, sh.hh, i0, i1, w, F, Facc, p, po, lj_clus_prunes(mode), sh.extra[w], lane);
+        atom_rows<FV, F32>(c, pos, sh.hh, i0, i1, w, F, Facc, p, po, mode, sh.part, sh.extra[w], lane);
     } else {
         __syncthreads();                       // image offsets, clusters
         if (mode == CLUS_PRUNE)

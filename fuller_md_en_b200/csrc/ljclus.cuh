@@ -8,11 +8,11 @@
 namespace fmd {
 
 // Rows of atoms or of clusters; built from the lists now, or walked as the last
-// prune left them.
-enum LJClusMode { ATOMS_PRUNE = 0, ATOMS_WALK = 1, CLUS_PRUNE = 2, CLUS_WALK = 3 };
+// prune left them; the full rows of atoms as they are.
+enum LJClusMode { ATOMS_PRUNE = 0, ATOMS_WALK = 1, CLUS_PRUNE = 2, CLUS_WALK = 3, ATOMS_FULL = 4, LJ_MODES = 5 };
 __device__ __forceinline__ bool lj_clus_prunes(int mode) { return mode == ATOMS_PRUNE || mode == CLUS_PRUNE; }
 __device__ __forceinline__ unsigned long long lj_clus_kind(int mode) {
-    return mode == ATOMS_PRUNE || mode == ATOMS_WALK ? kRowsAtoms : kRowsClusters;
+    return mode == CLUS_PRUNE || mode == CLUS_WALK ? kRowsClusters : kRowsAtoms;
 }
 
 // Cluster rows need the molecule builder's bitmaps, a diagonal cell and edges
@@ -27,6 +27,7 @@ __device__ __forceinline__ int lj_clus_mode(const LJClus& c, const unsigned long
     const double edge = fmin(hh[0], fmin(hh[4], hh[8]));
     const bool clusters = built && diag && edge > 2.0 * (rc + delta) + 0.1;
     const bool stale = lj_prune_needed(words, hh, hb, delta, rc, clusters ? kRowsClusters : kRowsAtoms);
+    if (c.flag[3] > 1 && c.flag[2] == 0) return ATOMS_FULL;
     return clusters ? (stale ? CLUS_PRUNE : CLUS_WALK) : (stale ? ATOMS_PRUNE : ATOMS_WALK);
 }
 

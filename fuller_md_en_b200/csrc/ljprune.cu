@@ -23,6 +23,7 @@
 // the evaluation pruned.  A list build marks the next evaluation as a prune.
 #include <cmath>
 
+#include "ljclus.cuh"
 #include "ljprune.h"
 
 namespace fmd {
@@ -36,7 +37,7 @@ cudaError_t lj_prune_clear(const LJPrune& p, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(p.cnt, 0, sizeof(int) * p.n, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(p.sb, 0, sizeof(double) * 3 * p.n, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(p.hb, 0, sizeof(double) * 9, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p.stats, 0, sizeof(unsigned long long) * 8, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(p.stats, 0, sizeof(unsigned long long) * (4 + LJ_MODES), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(p.words, 0x7F, sizeof(unsigned long long), st);
     return e;
 }

@@ -21,7 +21,7 @@ struct LJPrune {
     double* sb = nullptr;         // [3 n] fractional positions at the last prune
     double* hb = nullptr;         // [9] cell at the last prune
     unsigned long long* words = nullptr;  // [2] bits of the largest displacement since the last prune, kind of rows
-    unsigned long long* stats = nullptr;  // [8] {force evaluations, prunes}, both at the last list build, evaluations by LJClusMode
+    unsigned long long* stats = nullptr;  // [4 + LJ_MODES] {force evaluations, prunes}, both at the last list build, evaluations by LJClusMode
 };
 
 // Displacement bound that forces the next evaluation to prune (~1.4e306 A).

@@ -153,14 +153,16 @@ __global__ void k_mol_pairs(const double* __restrict__ hh, int M, const double* 
     mol_pairs_body(hh, M, cen, rad, rc, pmax, npart, part, flag, blockIdx.x);
 }
 
-// Whether the LJ gather walks rows of atoms until the next build: when more
-// than a quarter of the evaluations since the last build pruned because atoms
-// had moved (the first one after a build prunes anyway).  us per evaluation
-// over cluster rows, walk / prune, and over rows of atoms, with the full rows a
-// build then makes (FP64, molecules heating up): 1,920 atoms 8 / 32 and 12 /
-// 16 + 20 a build, 30,000 atoms 40 / 185 and 66 / 126 + 65, 122,880 atoms 160 /
-// 720 and 300 / 485 + 243; with a build every 20 steps these meet at 3, 6 and 7
-// such prunes between two builds.
+// Which rows the LJ gather walks until the next build.  Of atoms, when more than
+// a quarter of the evaluations since the last build pruned because atoms had
+// moved (the first one after a build prunes anyway).  us per evaluation over
+// cluster rows, walk / prune, and over rows of atoms, with the full rows a build
+// then makes (FP64, molecules heating up): 1,920 atoms 8 / 32 and 12 / 16 + 20 a
+// build, 30,000 atoms 40 / 185 and 66 / 126 + 65, 122,880 atoms 160 / 720 and 300
+// / 485 + 243; with a build every 20 steps these meet at 3, 6 and 7 such prunes
+// between two builds.  When nearly every evaluation pruned, the full rows are
+// walked as they are for kFullBuilds builds, then the prunes are counted again.
+constexpr int kFullBuilds = 8;
 __device__ __forceinline__ void rows_decide(unsigned long long* stats, int* flag) {
     if (!stats) {
         flag[3] = 0;
@@ -168,7 +170,8 @@ __device__ __forceinline__ void rows_decide(unsigned long long* stats, int* flag
     }
     const unsigned long long n = stats[0] - stats[2], p = stats[1] - stats[3];
     if (n == 0) return;                    // no evaluation since the last build
-    flag[3] = 4 * (p - (p > 0)) > n ? 1 : 0;
+    if (flag[3] > 1) flag[3]--;
+    else flag[3] = 10 * p >= 9 * n && n > 4 ? 1 + kFullBuilds : (4 * (p - (p > 0)) > n ? 1 : 0);
     stats[2] = stats[0];
     stats[3] = stats[1];
 }

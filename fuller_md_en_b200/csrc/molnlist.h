@@ -31,7 +31,7 @@ struct MolLists {
     int* npart = nullptr;     // [M] partner count
     int* part = nullptr;      // [M * pmax] partners, ascending
     int* flag = nullptr;      // [4] {molecule path valid, partner overflow, full rows left unbuilt,
-                              //      LJ rows of atoms until the next build}
+                              //      LJ rows until the next build: 0 of clusters, 1 of atoms, above: of atoms, not pruned}
 };
 
 // Host set-up from the atoms' molecule ids; m.ok stays false (the cell-grid

@@ -173,10 +173,10 @@ int System::alloc_prune(double rc_lj) {
     LJPrune q;
     if (alloc(&q.cnt, n, (const int*)nullptr) || alloc(&q.list, (size_t)n * arr.in_cap, (const int*)nullptr) ||
         alloc(&q.sb, 3 * (size_t)n, (const double*)nullptr) ||
-        alloc(&q.words, 2 + 8 + 9, (const unsigned long long*)nullptr))
+        alloc(&q.words, 2 + 4 + LJ_MODES + 9, (const unsigned long long*)nullptr))
         return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
     q.stats = q.words + 2;
-    q.hb = reinterpret_cast<double*>(q.words + 10);
+    q.hb = reinterpret_cast<double*>(q.words + 2 + 4 + LJ_MODES);
     q.n = n;
     q.stride = arr.in_cap;
     q.rc = rc_lj;
@@ -1359,14 +1359,14 @@ extern "C" int fmd_system_lj_prune(fmd_system* s, double* delta, long long* eval
     return FMD_OK;
 }
 
-extern "C" int fmd_system_lj_gathers(fmd_system* s, long long counts[4]) {
+extern "C" int fmd_system_lj_gathers(fmd_system* s, long long counts[5]) {
     if (!s || !s->sys || !counts) return FMD_ERR_ARG;
     fmd::System& y = *s->sys;
-    unsigned long long n[4] = {0ull, 0ull, 0ull, 0ull};
+    unsigned long long n[LJ_MODES] = {};
     if (y.prune.ok && (cudaStreamSynchronize(y.ctx->stream) != cudaSuccess ||
                        cudaMemcpy(n, y.prune.stats + 4, sizeof(n), cudaMemcpyDeviceToHost) != cudaSuccess))
         return y.ctx->fail(FMD_ERR_CUDA, "fmd_system_lj_gathers: read failed");
-    for (int k = 0; k < 4; k++) counts[k] = (long long)n[k];
+    for (int k = 0; k < LJ_MODES; k++) counts[k] = (long long)n[k];
     return FMD_OK;
 }
 

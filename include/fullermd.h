@@ -378,7 +378,9 @@ int fmd_system_lj_shape_pruned(fmd_system *s, int *threads, int *unroll, int *fe
  * the gather walks the full rows and keeps each row's entries within
  * rc + delta, in row order; other steps walk those rows.  Every pair within
  * the cutoff stays in them, so the pairs and pair terms are the full rows'
- * (on non-diagonal cells every step prunes).  delta in A: 0 = off, default
+ * (on non-diagonal cells every step prunes).  A system of equal molecules whose
+ * evaluations nearly all prune walks the full rows for some list builds without
+ * pruning them (fmd_system_lj_gathers).  delta in A: 0 = off, default
  * 0.5.  fmd_system_lj_prune reports delta and the numbers of force
  * evaluations and of prunes among them since set-up. */
 int fmd_system_set_lj_prune(fmd_system *s, double delta);
@@ -387,8 +389,10 @@ int fmd_system_lj_prune(fmd_system *s, double *delta, long long *evaluations, lo
 /* Force evaluations since set-up by the rows the LJ gather walked: counts[0]
  * rows of single atoms, pruned in that evaluation, [1] as the last prune left
  * them, [2], [3] likewise rows of clusters of atoms (equal contiguous molecules
- * of 32-64 atoms in a wide diagonal cell whose atoms do not move too fast). */
-int fmd_system_lj_gathers(fmd_system *s, long long counts[4]);
+ * of 32-64 atoms in a wide diagonal cell whose atoms do not move too fast), [4]
+ * the full rows, not pruned because nearly every evaluation had to.  Not counted
+ * with pruning off. */
+int fmd_system_lj_gathers(fmd_system *s, long long counts[5]);
 int fmd_system_set_lj_shape(fmd_system *s, int threads, int unroll, int feed);
 int fmd_system_step_kernels(fmd_system *s, int rebuild, int phase, int *nkernels);
 /* Rigid systems: the number of site pairs within the LJ cutoff in the

@@ -68,9 +68,29 @@ def test_fast_atoms_get_rows_of_atoms(ctx, oracle, T, prec):
         _matches_oracle(oracle, y, prec, g)
     n = y.lj_gathers()
     assert n["clusters_built"] >= 3 and n["clusters_built"] + n["clusters_walked"] == 10, n   # until the first build
-    assert n["atoms_built"] >= 5 and n["atoms_walked"] >= (3 if T < 1e5 else 0), n
+    if T < 1e5:
+        assert n["atoms_built"] >= 5 and n["atoms_walked"] >= 3 and n["full"] == 0, n
+    else:                                            # every evaluation pruned: not any more
+        assert n["full"] == 16 and n["atoms_built"] + n["atoms_walked"] == 0, n
     assert sum(n.values()) == 26 and n["atoms_built"] + n["clusters_built"] == y.lj_prune()["prunes"]
     y.close()
+
+
+def test_prunes_are_counted_again(ctx, oracle):
+    """Eight builds of full rows, then one of pruned rows, and so on."""
+    y = _gas(ctx, 2, 6e5, seed=6)
+    y.init()
+    seen = []
+    for g in range(1, 221):
+        y.run(g, g)
+        if g % 10 == 5:
+            before = y.lj_gathers()
+            y.run(g + 1000000, g + 1000000)          # a step more, no build
+            after = y.lj_gathers()
+            seen.append([k for k in after if after[k] > before[k]][0])
+            _matches_oracle(oracle, y, FMD_PREC_FP64, g)
+    y.close()
+    assert seen[1:9] == ["full"] * 8 and seen[9] == "atoms_built" and seen[10:18] == ["full"] * 8, seen
 
 
 def test_slow_atoms_keep_clusters(ctx):
@@ -91,7 +111,7 @@ def test_batch_chooses_by_replica(ctx, oracle):
     b.close()
     cold, hot = (y.lj_gathers() for y in reps)
     assert cold["atoms_built"] + cold["atoms_walked"] == 0 and cold["clusters_walked"] > 15, cold
-    assert hot["atoms_built"] >= 5, hot
+    assert hot["full"] == 16, hot
     for y in reps:
         y.close()
 
