@@ -75,7 +75,10 @@ template <bool F32> constexpr int kWarps = F32 ? 8 : 12;
 template <bool F32> constexpr int kBlocks = F32 ? 2 : 1;
 constexpr int kMaxWarps = 12;
 constexpr int kAtomUnroll = 4;             // entries per lane in flight of rows of atoms
-constexpr int kClusUnroll = 2;             // slices per trip: saves the feed's register moves (142 -> 138 us)
+// Slices per trip: saves the feed's register moves.  1 / 2 / 4, walk in us: FP64
+// 30,000 atoms 37.8 / 37.9 / 37.2, 122,880 atoms 141 / 141 / 136.5, 16 replicas of
+// 215,000 in all (a step) 500 / 492 / 462; FP32 pairs 44.8 / 42.9 / 43.8.
+template <bool F32> constexpr int kClusUnroll = F32 ? 2 : 4;
 constexpr int kMaskBit = 22, kCodeBit = 27;
 constexpr unsigned kAtomBits = (1u << kMaskBit) - 1u;
 static_assert(kClusG <= kCodeBit - kMaskBit, "mask bits of a row entry");
@@ -89,8 +92,17 @@ struct ClusShared {
     double shift[32][4];                       // image offsets of each code; from 27: far away
     int perm[64 + kClusG];                     // LJClus::perm (molecules of up to 64 atoms)
     double part[kMaxWarps][3 * kClusG];       // force sums of a row split over warps
-    double extra[kMaxWarps][kNV];              // {E, W} of rows of atoms
     unsigned cand[kMaxWarps][kCandMax];        // candidates of the row being built
+};
+
+// What an evaluation is of (the kernel's parameter; of a batch, in shared memory).
+struct ClusArgs {
+    LJClus c;
+    LJPruneOut po;
+    LJP p;
+    const double *pos, *hh;
+    double *F, *Facc, *part;
+    int na, nrec, mode;
 };
 
 // The cluster's atoms (-1: none) and their positions: the first absolute, the
@@ -440,7 +452,8 @@ template <bool FV, bool F32, bool OWN>
 __device__ __forceinline__ void clus_slices(const double* __restrict__ pos, int n, int step, ClusFeed& f,
                                             const Cluster& q, const double (*shift)[4], const LJP& p, const LJF& pf,
                                             const ClusConst& cc, ClusSum& s) {
-#pragma unroll kClusUnroll
+    constexpr int unroll = kClusUnroll<F32>;
+#pragma unroll unroll
     for (int t = 0; t < n; t++) {
         const unsigned ec = f.e1;
         const double cx = f.x, cy = f.y, cz = f.z;
@@ -551,15 +564,20 @@ __device__ __noinline__ void build_full_row(const LJClus& c, int i, int lane) {
 // left them out, writing the pruned ones (ATOMS_PRUNE) or not (ATOMS_FULL), or
 // over those of the last prune.  Rounds of one atom per warp, then the remaining
 // atoms with their rows split over the warps where no row is written.  F, and
-// {E, W} into the warp's record.  Apart from the cluster walk, so that its
-// registers are not the walk's.
+// {E, W} into the block's record.  All of the block's work, called with nothing
+// left to do: values kept across the call would cost the cluster walk registers
+// (2 % of its time).
 template <bool FV, bool F32>
-__device__ __noinline__ void atom_rows(const LJClus& c, const double* __restrict__ pos, const double* hh, int i0,
-                                       int i1, int w, double* __restrict__ F, double* __restrict__ Facc, LJP p,
-                                       const LJPruneOut& rows, int mode, double (*part)[3 * kClusG], double* extra,
-                                       int lane) {
-    const double* h = hh;
-    const double* hi = hh + 9;
+__device__ __noinline__ void atom_rows(const ClusArgs& a, int blk, int nblk, int mode, ClusShared& sh) {
+    const LJClus& c = a.c;
+    const LJP p = a.p;
+    const double* __restrict__ pos = a.pos;
+    double *F = a.F, *Facc = a.Facc;
+    const int i0 = (int)((long long)blk * a.na / nblk), i1 = (int)((long long)(blk + 1) * a.na / nblk);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const double* h = sh.hh;
+    const double* hi = sh.hh + 9;
+    double (*part)[3 * kClusG] = sh.part;
     const bool diag = h[1] == 0.0 && h[2] == 0.0 && h[3] == 0.0 && h[5] == 0.0 && h[6] == 0.0 && h[7] == 0.0 &&
                       hi[1] == 0.0 && hi[2] == 0.0 && hi[3] == 0.0 && hi[5] == 0.0 && hi[6] == 0.0 && hi[7] == 0.0;
     const bool wide = diag && 0.25 * fmin(h[0] * h[0], fmin(h[4] * h[4], h[8] * h[8])) > p.rc2 * (1.0 + 1e-9);
@@ -571,7 +589,7 @@ __device__ __noinline__ void atom_rows(const LJClus& c, const double* __restrict
 #pragma unroll
     for (int k = 0; k < kNV; k++) acc[k] = 0.0;
     constexpr int U = kAtomUnroll;
-    LJPruneOut po = rows;
+    LJPruneOut po = a.po;
     po.list = c.rows;
     const int* cnt = mode == ATOMS_WALK ? po.cnt : c.full_cnt;
     const int* list = mode == ATOMS_WALK ? c.rows : c.full_list;
@@ -675,11 +693,7 @@ __device__ __noinline__ void atom_rows(const LJClus& c, const double* __restrict
     acc[1] += fs * vir[0]; acc[5] += fs * vir[3]; acc[9] += fs * vir[5];
     acc[2] += fs * vir[1]; acc[3] += fs * vir[2]; acc[6] += fs * vir[4];
     lj_virial_mirror<FV>(acc);
-#pragma unroll
-    for (int k = 0; k < kNV; k++) {
-        const double t = warp_sum(acc[k]);
-        if (lane == 0) extra[k] = t;
-    }
+    block_sum_fields<kNV>(acc, sh.sm, a.part + (size_t)blk * kNV);
 }
 
 // Block blk of nblk: its run of clusters.  Rounds of one cluster per warp,
@@ -688,16 +702,23 @@ __device__ __noinline__ void atom_rows(const LJClus& c, const double* __restrict
 // 30,000 atoms; a system of 1,920 has fewer clusters than the GPU has
 // schedulers).
 template <bool FV, bool F32>
-__device__ __forceinline__ void lj_clus_body(const LJClus& c, const double* __restrict__ pos,
-                                             const double* __restrict__ hh, int na, double* __restrict__ F,
-                                             double* __restrict__ Facc, const LJP& p, double* __restrict__ part,
-                                             const LJPruneOut& po, int mode, int blk, int nblk, ClusShared& sh) {
+__device__ __forceinline__ void lj_clus_body(const ClusArgs& a, const LJP& p, int blk, int nblk, ClusShared& sh) {
+    const LJClus& c = a.c;
+    const LJPruneOut& po = a.po;
+    const double* __restrict__ pos = a.pos;
+    const double* __restrict__ hh = a.hh;
+    double* __restrict__ F = a.F;
+    double* __restrict__ Facc = a.Facc;
+    int mode = a.mode;
     constexpr int kClusWarps = kWarps<F32>, kClusThreads = 32 * kClusWarps;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x < 18) sh.hh[threadIdx.x] = hh[threadIdx.x];
-    if (lane < kNV) sh.extra[w][lane] = 0.0;
     __syncthreads();
     if (mode < 0) mode = lj_clus_mode(c, po.words, sh.hh, po.hb, po.delta, po.rc);
+    if (lj_clus_kind(mode) == kRowsAtoms) {
+        atom_rows<FV, F32>(a, blk, nblk, mode, sh);
+        return;
+    }
     if (threadIdx.x < 32) {
         const int t = threadIdx.x;
         sh.shift[t][0] = sh.hh[0] * (t < 27 ? t % 3 - 1 : 4);
@@ -711,108 +732,96 @@ __device__ __forceinline__ void lj_clus_body(const LJClus& c, const double* __re
     s.np = 0;
 #pragma unroll
     for (int k = 0; k < 6; k++) s.w[k] = 0.0;
-    if (lj_clus_kind(mode) == kRowsAtoms) {
-        const int i0 = (int)((long long)blk * na / nblk), i1 = (int)((long long)(blk + 1) * na / nblk);
-        atom_rows<FV, F32>(c, pos, sh.hh, i0, i1, w, F, Facc, p, po, mode, sh.part, sh.extra[w], lane);
-    } else {
-        __syncthreads();                       // image offsets, clusters
-        if (mode == CLUS_PRUNE)
-            for (int k = c0 + w; k < c1; k += kClusWarps) build_row(c, k, pos, sh, po, w, lane);
-        __syncthreads();                       // rows of this block
-        const double* x = mode == CLUS_PRUNE ? pos : c.upos;
-        const LJF pf{(float)p.sig2, (float)(p.sig2 - (double)(float)p.sig2), (float)p.c4, (float)p.c24};
-        const ClusConst cc{p.sig2 * p.sig2 * p.sig2, 2.0 * (p.sig2 * p.sig2 * p.sig2)};
-        const double fs = F32 ? 1.0 : p.c24 * cc.s6;
-        const int whole = (c1 - c0) / kClusWarps * kClusWarps, rest = c1 - c0 - whole;
-        const int split = rest > 0 ? kClusWarps / rest : 1;
-        for (int r = 0; r <= whole; r += kClusWarps) {
-            const bool tail = r == whole;
-            if (tail && rest == 0) break;
-            const int sp = tail ? split : 1;
-            const int kk = w / sp, first = w % sp;
-            const int k = c0 + r + kk;
-            const bool mine = !tail || kk < rest;
-            const int own = owner_atom(lane);
-            double fx = 0.0, fy = 0.0, fz = 0.0;
-            int io = -1;                       // atom this lane writes
-            LJAcc fa;
-            if (mine) {
-                const int4 n = c.cnt[k];
-                const Cluster q = load_cluster(c, k, n.z, x, sh);
+    __syncthreads();                       // image offsets, clusters
+    if (mode == CLUS_PRUNE)
+        for (int k = c0 + w; k < c1; k += kClusWarps) build_row(c, k, pos, sh, po, w, lane);
+    __syncthreads();                       // rows of this block
+    const double* x = mode == CLUS_PRUNE ? pos : c.upos;
+    const LJF pf{(float)p.sig2, (float)(p.sig2 - (double)(float)p.sig2), (float)p.c4, (float)p.c24};
+    const ClusConst cc{p.sig2 * p.sig2 * p.sig2, 2.0 * (p.sig2 * p.sig2 * p.sig2)};
+    const double fs = F32 ? 1.0 : p.c24 * cc.s6;
+    const int whole = (c1 - c0) / kClusWarps * kClusWarps, rest = c1 - c0 - whole;
+    const int split = rest > 0 ? kClusWarps / rest : 1;
+    for (int r = 0; r <= whole; r += kClusWarps) {
+        const bool tail = r == whole;
+        if (tail && rest == 0) break;
+        const int sp = tail ? split : 1;
+        const int kk = w / sp, first = w % sp;
+        const int k = c0 + r + kk;
+        const bool mine = !tail || kk < rest;
+        const int own = owner_atom(lane);
+        double fx = 0.0, fy = 0.0, fz = 0.0;
+        int io = -1;                       // atom this lane writes
+        LJAcc fa;
+        if (mine) {
+            const int4 n = c.cnt[k];
+            const Cluster q = load_cluster(c, k, n.z, x, sh);
 #pragma unroll
-                for (int g = 0; g < kClusG; g++)
-                    if (own == g) io = q.id[g];
-                if (io >= 0 && first == 0) { fa.x = Facc[3 * io]; fa.y = Facc[3 * io + 1]; fa.z = Facc[3 * io + 2]; }
+            for (int g = 0; g < kClusG; g++)
+                if (own == g) io = q.id[g];
+            if (io >= 0 && first == 0) { fa.x = Facc[3 * io]; fa.y = Facc[3 * io + 1]; fa.z = Facc[3 * io + 2]; }
 #pragma unroll
-                for (int g = 0; g < kClusG; g++) s.fx[g] = s.fy[g] = s.fz[g] = 0.0;
-                // slices first, first + sp, ...: the counting ones, then the others
-                const int nsl = (n.y + 31) >> 5, nown = n.x >> 5;
-                const int mine_all = nsl > first ? (nsl - first + sp - 1) / sp : 0;
-                const int mine_own = nown > first ? (nown - first + sp - 1) / sp : 0;
-                ClusFeed f;
-                f.row = c.rows + (size_t)k * c.stride;
-                f.end = n.y;
-                f.k = 32 * first + lane;
-                f.e1 = f.entry();
-                f.load(x);
-                f.k += 32 * sp;
-                f.e2 = f.entry();
-                clus_slices<FV, F32, true>(x, mine_own, 32 * sp, f, q, sh.shift, p, pf, cc, s);
+            for (int g = 0; g < kClusG; g++) s.fx[g] = s.fy[g] = s.fz[g] = 0.0;
+            // slices first, first + sp, ...: the counting ones, then the others
+            const int nsl = (n.y + 31) >> 5, nown = n.x >> 5;
+            const int mine_all = nsl > first ? (nsl - first + sp - 1) / sp : 0;
+            const int mine_own = nown > first ? (nown - first + sp - 1) / sp : 0;
+            ClusFeed f;
+            f.row = c.rows + (size_t)k * c.stride;
+            f.end = n.y;
+            f.k = 32 * first + lane;
+            f.e1 = f.entry();
+            f.load(x);
+            f.k += 32 * sp;
+            f.e2 = f.entry();
+            clus_slices<FV, F32, true>(x, mine_own, 32 * sp, f, q, sh.shift, p, pf, cc, s);
 #pragma unroll
-                for (int g = 1; g < kClusG; g++) {     // the virial's second part
-                    s.w[0] = fma(-q.x[g], s.fx[g], s.w[0]);
-                    if (FV) { s.w[1] = fma(-q.x[g], s.fy[g], s.w[1]); s.w[2] = fma(-q.x[g], s.fz[g], s.w[2]); }
-                    s.w[3] = fma(-q.y[g], s.fy[g], s.w[3]);
-                    if (FV) s.w[4] = fma(-q.y[g], s.fz[g], s.w[4]);
-                    s.w[5] = fma(-q.z[g], s.fz[g], s.w[5]);
+            for (int g = 1; g < kClusG; g++) {     // the virial's second part
+                s.w[0] = fma(-q.x[g], s.fx[g], s.w[0]);
+                if (FV) { s.w[1] = fma(-q.x[g], s.fy[g], s.w[1]); s.w[2] = fma(-q.x[g], s.fz[g], s.w[2]); }
+                s.w[3] = fma(-q.y[g], s.fy[g], s.w[3]);
+                if (FV) s.w[4] = fma(-q.y[g], s.fz[g], s.w[4]);
+                s.w[5] = fma(-q.z[g], s.fz[g], s.w[5]);
+            }
+            clus_slices<FV, F32, false>(x, mine_all - mine_own, 32 * sp, f, q, sh.shift, p, pf, cc, s);
+            clus_reduce(s, lane, fx, fy, fz);
+        }
+        if (sp > 1) {
+            if (own >= 0) {
+                sh.part[w][3 * own] = fx; sh.part[w][3 * own + 1] = fy; sh.part[w][3 * own + 2] = fz;
+            }
+            __syncthreads();
+            if (first == 0 && own >= 0)
+                for (int t = 1; t < sp; t++) {
+                    fx += sh.part[w + t][3 * own];
+                    fy += sh.part[w + t][3 * own + 1];
+                    fz += sh.part[w + t][3 * own + 2];
                 }
-                clus_slices<FV, F32, false>(x, mine_all - mine_own, 32 * sp, f, q, sh.shift, p, pf, cc, s);
-                clus_reduce(s, lane, fx, fy, fz);
-            }
-            if (sp > 1) {
-                if (own >= 0) {
-                    sh.part[w][3 * own] = fx; sh.part[w][3 * own + 1] = fy; sh.part[w][3 * own + 2] = fz;
-                }
-                __syncthreads();
-                if (first == 0 && own >= 0)
-                    for (int t = 1; t < sp; t++) {
-                        fx += sh.part[w + t][3 * own];
-                        fy += sh.part[w + t][3 * own + 1];
-                        fz += sh.part[w + t][3 * own + 2];
-                    }
-            }
-            if (io >= 0 && first == 0) {
-                F[3 * io] = fa.x - fs * fx;
-                F[3 * io + 1] = fa.y - fs * fy;
-                F[3 * io + 2] = fa.z - fs * fz;
-                if (Facc != F) { Facc[3 * io] = 0.0; Facc[3 * io + 1] = 0.0; Facc[3 * io + 2] = 0.0; }
-            }
+        }
+        if (io >= 0 && first == 0) {
+            F[3 * io] = fa.x - fs * fx;
+            F[3 * io + 1] = fa.y - fs * fy;
+            F[3 * io + 2] = fa.z - fs * fz;
+            if (Facc != F) { Facc[3 * io] = 0.0; Facc[3 * io + 1] = 0.0; Facc[3 * io + 2] = 0.0; }
         }
     }
     double acc[kNV];
-    const double s6 = p.sig2 * p.sig2 * p.sig2, fs = F32 ? 1.0 : p.c24 * s6;
-    acc[0] = F32 ? s.e : p.c4 * s6 * s.e - p.vshift * s.np;
+    acc[0] = F32 ? s.e : p.c4 * cc.s6 * s.e - p.vshift * s.np;
     acc[1] = fs * s.w[0]; acc[5] = fs * s.w[3]; acc[9] = fs * s.w[5];
     acc[2] = acc[4] = FV ? fs * s.w[1] : 0.0;
     acc[3] = acc[7] = FV ? fs * s.w[2] : 0.0;
     acc[6] = acc[8] = FV ? fs * s.w[4] : 0.0;
-    __syncwarp();
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < kNV; k++) acc[k] += sh.extra[w][k];
-    block_sum_fields<kNV>(acc, sh.sm, part + (size_t)blk * kNV);
+    block_sum_fields<kNV>(acc, sh.sm, a.part + (size_t)blk * kNV);
 }
 
 template <bool FV, bool F32>
 __global__ void __launch_bounds__(32 * kWarps<F32>, kBlocks<F32>)
-k_lj_clus(const __grid_constant__ LJClus c, const double* __restrict__ pos, const double* __restrict__ hh, int na,
-          double* __restrict__ F, double* __restrict__ Facc, LJP p, double* __restrict__ part,
-          const __grid_constant__ LJPruneOut po, int nrec, int mode) {
+k_lj_clus(const __grid_constant__ ClusArgs a) {
     FMD_PDL_WAIT();
     __shared__ ClusShared sh;
-    lj_clus_body<FV, F32>(c, pos, hh, na, F, Facc, p, part, po, mode, blockIdx.x, gridDim.x, sh);
+    lj_clus_body<FV, F32>(a, a.p, blockIdx.x, gridDim.x, sh);
     if (threadIdx.x < kNV)
-        for (int r = gridDim.x + blockIdx.x; r < nrec; r += gridDim.x) part[(size_t)r * kNV + threadIdx.x] = 0.0;
+        for (int r = gridDim.x + blockIdx.x; r < a.nrec; r += gridDim.x) a.part[(size_t)r * kNV + threadIdx.x] = 0.0;
 }
 
 // Replica batch (MM): block b serves replica r as its local block b - off[r].
@@ -820,20 +829,24 @@ template <bool F32>
 __global__ void __launch_bounds__(32 * kWarps<F32>, kBlocks<F32>)
 k_b_lj_clus(const StepArrays* __restrict__ As, const int* __restrict__ off, int R) {
     __shared__ ClusShared sh;
+    __shared__ ClusArgs args;
     const int r = batch_rep(off, R, blockIdx.x);
-    const StepArrays& a = As[r];
     const LJP p = lj_params_dev(FMD_FF_MM);
-    LJPruneOut po;
-    po.cnt = a.prune_cnt;
-    po.sb = const_cast<double*>(a.prune_sb);
-    const double rp = a.prune_rc + a.prune_delta;
-    po.r2 = rp * rp;
-    po.words = a.prune_umax;
-    po.hb = a.prune_hb;
-    po.delta = a.prune_delta;
-    po.rc = a.prune_rc;
-    lj_clus_body<false, F32>(a.clus, a.pos, a.S->h, a.n, a.F, a.Facc, p, a.part_f2, po, -1, blockIdx.x - off[r],
-                             off[r + 1] - off[r], sh);
+    if (threadIdx.x == 0) {
+        const StepArrays& a = As[r];
+        const double rp = a.prune_rc + a.prune_delta;
+        LJPruneOut po;
+        po.cnt = a.prune_cnt;
+        po.sb = const_cast<double*>(a.prune_sb);
+        po.r2 = rp * rp;
+        po.words = a.prune_umax;
+        po.hb = a.prune_hb;
+        po.delta = a.prune_delta;
+        po.rc = a.prune_rc;
+        args = ClusArgs{a.clus, po, p, a.pos, a.S->h, a.F, a.Facc, a.part_f2, a.n, 0, -1};
+    }
+    __syncthreads();
+    lj_clus_body<false, F32>(args, p, blockIdx.x - off[r], off[r + 1] - off[r], sh);
 }
 
 template <bool FV, bool F32>
@@ -865,7 +878,7 @@ cudaError_t lj_clus_launch(int ff, const LJClus& c, const double* pos, const dou
     const bool f32 = precision == FMD_PREC_FP32_PAIR;
     const dim3 grid(lj_clus_blocks(ff, precision)), block(lj_clus_threads(precision));
 #define FMD_CLUS(FV, F32)                                                                                            \
-    launch_pdl(k_lj_clus<FV, F32>, grid, block, 0, st, c, pos, hh, na, F, Facc, p, part, po, nrec, mode)
+    launch_pdl(k_lj_clus<FV, F32>, grid, block, 0, st, ClusArgs{c, po, p, pos, hh, F, Facc, part, na, nrec, mode})
     if (ff == FMD_FF_AIREBO) return f32 ? FMD_CLUS(true, true) : FMD_CLUS(true, false);
     return f32 ? FMD_CLUS(false, true) : FMD_CLUS(false, false);
 #undef FMD_CLUS

@@ -22,12 +22,13 @@ __device__ __forceinline__ unsigned long long lj_clus_kind(int mode) {
 // gather and by the step's reduction.
 __device__ __forceinline__ int lj_clus_mode(const LJClus& c, const unsigned long long* words, const double* hh,
                                             const double* hb, double delta, double rc) {
-    const bool built = c.flag[0] != 0 && c.flag[3] == 0;
+    const int4 flag = *reinterpret_cast<const int4*>(c.flag);      // with the loads of the bound
+    const bool built = flag.x != 0 && flag.w == 0;
     const bool diag = hh[1] == 0.0 && hh[2] == 0.0 && hh[3] == 0.0 && hh[5] == 0.0 && hh[6] == 0.0 && hh[7] == 0.0;
     const double edge = fmin(hh[0], fmin(hh[4], hh[8]));
     const bool clusters = built && diag && edge > 2.0 * (rc + delta) + 0.1;
     const bool stale = lj_prune_needed(words, hh, hb, delta, rc, clusters ? kRowsClusters : kRowsAtoms);
-    if (c.flag[3] > 1 && c.flag[2] == 0) return ATOMS_FULL;
+    if (flag.w > 1 && flag.z == 0) return ATOMS_FULL;
     return clusters ? (stale ? CLUS_PRUNE : CLUS_WALK) : (stale ? ATOMS_PRUNE : ATOMS_WALK);
 }
 
