@@ -137,16 +137,6 @@ def make_system(ctx, rank: int, precision=None):
     return s, na, cfg, npt
 
 
-def list_bytes(sysd, na):
-    """Algorithmic bytes of one LJ gather launch over the full rows and over
-    the pruned rows of the last prune: row entries read (int32), the row
-    lengths, positions of the atoms and their partners (FP64 x3, each atom
-    read once), F written, accumulator read and cleared."""
-    full, pruned = sysd.lj_rows()
-    fixed = na * 4 + na * 24 + 3 * na * 24
-    return (int(full.sum()) * 4 + fixed, int(pruned.sum()) * 4 + fixed, int(full.sum()), int(pruned.sum()))
-
-
 def timed_steps(ctx, stream, sysd, K, flush):
     """CUDA-event time (ms) of global steps 1..K of an initialised system,
     L2 flushed before each step outside its window."""
@@ -214,24 +204,27 @@ def run_ours(args, ws, rank, local):
     value = job_throughput(na, K, ms_total, ws)
 
     # ---------------- roofline of the dominant kernel ----------------
-    # The LJ gather over the pruned rows runs on most steps (the full-row
-    # gather only when the rows are pruned again), so it is the kernel whose
-    # roofline is reported.
-    stages = {"lj_gather_pruned": sysd.kernel_ms(4, 20), "lj_gather_full": sysd.kernel_ms(0, 20),
-              "rebo": sysd.kernel_ms(1, 20), "list_rebuild": sysd.kernel_ms(2, 5)}
+    # The LJ gather walking the cluster rows of the last prune runs on most
+    # steps (it builds them on the rest), so it is the kernel whose roofline is
+    # reported: FP64 instructions bound it, of 48 FLOP a pair within the cutoff.
+    gathers = sysd.lj_gathers()
+    stages = {"lj_gather": sysd.kernel_ms(4, 20), "rebo": sysd.kernel_ms(1, 20),
+              "list_rebuild": sysd.kernel_ms(2, 5)}
     prune = sysd.lj_prune()
-    per_step = {"lj_gather_pruned": stages["lj_gather_pruned"], "lj_gather_full": stages["lj_gather_full"],
-                "lj_prune_fraction": prune["prunes"] / max(1, prune["evaluations"]), "rebo": stages["rebo"],
-                "list_rebuild": stages["list_rebuild"] / NLUP}
-    full_bytes, lj_bytes, n_full, n_pruned = list_bytes(sysd, na)
-    lj_shape = {"full_rows": sysd.lj_shape(), "pruned_rows": sysd.lj_shape_pruned()}
+    per_step = {"lj_gather": stages["lj_gather"], "lj_prune_fraction": prune["prunes"] / max(1, prune["evaluations"]),
+                "rebo": stages["rebo"], "list_rebuild": stages["list_rebuild"] / NLUP}
+    n_pruned = int(sysd.lj_rows()[1].sum())
+    lj_bytes = na * 24 + 3 * na * 24           # positions read; F written, accumulator read and cleared
+    lj_shape = sysd.lj_shape_pruned()
     peak, peak_src = peaks()
-    achieved = lj_bytes / (stages["lj_gather_pruned"] / 1e3) / 1e9
     traffic = None
     tfile = ROOT / "profiles" / "traffic.json"
     if tfile.exists():
-        traffic = json.loads(tfile.read_text()).get("k_lj_gather_pruned_nc5")
+        traffic = json.loads(tfile.read_text()).get("k_lj_clus_nc5")
     composite = composite_roofline(sysd, na, ms_total / K, stages, per_step, peak, peak_src, clk)
+    lj_flop = composite["kernels"]["lj"]["flop"]
+    fp64_peak = composite["kernels"]["lj"]["peak"]
+    achieved = lj_flop / (stages["lj_gather"] / 1e3) / 1e12
     n_prod = sysd.step_kernels(False, False)
     n_reb = sysd.step_kernels(True, False)
     launches = sum(n_reb if (1 + k) % NLUP == 0 else n_prod for k in range(K))
@@ -313,7 +306,7 @@ def run_ours(args, ws, rank, local):
     sys32 = System.airebo(ctx, cfg32, s["pos"], s["vel"], s["mass"], s["mol_id"], s["h"], npt)
     sys32.init()
     ms32 = float(sum(timed_steps(ctx, stream, sys32, K, flush)))
-    lj32_ms = sys32.kernel_ms(0, 20)
+    lj32_ms = sys32.kernel_ms(4, 20)
     sys32.close()
     value32 = ws * na * K / (ms32 / 1e3)
 
@@ -346,13 +339,12 @@ def run_ours(args, ws, rank, local):
                    "l2": "flushed between timed steps (512 MB write outside the timed windows); "
                          "working set ~75 MB < 126 MB L2",
                    "step_graph": "one CUDA graph per step variant", "wall_s_timed_loop": t_wall},
-        "roofline": {"bound": "hbm", "kernel": "k_lj_gather_staged over the pruned rows (atomistic LJ gather)",
-                     "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "peak_source": peak_src, "traffic": traffic,
-                     "algorithmic_bytes_per_launch": lj_bytes, "pruned_row_entries": n_pruned,
-                     "full_row_entries": n_full, "full_rows_bytes_per_launch": full_bytes,
-                     "launch_shape": lj_shape, "prune": prune,
-                     "launch_ms": stages["lj_gather_pruned"], "composite": composite},
+        "roofline": {"bound": "fp64 simt", "kernel": "k_lj_clus walking its cluster rows (atomistic LJ gather)",
+                     "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s", "frac": achieved / fp64_peak,
+                     "peak_source": composite["fp64_peak_source"], "traffic": traffic,
+                     "flop_per_launch": lj_flop, "bytes_per_launch_without_rows": lj_bytes,
+                     "pairs_in_rows": n_pruned, "launch_shape": lj_shape, "prune": prune,
+                     "evaluations_by_rows": gathers, "launch_ms": stages["lj_gather"], "composite": composite},
         "stage_ms_per_step": per_step,
         "gpu_launches": launches,
         "clocks": clk,
@@ -409,7 +401,7 @@ def composite_roofline(sysd, na, step_ms, stages, per_step, hbm_peak, hbm_src, c
     return {"frac": total / (step_ms * 1e3), "roofline_us_per_step": total, "step_us": step_ms * 1e3,
             "kernels": work, "fp64_peak_source": f"nominal (148 SMs x 64 FP64 FMA/clk x {sm_mhz:.0f} MHz)",
             "hbm_peak_source": hbm_src,
-            "lj_kernel_frac_fp64": (work["lj"]["flop"] / (stages["lj_gather_pruned"] * 1e-3)) / (fp64_peak * 1e12)}
+            "lj_kernel_frac_fp64": (work["lj"]["flop"] / (stages["lj_gather"] * 1e-3)) / (fp64_peak * 1e12)}
 
 
 def surrogate_nc8(ctx, stream, flush, model, K, judge, rmse_max):
@@ -470,7 +462,7 @@ def run_rigid(args, ctx, stream, flush, ws, rank, local):
            "workload": "rigid-body LJ, C60 FCC nc=10: 4,000 molecules / 240,000 sites, 300 K, 1 GPa, dt 1 fs, "
                        "molecule lists every 25 steps, FP32 site pairs with FP64 sums and integrator",
            "site_pair_kernel_ms": pair_ms,
-           "roofline": {"bound": "fp32 simt", "kernel": "k_rigid_w (site pairs)", "achieved": achieved,
+           "roofline": {"bound": "fp32 simt", "kernel": "k_rigid_pairs with its set-up and sums (each pair once)", "achieved": achieved,
                         "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
                         "peak_source": "nominal (148 SMs x 128 FP32 lanes x 2 x 1965 MHz)",
                         "site_pairs_in_cutoff": pairs, "flop_per_pair": 72}}
@@ -711,20 +703,20 @@ def run_stage(args):
     --reps launches of the stage with CUDA events (System.kernel_ms: one
     untimed launch first, then the timed ones, then the current forces are
     recomputed).  Stages of the AIREBO workload (C60 FCC --nc, default 5):
-    lj_full / lj_pruned (the LJ gather over the full / pruned rows), rebo,
-    rebuild, forces; "sg": the learned REBO term (a randomly initialised
-    model: its kernels' cost does not depend on the weights); "rigid": the
-    rigid site-pair kernel of C60 FCC --nc (default 10; 240,000 sites, 1 GPa,
-    FP32 site pairs).  FMD_LJ_SHAPE pins the LJ gather's launch shape
-    (threads, entries per lane, row feed) so the launch sequence does not
-    depend on the autotuner: with --stage-steps 0 and --reps 1 the LJ gather
-    launches are set-up's (one, pruning the full rows), the untimed and the
-    timed launch of the stage, then the recomputation's, so a profiler
+    lj_full (the row gather over the full rows, which pinned or small systems
+    run) / lj_pruned (the system's gather over the rows of its last prune:
+    cluster rows here), rebo, rebuild, forces; "sg": the learned REBO term (a
+    randomly initialised model: its kernels' cost does not depend on the
+    weights); "rigid": the rigid site-pair kernels of C60 FCC --nc (default 10;
+    240,000 sites, 1 GPa, FP32 site pairs).  With --stage-steps 0 and --reps 1
+    the LJ gather launches are set-up's (one, building the rows), the untimed
+    and the timed launch of the stage, then the recomputation's, so a profiler
     capturing the gather's launch 3 sees the timed, warm launch on the bench
-    state.  The REBO kernels launch twice per force evaluation (geometry +
-    bond order, forces).  "rebo2" / "lj_switch": the REBO-II term (coordination
-    and bond kernels) / the switched-LJ correction of the same workload with
-    both extensions on and synthetic spline knots.  Prints one JSON line."""
+    state.  FMD_LJ_SHAPE makes the system run the row gather in that launch
+    shape (threads, entries per lane, row feed) instead.  "rebo2" / "lj_switch":
+    the REBO-II term (coordination and bond kernels) / the switched-LJ
+    correction of the same workload with both extensions on and synthetic
+    spline knots.  Prints one JSON line."""
     from fuller_md_en_b200 import Context, RunConfig, System, crystal
     from fuller_md_en_b200._lib import FMD_PREC_FP32_PAIR
     ctx = Context(0)
@@ -765,8 +757,8 @@ def run_stage(args):
         ms = y.kernel_ms(STAGES[args.stage], args.reps)
         full, pruned = y.lj_rows()
         out = {"stage": args.stage, "ms_per_launch": ms, "atoms": na, "steps": args.stage_steps,
-               "shape": y.lj_shape(), "full_row_entries": int(full.sum()), "pruned_row_entries": int(pruned.sum()),
-               "prune": y.lj_prune()}
+               "shape": y.lj_shape_pruned(), "full_row_entries": int(full.sum()),
+               "pruned_row_entries": int(pruned.sum()), "prune": y.lj_prune(), "gathers": y.lj_gathers()}
         if model is not None:
             y.close()
             model.close()

@@ -486,45 +486,33 @@ __device__ __forceinline__ void clus_slices(const double* __restrict__ pos, int 
     }
 }
 
-// Sums the cluster's force over the warp.  With 4 (2) atoms the lanes first
-// split the atoms among themselves, so lanes 8 g (16 g) hold atom g's sum;
-// else every lane holds every sum and lane g stands for atom g.
-constexpr int kOwnerStep = kClusG == 4 ? 8 : (kClusG == 2 ? 16 : 1);
-__device__ __forceinline__ int owner_atom(int lane) {
-    const int g = lane / kOwnerStep;
-    return lane % kOwnerStep == 0 && g < kClusG ? g : -1;
-}
+// Sums the cluster's force over the warp: the lanes first split the atoms among
+// themselves, so lanes 8 g hold atom g's sum.
+static_assert(kClusG == 4, "lanes of an atom's sum");
+constexpr int kOwnerStep = 32 / kClusG;
+__device__ __forceinline__ int owner_atom(int lane) { return lane % kOwnerStep == 0 ? lane / kOwnerStep : -1; }
 __device__ __forceinline__ void swap_add(double& keep, double other, bool hi, int o) {
     const double send = hi ? keep : other;
     keep = (hi ? other : keep) + __shfl_xor_sync(kFull, send, o);
 }
 __device__ __forceinline__ void clus_reduce(ClusSum& s, int lane, double& fx, double& fy, double& fz) {
-    if (kClusG == 4 || kClusG == 2) {
-        int o = 16;
+    int o = 16;
 #pragma unroll
-        for (int half = kClusG / 2; half > 0; half >>= 1, o >>= 1) {
-            const bool hi = lane & o;
+    for (int half = kClusG / 2; half > 0; half >>= 1, o >>= 1) {
+        const bool hi = lane & o;
 #pragma unroll
-            for (int g = 0; g < half; g++) {
-                swap_add(s.fx[g], s.fx[g + half], hi, o);
-                swap_add(s.fy[g], s.fy[g + half], hi, o);
-                swap_add(s.fz[g], s.fz[g + half], hi, o);
-            }
+        for (int g = 0; g < half; g++) {
+            swap_add(s.fx[g], s.fx[g + half], hi, o);
+            swap_add(s.fy[g], s.fy[g + half], hi, o);
+            swap_add(s.fz[g], s.fz[g + half], hi, o);
         }
-        fx = s.fx[0]; fy = s.fy[0]; fz = s.fz[0];
-#pragma unroll
-        for (; o > 0; o >>= 1) {
-            fx += __shfl_xor_sync(kFull, fx, o);
-            fy += __shfl_xor_sync(kFull, fy, o);
-            fz += __shfl_xor_sync(kFull, fz, o);
-        }
-        return;
     }
-    fx = fy = fz = 0.0;
+    fx = s.fx[0]; fy = s.fy[0]; fz = s.fz[0];
 #pragma unroll
-    for (int g = 0; g < kClusG; g++) {
-        const double a = warp_sum(s.fx[g]), b = warp_sum(s.fy[g]), c = warp_sum(s.fz[g]);
-        if (lane == g) { fx = a; fy = b; fz = c; }
+    for (; o > 0; o >>= 1) {
+        fx += __shfl_xor_sync(kFull, fx, o);
+        fy += __shfl_xor_sync(kFull, fy, o);
+        fz += __shfl_xor_sync(kFull, fz, o);
     }
 }
 

@@ -14,9 +14,11 @@
 // and k = max_a |h_aa - h_p,aa| / h_p,aa, an entry at distance > rc + delta at
 // the prune is now farther than (1 - k)(rc + delta) - 2u.  While
 // k (rc + delta) + 2u < delta (less a rounding margin) every entry dropped by
-// the prune is still beyond the cutoff, so the pruned rows yield exactly the
+// the prune is still beyond the cutoff, so pruned rows of atoms yield exactly the
 // pairs of the full rows and the same pair terms; only the lanes that add
-// them, and so the rounding of the sums, change.  The drift raises u
+// them, and so the rounding of the sums, change.  (Cluster rows hold the same
+// pairs; their distances, from positions followed without wrapping, round
+// otherwise.)  The drift raises u
 // (kick_body); each block of the gather evaluates the condition
 // (lj_prune_needed) and walks either the full rows, writing pruned ones, or
 // the pruned rows; the step's reduction kernel then restarts the bound when

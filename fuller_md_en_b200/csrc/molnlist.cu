@@ -861,9 +861,6 @@ cudaError_t mol_rebuild_batch_rows(const MolBatch& b, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-namespace {
-}  // namespace
-
 cudaError_t mol_lists_alloc(MolLists& m, int n, const int* mol_id_host, const DevAlloc& da) {
     m = MolLists();
     if (n <= 0 || !mol_id_host) return cudaSuccess;

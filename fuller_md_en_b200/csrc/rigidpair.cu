@@ -49,6 +49,7 @@ constexpr int kPairBlocks32 = 6, kPairBlocks64 = 4;
 struct __align__(32) Vec {
     double x, y, z, pad;
 };
+static_assert(sizeof(Vec) == sizeof(double) * kRigidLabDoubles, "the sites of rigid.cu fit in");
 
 // R(q) (LJ:155-159) with reference rounding.
 __device__ __forceinline__ void rotation(const double* q, double* R) {

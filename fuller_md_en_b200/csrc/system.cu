@@ -781,10 +781,6 @@ extern "C" int fmd_system_create_rigid(fmd_ctx* ctx, const fmd_run_params* p, in
         return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
     cudaMemsetAsync(T, 0, sizeof(double) * 3 * n, ctx->stream);
     s->arr.body = bd; s->arr.qv = q; s->arr.omg = w; s->arr.T = T;
-    double* lab;
-    if (s->alloc(&lab, (size_t)n * natom * kRigidLabDoubles, (const double*)nullptr))
-        return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
-    s->arr.rigid_lab = lab;
     // The list radius is rmcut+3 (LJ:259); the force kernel skips pairs
     // beyond rmcut (LJ:320).
     if ((rc = s->alloc_lists(rmc, max_neigh, 0.0, 0, false)) != FMD_OK) return rc;
@@ -794,6 +790,9 @@ extern "C" int fmd_system_create_rigid(fmd_ctx* ctx, const fmd_run_params* p, in
         if (s->alloc(&mem, rigid_pair_bytes(n, natom, max_neigh), (const char*)nullptr))
             return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
         s->arr.rigid_pair = rigid_pair_layout(mem, n, natom, max_neigh);
+        s->arr.rigid_lab = static_cast<double*>(s->arr.rigid_pair.lab);     // each evaluation writes it before use
+    } else if (s->alloc(&s->arr.rigid_lab, (size_t)n * natom * kRigidLabDoubles, (const double*)nullptr)) {
+        return ctx->fail(FMD_ERR_CUDA, "device allocation failed");
     }
     out[0] = new fmd_system{std::move(s)};
     return FMD_OK;
