@@ -68,12 +68,20 @@ class Context:
             raise FmdError(rc, f"fmd_ctx_create(device={device}) failed: "
                            f"{self.lib.fmd_status_string(rc).decode()}")
         self.h = h
-        self._owned = []          # weak references to handles made on this context
+        self._owned = {}          # handles made on this context, oldest first
 
     def adopt(self, obj) -> None:
         """Registers a handle (system, batch, model, dataset) that must be
-        released before the context itself."""
-        self._owned.append(weakref.ref(obj))
+        released before the context itself.  The context keeps the handle, not
+        only a reference to its object: objects of one garbage cycle are
+        finalised in any order, after the weak references to them are gone."""
+        self._owned[id(obj)] = (type(obj)._destroy, obj.h, weakref.ref(obj))
+
+    def release(self, obj) -> None:
+        """Destroys obj's handle, unless the context has done so already."""
+        destroy, h, _ = self._owned.pop(id(obj), (None, None, None))
+        if destroy is not None:
+            getattr(self.lib, destroy)(h)
 
     def check(self, rc: int, what: str) -> None:
         if rc != 0:
@@ -98,11 +106,12 @@ class Context:
         if self.h:
             # handles made on this context go first, newest first (a batch
             # before its systems); they hold the context's stream
-            for r in reversed(self._owned):
-                o = r()
+            while self._owned:
+                destroy, h, ref = self._owned.popitem()[1]
+                getattr(self.lib, destroy)(h)
+                o = ref()
                 if o is not None:
-                    o.close()
-            self._owned.clear()
+                    o.h = None
             self.lib.fmd_ctx_destroy(self.h)
             self.h = None
 
@@ -357,6 +366,8 @@ class RunConfig:
 class System:
     """A device-resident system (fmd_system): state stays in HBM across steps."""
 
+    _destroy = "fmd_system_destroy"
+
     def __init__(self, ctx: Context, handle: ctypes.c_void_p, n: int, kind: int):
         self.ctx, self.h, self.n, self.kind = ctx, handle, n, kind
         ctx.adopt(self)
@@ -593,7 +604,7 @@ class System:
 
     def close(self) -> None:
         if self.h:
-            self.ctx.lib.fmd_system_destroy(self.h)
+            self.ctx.release(self)
             self.h = None
 
     def __del__(self):
@@ -607,6 +618,8 @@ class Batch:
     """Replicas advanced together (fmd_batch): MM systems of one context,
     each phase of a step one launch over all of them.  The systems stay
     usable for download/averages/lists and must outlive the batch."""
+
+    _destroy = "fmd_batch_destroy"
 
     def __init__(self, ctx: Context, systems: list, autotune: bool = True):
         self.ctx = ctx
@@ -646,7 +659,7 @@ class Batch:
 
     def close(self) -> None:
         if self.h:
-            self.ctx.lib.fmd_batch_destroy(self.h)
+            self.ctx.release(self)
             self.h = None
 
     def __del__(self):

@@ -66,6 +66,8 @@ def load_params(path: str | Path) -> dict:
 class Surrogate:
     """A model on one context's device (fmd_sg)."""
 
+    _destroy = "fmd_sg_destroy"
+
     def __init__(self, ctx, P: dict):
         self.lib = _lib.load()
         self.ctx = ctx
@@ -77,7 +79,7 @@ class Surrogate:
 
     def close(self):
         if self.h:
-            self.lib.fmd_sg_destroy(self.h)
+            self.ctx.release(self)
             self.h = ctypes.c_void_p()
             self.ctx = None
 
@@ -172,6 +174,8 @@ class Dataset:
     """Training snapshots on the device (fmd_sg_data); reference REBO energy,
     forces and virial come from the plain REBO kernel."""
 
+    _destroy = "fmd_sg_data_destroy"
+
     def __init__(self, ctx):
         self.lib = _lib.load()
         self.ctx = ctx
@@ -207,7 +211,7 @@ class Dataset:
 
     def close(self):
         if self.h:
-            self.lib.fmd_sg_data_destroy(self.h)
+            self.ctx.release(self)
             self.h = ctypes.c_void_p()
 
     def __del__(self):
