@@ -499,8 +499,8 @@ k_rebo2_bonds(const double* __restrict__ pos, const double* __restrict__ hh, con
 // from the half rows: a warp per atom, kScanU slices of 32 entries in flight.
 // The distance is FP32 (its square off by less than 0.006 A^2 where it is used:
 // cell edges below 2048 A, half the narrowest beyond the radius by 1 A); the
-// FP64 test decides within 0.01 A^2 of the radius, so the list holds no pair
-// more than the room for it was counted for.  30,000 atoms: 42 us; 79 us with a
+// FP64 test decides within 0.01 A^2 of the radius, so the list holds the pairs
+// within it and no other (its room is counted in those).  30,000 atoms: 42 us; 79 us with a
 // thread per slot of the table (occupied or not), a 64-bit division to find its
 // atom and the FP64 image of every entry.
 constexpr int kScanU = 4;
